@@ -31,11 +31,10 @@ namespace {
 
 constexpr int kSegThreads = 256;
 constexpr int kSegCands = kSegThreads * 8;  // candidates per segment
-constexpr int kCrsFmaAdds = 0;              // keystream additions on the FMA pipe: 4 measured no faster
 
 __device__ __forceinline__ void rng_block(const chacha::ChachaKey& key, unsigned long long blk,
                                           uint32_t (&w)[16]) {
-  chacha::chacha20_block<kCrsFmaAdds>(key, (uint32_t)blk, (uint32_t)(blk >> 32), w);
+  chacha::chacha20_block(key, (uint32_t)blk, (uint32_t)(blk >> 32), w);
 }
 
 __device__ __forceinline__ unsigned long long cand(const uint32_t (&w)[16], int c) {
@@ -164,10 +163,7 @@ int launch_sample_uniform(const grid_gpu_plan* p, const uint8_t seed[32], unsign
   unsigned* seg_rej = static_cast<unsigned*>(ws);
   unsigned long long* seg_off = reinterpret_cast<unsigned long long*>(
       static_cast<char*>(ws) + ((g.nseg * 4 + 255) / 256) * 256);
-  chacha::ChachaKey key;
-  for (int i = 0; i < 8; ++i)
-    key.k[i] = (uint32_t)seed[4 * i] | ((uint32_t)seed[4 * i + 1] << 8) |
-               ((uint32_t)seed[4 * i + 2] << 16) | ((uint32_t)seed[4 * i + 3] << 24);
+  const chacha::ChachaKey key = chacha::make_key(seed);
   const uint32_t r3 = (uint32_t)(((unsigned __int128)1 << 96) % p->f.q);
   unsigned long long grid = (unsigned long long)p->num_sms * 8;
   if (grid > g.nseg) grid = g.nseg;

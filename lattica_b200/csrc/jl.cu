@@ -13,13 +13,6 @@
 // The keystream is regenerated on the fly (the reference materialises the
 // whole [rows][parts][d][n] i8 matrix, 2 GiB at the LaBRADOR round size);
 // the i8 extraction is a separate, optional kernel.
-//
-// Projection kernel: a warp takes 32 consecutive columns of one part; lane l
-// computes the keystream bytes of column c0 + l into shared memory, then owns
-// rows 8l .. 8l+7 and sweeps the 32 columns, adding the coefficient to a
-// 64-bit "plus" or "minus" accumulator per row (exact while one warp sees
-// fewer than 2^32 columns of 32-bit words). Per-lane totals are folded mod q and added to
-// 64-bit global row sums with atomics; a final kernel reduces them mod q.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,7 +29,7 @@ namespace {
 using chacha::ChachaKey;
 using chacha::chacha20_block;
 
-constexpr int kJlWarps = 8;
+constexpr int kJlWarps = 8;  // jl_flat_kernel
 constexpr int kJlThreads = kJlWarps * 32;
 
 // Keystream bytes [off, off + 64) of stream (key, nonce0) as 16 words
@@ -65,267 +58,352 @@ __device__ __forceinline__ void keystream64(const ChachaKey& key, uint32_t nonce
   }
 }
 
-template <bool kWholeBlocks>
-__global__ void __launch_bounds__(kJlThreads) jl_project_kernel(
-    const uint32_t* __restrict__ parts, unsigned long long cols, int num_parts, int rows,
-    int packed_len, ChachaKey key, unsigned long long* __restrict__ gsum_pos,
-    unsigned long long* __restrict__ gsum_neg, uint32_t q) {
-  __shared__ uint32_t ks[kJlWarps][32][17];
-  __shared__ uint32_t xs[kJlWarps][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned long long chunks_per_part = (cols + 31) / 32;
-  const unsigned long long total = chunks_per_part * (unsigned long long)num_parts;
-  const unsigned long long stride = (unsigned long long)gridDim.x * kJlWarps;
-  unsigned long long pos[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  unsigned long long neg[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const int word = lane >> 1, shift = (lane & 1) * 16;
-
-  for (unsigned long long ch = (unsigned long long)blockIdx.x * kJlWarps + warp; ch < total;
-       ch += stride) {
-    const uint32_t part = (uint32_t)(ch / chunks_per_part);
-    const unsigned long long c = (ch % chunks_per_part) * 32 + lane;
-    uint32_t w[16];
-    uint32_t x = 0;
-    if (c < cols) {
-      if constexpr (kWholeBlocks)
-        chacha20_block(key, (uint32_t)c, part, w);  // 256 rows: column c is block c
-      else
-        keystream64(key, part, c * (unsigned long long)packed_len, w);
-      x = parts[(unsigned long long)part * cols + c];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) w[i] = 0xFFFFFFFFu;  // code 11 -> 0
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) ks[warp][lane][i] = w[i];
-    xs[warp][lane] = x;
-    __syncwarp();
-#pragma unroll 4
-    for (int cc = 0; cc < 32; ++cc) {
-      const uint32_t h = ks[warp][cc][word] >> shift;
-      const uint32_t xc = xs[warp][cc];
-      const uint32_t lo = h & 0x5555u, hi = (h >> 1) & 0x5555u;
-      const uint32_t plus = ~(lo | hi) & 0x5555u;  // code 00
-      const uint32_t minus = lo & ~hi;             // code 01
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        pos[k] += (unsigned long long)(xc & (0u - ((plus >> (2 * k)) & 1u)));
-        neg[k] += (unsigned long long)(xc & (0u - ((minus >> (2 * k)) & 1u)));
-      }
-    }
-  }
-  // Fold to residues and publish. Rows beyond `rows` only saw code 11.
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int row = lane * 8 + k;
-    if (row < rows && (pos[k] | neg[k])) {
-      atomicAdd(&gsum_pos[row], pos[k] % q);
-      atomicAdd(&gsum_neg[row], neg[k] % q);
-    }
-  }
-}
-
-__global__ void jl_finish_kernel(const unsigned long long* __restrict__ gsum_pos,
-                                 const unsigned long long* __restrict__ gsum_neg, uint32_t* p_out,
-                                 int rows, uint32_t q) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < rows) {
-    const uint32_t a = (uint32_t)(gsum_pos[r] % q), b = (uint32_t)(gsum_neg[r] % q);
-    p_out[r] = sub_mod(a, b, q);
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Tensor-core projection. A CTA takes chunks of 256 columns of one part:
-// thread t computes the keystream of column c0 + t and writes its 256
-// entries shifted by one, M' = M + 1 in {0, 1, 2}, as column t of an
-// MN-major u8 A tile (rows contiguous), and the column's word as a
-// zero-padded 16-byte column of an MN-major u8 B tile (bytes = N). One u8
-// MMA per (128-row half, 32-column step) accumulates
-// D'[r][i] = sum_c M'[r][c] * byte_i(x_c) in tensor memory across all of the
-// CTA's chunks; then p_r = sum_i 2^(8i) (D'[r][i] - sum_c byte_i(x_c)) mod q.
-// D' < 2 * 255 * (columns per CTA) stays below 2^31 (the host bounds the
-// columns per CTA).
+// Tensor-core projection. A producer warp takes a unit of 32 columns of one
+// part: lane l computes the keystream of its column and writes the column's 256
+// entries, shifted to M' = M + 1 in {0, 1, 2}, into an MN-major u8 A tile (rows
+// contiguous), and the column's word as a zero-padded 16-byte column of an
+// MN-major u8 B tile (bytes = N). Two u8 MMAs (128-row halves, K = 32) per unit
+// accumulate D[r][i] = sum_c M'[r][c] * byte_i(x_c) in tensor memory across all
+// of the CTA's units; then p_r = sum_i 2^(8i) (D[r][i] - sum_c byte_i(x_c)).
+//
+// The bound is the ALU pipe: a ChaCha20 block is 80 quarter rounds of 8 XORs
+// and rotations, 1280 cycles of one sub-partition per warp (its additions run
+// beside them: measured 1279-1301 cycles with none, half or all of them on the
+// FMA pipe), so 0.29 ms for the LaBRADOR round's 8.4 M columns. Everything else
+// is kept small against that:
+//  * Entries are unpacked without a table. Bit by bit M' is (h, ~h & ~l) for a
+//    code (h, l), a shift and two logic operations for the 16 entries of a word;
+//    three masks then leave entry 4j + s of byte j in place, scaled by 4^s, and
+//    the packed word itself serves for s = 0 (it holds e_0 + 4 e_1 + 16 e_2 +
+//    64 e_3 per byte: the other three sums, subtracted at the end, leave e_0's).
+//    A tile row 16 g + 4 s + j is therefore matrix row 16 g + 4 j + s, 4^s times
+//    its entry. (Table lookups: 64 a column, each conflicting over the 32 lanes.)
+//  * Every producer warp owns its A and B tile and hands it to the MMA warp
+//    through two mbarriers, so no barrier holds the CTA's warps together: one
+//    CTA of 20 producer warps per SM, where three CTAs of 8 met at two CTA
+//    barriers per chunk of 256 columns.
+// Measured at 64 x 131072 columns: 0.51 ms before, 0.42 ms now; with the int8 entries
+// 1.21 ms before, 0.90 ms now.
 // ---------------------------------------------------------------------------
-constexpr int kTcThreads = 256;
-constexpr int kTcCols = 256;                      // columns (K) per chunk
-// Keystream additions issued on the FMA pipe per quarter round (chacha20_block).
-// Measured: the projection 0.552 / 0.532 / 0.524 ms with 0 / 2 / 4, the
-// evaluations (whose FMA pipe is busier) 0.795 / 0.828 / 0.829 ms.
-constexpr int kTcFmaAdds = 4;
-constexpr int kEvFmaAdds = 0;
-constexpr uint32_t kTcA = 256u * kTcCols;         // A tile: 256 rows x 256 columns
-constexpr uint32_t kTcB = 16u * kTcCols;          // B tile: 16 bytes x 256 columns
-constexpr uint32_t kTcSmem = kTcA + kTcB + 1024 + 64 + 1024;  // + LUT, barrier, slack
-constexpr unsigned long long kTcMaxColsPerCta = 1ull << 22;    // 2 * 255 * 2^22 < 2^31
+constexpr uint32_t kUnitCols = 32;                      // columns per unit (K of one MMA)
+constexpr uint32_t kUnitA = 256u * kUnitCols;           // A tile: 256 rows x 32 columns
+constexpr uint32_t kPjB = 16u * kUnitCols;              // B tile: 16 bytes x 32 columns
+constexpr int kGroup = 4;                               // warps per hand-over (mma_loop)
+// The plain projection runs 20 producer warps (0.416 ms at 64 x 131072 columns with 16
+// or 20, 0.421 with 24, 0.438 with 12). With the int8 entries it runs 12: the scattered
+// 32-byte sector stores of more warps get in each other's way (0.90 ms with 12, 0.95
+// with 8, 1.2 with 16, 1.6 with 20).
+template <bool kFlat>
+struct PjShape {
+  static constexpr int WARPS = kFlat ? 12 : 20;         // producer warps
+  static constexpr int THREADS = (WARPS + 1) * 32;      // + the MMA warp
+  static constexpr uint32_t OFF_B = WARPS * kUnitA;
+  static constexpr uint32_t OFF_BAR = OFF_B + WARPS * kPjB;
+  static constexpr uint32_t SMEM =
+      OFF_BAR + (2 * WARPS / kGroup + 1) * 8 + 32 + 128;  // + alignment slack
+  static_assert(SMEM <= 232448 && WARPS % kGroup == 0, "shape");
+};
+// A packed byte is at most 2 (1 + 4 + 16 + 64) = 170, a byte of x 255: 170 * 255 * 2^16
+// stays below 2^32, the accumulators' wrap.
+constexpr unsigned long long kMaxUnitsPerCta = (1ull << 16) / kUnitCols;
 
-// row m, column k of the A tile: 16-row x 8-column core matrices
-__device__ __forceinline__ uint32_t jl_a_off(uint32_t m, uint32_t k) {
+// Row m, column k of a unit's A tile: 16-row x 8-column core matrices.
+__device__ __forceinline__ uint32_t unit_a_off(uint32_t m, uint32_t k) {
   return (k >> 3) * 2048u + (m >> 4) * 128u + (k & 7u) * 16u + (m & 15u);
 }
 
-// M' = M + 1 for the 4 codes of one keystream byte: 00 -> 2, 01 -> 0, 1x -> 1.
-__device__ __forceinline__ uint32_t shifted_entries_of_byte(uint32_t byte) {
-  uint32_t out = 0;
+// The 16 entries of a keystream word as M' = M + 1, two bits each: 00 -> 2, 01 -> 0,
+// 1x -> 1, i.e. low bit = h, high bit = ~h & ~l.
+__device__ __forceinline__ uint32_t packed_entries(uint32_t w) {
+  const uint32_t high = ~(w | (w + w)) & 0xAAAAAAAAu;
+  return ((w >> 1) & 0x55555555u) | high;
+}
+
+// One column's entries into the A tile (dst = its column's first 16 rows).
+__device__ __forceinline__ void store_entries(unsigned char* dst, const uint32_t (&w)[16]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = (byte >> (2 * i)) & 3u;
-    const uint32_t v = c == 0 ? 2u : (c == 1 ? 0u : 1u);
-    out |= v << (8 * i);
+  for (int g = 0; g < 16; ++g) {
+    const uint32_t m = packed_entries(w[g]);
+    *reinterpret_cast<uint4*>(dst + 128 * g) =
+        make_uint4(m, m & 0x0C0C0C0Cu, m & 0x30303030u, m & 0xC0C0C0C0u);
   }
-  return out;
+}
+
+// Matrix row of tile row m, and the sum of a tile row's true entries from the
+// accumulators of the warp's 32 tile rows (lane = m % 32; all lanes take part).
+__device__ __forceinline__ int tile_row_to_row(int m) {
+  return (m & ~15) | ((m & 3) << 2) | ((m >> 2) & 3);
+}
+__device__ __forceinline__ uint32_t unscale(uint32_t d, int lane) {
+  const int s = (lane >> 2) & 3;
+  uint32_t rest = __shfl_down_sync(0xffffffffu, d, 4);
+  rest += __shfl_down_sync(0xffffffffu, d, 8);
+  rest += __shfl_down_sync(0xffffffffu, d, 12);
+  return s == 0 ? d - rest : d >> (2 * s);
+}
+
+// sum_i 2^(8i) (d_i - corr_i), exact in 64 bits.
+__device__ __forceinline__ long long weigh(const uint32_t* d, const uint32_t* corr) {
+  long long v = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v += ((long long)d[i] - (long long)corr[i]) << (8 * i);
+  return v;
+}
+
+// v mod q in [0, q).
+__device__ __forceinline__ uint32_t residue(long long v, uint32_t q) {
+  const long long r = v % (long long)q;
+  return (uint32_t)(r < 0 ? r + q : r);
+}
+
+// Descriptor `off` bytes after one whose address field cannot carry out of its word.
+__device__ __forceinline__ uint64_t desc_plus(uint64_t desc, uint32_t off) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"((uint32_t)desc + (off >> 4)), "r"((uint32_t)(desc >> 32)));
+  return r;
+}
+
+// The MMA warp's loop (one lane): warp w's units are first(w), first(w) + stride, ...
+// below nunits, first() ascending; issue(w, accumulate) issues one unit's MMAs. A group
+// of kGroup warps is handed over through one barrier and released by one commit, and the
+// full rounds are unrolled, every descriptor one addition away from a constant: the
+// MMA warp shares its sub-partition with six warps that saturate the ALU pipe, so each
+// of its instructions costs 10 to 15 cycles, and a tcgen05 instruction 44 on an idle SM.
+// (One barrier and commit per unit, descriptors built in the loop: 600 cycles a unit,
+// where the units come every 380.)
+// Ends when every unit is issued (or a wait gave up) and all MMAs are done.
+template <int WARPS, typename First, typename Issue>
+__device__ __forceinline__ void mma_loop(uint64_t* full, uint64_t* empty, uint64_t* done,
+                                         uint32_t nunits, uint32_t stride, First first,
+                                         Issue issue, int* err) {
+  static_assert(WARPS % kGroup == 0, "whole groups");
+  bool ok = true;
+  uint32_t acc = 0;
+  // nunits + stride stays below 2^32
+  for (uint32_t base = 0, it = 0; ok && first(0) + base < nunits; base += stride, ++it) {
+    if (acc && first(WARPS - 1) + base < nunits) {
+#pragma unroll
+      for (int g = 0; g < WARPS / kGroup; ++g) {
+        ok = ok && mbar_wait(&full[g], it & 1, err);
+        if (ok) {
+          tc::fence_after_sync();
+#pragma unroll
+          for (int i = 0; i < kGroup; ++i) issue(kGroup * g + i, 1u);
+          tc::mma_commit(&empty[g]);
+        }
+      }
+      continue;
+    }
+#pragma unroll 1
+    for (int g = 0; g < WARPS / kGroup && first(kGroup * g) + base < nunits; ++g) {
+      if (!(ok = mbar_wait(&full[g], it & 1, err))) break;
+      tc::fence_after_sync();
+#pragma unroll 1
+      for (int w = kGroup * g; w < kGroup * (g + 1) && first(w) + base < nunits; ++w) {
+        issue(w, acc);
+        acc = 1;
+      }
+      tc::mma_commit(&empty[g]);
+    }
+  }
+  tc::mma_commit(done);  // completes once every MMA issued above has (at once if none was)
+  mbar_wait_sleep(done, 0, err);
+}
+
+// The producers' wait for their tiles: asleep in the barrier, since polling warps
+// hold up the MMA warp's own waits.
+__device__ __forceinline__ bool tiles_free(uint64_t* bar, uint32_t it, int lane, int* err) {
+  bool ok = true;
+  if (it > 0) {
+    if (lane == 0) ok = mbar_wait_sleep(bar, (it - 1) & 1, err);
+    __syncwarp();
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+  }
+  return ok;
 }
 
 // kFlat (whole blocks, d % 8 == 0, n % 32 == 0): the kernel also writes the
-// int8 entries flat[row][part][k][j] (col = j d + k) from the words it builds
-// for the A tile, so the keystream is generated once. A chunk is then 32
-// consecutive polynomials x 8 coefficient indices: warp w takes coefficient
-// 8 kg + w and lane l polynomial 32 jg + l. For each keystream byte, the four
-// lanes of a quad swap bytes (a 4 x 4 transpose: two shuffles, two byte
-// permutes) so that lane 4 g + r holds row 4 b + r of polynomials 4 g .. 4 g + 3,
-// and the warp's stores fill whole 32-byte sectors of four rows.
+// int8 entries flat[row][part][k][j] (col = j d + k), so the keystream is generated
+// once. A unit is then 32 consecutive polynomials of one coefficient index: lane l
+// takes polynomial 32 jg + l. For each word of 4 rows the four lanes of a quad
+// swap bytes (a 4 x 4 transpose: two shuffles, two byte permutes) so that lane
+// 4 g + r holds one row of polynomials 4 g .. 4 g + 3, and the warp's stores fill
+// whole 32-byte sectors of four rows.
 template <bool kWholeBlocks, bool kFlat = false>
-__global__ void __launch_bounds__(kTcThreads) jl_tc_kernel(
+__global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
     const uint32_t* __restrict__ parts, unsigned long long cols, int rows, int packed_len,
-    ChachaKey key, unsigned long long nchunks, unsigned long long per_part, int d,
-    unsigned long long plane, int8_t* __restrict__ flat,
-    unsigned long long* __restrict__ gsum_pos, uint32_t q, int* __restrict__ err) {
-  extern __shared__ __align__(1024) unsigned char sm_raw[];
+    ChachaKey key, uint32_t nunits, uint32_t per_part, uint32_t d, unsigned long long plane,
+    int8_t* __restrict__ flat, unsigned long long* __restrict__ gsum, uint32_t q, bool fold,
+    int* __restrict__ err) {
+  using S = PjShape<kFlat>;
+  constexpr int WARPS = S::WARPS;
+  extern __shared__ __align__(128) unsigned char sm_raw[];
   const uint32_t raw = smem_addr(sm_raw);
-  unsigned char* sm = sm_raw + (((raw + 1023u) & ~1023u) - raw);
+  unsigned char* sm = sm_raw + (((raw + 127u) & ~127u) - raw);
   const uint32_t s0 = smem_addr(sm);
-  uint32_t* lut = reinterpret_cast<uint32_t*>(sm + kTcA + kTcB);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTcA + kTcB + 1024);
-  uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(bar + 1);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + S::OFF_BAR);
+  uint64_t* empty = full + WARPS / kGroup;
+  uint64_t* done = empty + WARPS / kGroup;
+  uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(done + 1);
   uint32_t* colsum = taddr_slot + 2;  // [4]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  for (int i = tid; i < 256; i += kTcThreads) lut[i] = shifted_entries_of_byte(i);
   if (tid < 4) colsum[tid] = 0;
-  if (warp == 0) {
+  if (warp == WARPS) {
     tc::tmem_alloc(taddr_slot, 32);
     tc::tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(bar, 1);
+    for (int i = 0; i < WARPS / kGroup; ++i) {
+      mbar_init(&full[i], kGroup);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
     fence_mbar_init();
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *taddr_slot;
-  // kind::i8, u8 x u8 -> s32, A and B MN-major, M = 128, N = 16
-  const uint32_t idesc = tc::idesc_u8(128, 16) | (1u << 15) | (1u << 16);
+  const uint32_t stride = gridDim.x * WARPS;
+  // consecutive units on consecutive SMs (few units: one warp of every SM), or, with
+  // the entries, on consecutive warps: neighbouring polynomials' sectors of a row
+  auto first = [&](int w) -> uint32_t {
+    return kFlat ? blockIdx.x * WARPS + w : (uint32_t)w * gridDim.x + blockIdx.x;
+  };
 
-  const unsigned long long npoly = cols / (unsigned long long)d;
-  // byte selectors of the quad transpose (step 1: lanes l, l ^ 1; step 2: l, l ^ 2)
-  const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u;
-  const uint32_t sel2 = (lane & 2) ? 0x3276u : 0x5410u;
-  uint32_t bsum[4] = {0, 0, 0, 0};
-  bool ok = true;
-  uint32_t it = 0;
-  for (unsigned long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x, ++it) {
-    const uint32_t part = (uint32_t)(ch / per_part);
-    const unsigned long long ci = ch % per_part;
-    unsigned long long c, jj = 0;
-    uint32_t kk = 0;
-    if constexpr (kFlat) {
-      const unsigned long long kgroups = (unsigned long long)d / 8;
-      jj = (ci / kgroups) * 32 + lane;
-      kk = (uint32_t)(ci % kgroups) * 8 + warp;
-      c = jj * d + kk;
-    } else {
-      c = ci * kTcCols + tid;
-    }
-    uint32_t w[16];
-    uint32_t x = 0;
-    if (c < cols) {
-      if constexpr (kWholeBlocks)
-        chacha20_block<kTcFmaAdds>(key, (uint32_t)c, part, w);
-      else
-        keystream64(key, part, c * (unsigned long long)packed_len, w);
-      x = parts[(unsigned long long)part * cols + c];
-    } else {
+  if (warp == WARPS) {
+    if (lane == 0) {
+      // kind::i8, u8 x u8 -> s32, A and B MN-major, M = 128, N = 16
+      const uint32_t idesc = tc::idesc_u8(128, 16) | (1u << 15) | (1u << 16);
+      const uint64_t da = tc::smem_desc(s0, 2048, 128);
+      const uint64_t db = tc::smem_desc(s0 + S::OFF_B, 128, 256);
+      mma_loop<WARPS>(
+          full, empty, done, nunits, stride, first,
+          [&](int w, uint32_t acc) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) w[i] = 0xFFFFFFFFu;  // padding column: x = 0
+            for (int h = 0; h < 2; ++h)
+              tc::mma_u8(tbase + 16 * h, desc_plus(da, w * kUnitA + h * 1024),
+                         desc_plus(db, w * kPjB), idesc, acc);
+          },
+          err);
     }
-    // the previous chunk's MMAs must be done reading the tiles
-    if (it > 0) ok = __syncthreads_and(mbar_wait(bar, (it - 1) & 1, err));
-    if (!ok) break;
-    // kFlat: this lane's row 4 b + (lane & 3) of polynomials jj - (lane & 3) .. + 3,
-    // keystream byte b = 0, 1, ...: one pointer advanced by 4 rows per byte
-    int8_t* rowp = nullptr;
-    if constexpr (kFlat)
-      rowp = flat + (unsigned long long)(lane & 3) * plane +
-             ((unsigned long long)part * d + kk) * npoly + (jj - (lane & 3));
-    const unsigned long long step4 = 4 * plane;
-#pragma unroll
-    for (int g = 0; g < 16; ++g) {
-      const uint32_t v[4] = {lut[w[g] & 0xFFu], lut[(w[g] >> 8) & 0xFFu],
-                             lut[(w[g] >> 16) & 0xFFu], lut[w[g] >> 24]};
-      *reinterpret_cast<uint4*>(sm + jl_a_off(16 * g, tid)) = make_uint4(v[0], v[1], v[2], v[3]);
+    __syncwarp();
+  } else {
+    unsigned char* at = sm + warp * kUnitA + unit_a_off(0, lane);
+    unsigned char* bt = sm + S::OFF_B + warp * kPjB + lane * 16;
+    const unsigned long long npoly = cols / d;
+    // byte selectors of the quad transpose (step 1: lanes l, l ^ 1; step 2: l, l ^ 2)
+    const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u;
+    const uint32_t sel2 = (lane & 2) ? 0x3276u : 0x5410u;
+    uint32_t bsum[4] = {0, 0, 0, 0};
+    uint32_t unit = first(warp);
+    uint32_t part = unit / per_part, ci = unit % per_part;
+    const uint32_t step_part = stride / per_part, step_ci = stride % per_part;
+    uint64_t* grp_full = &full[warp / kGroup];
+    uint64_t* grp_empty = &empty[warp / kGroup];
+    // a warp whose group still has a unit arrives with it
+    uint32_t lead = first(warp / kGroup * kGroup);
+    for (uint32_t it = 0; lead < nunits; ++it, unit += stride, lead += stride) {
+      if (unit >= nunits) {
+        if (tiles_free(grp_empty, it, lane, err) && lane == 0) mbar_arrive(grp_full);
+        break;
+      }
+      unsigned long long c, jj = 0;
+      uint32_t kk = 0;
       if constexpr (kFlat) {
+        const uint32_t groups = per_part / d;  // polynomials / 32
+        jj = (unsigned long long)(ci % groups) * 32 + lane;
+        kk = ci / groups;
+        c = jj * d + kk;
+      } else {
+        c = (unsigned long long)ci * kUnitCols + lane;
+      }
+      uint32_t w[16];
+      uint32_t x = 0;
+      if (c < cols) {
+        x = __ldg(parts + (unsigned long long)part * cols + c);
+        if constexpr (kWholeBlocks)
+          chacha20_block(key, (uint32_t)c, part, w);
+        else
+          keystream64(key, part, c * (unsigned long long)packed_len, w);
+      } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t m = (v[i] + 0x7F7F7F7Fu) ^ 0x80808080u;  // M = M' - 1 per byte
-          const uint32_t a = __byte_perm(m, __shfl_xor_sync(0xffffffffu, m, 1), sel1);
-          const uint32_t o = __byte_perm(a, __shfl_xor_sync(0xffffffffu, a, 2), sel2);
-          if (4 * (4 * g + i) + (lane & 3) < rows) *reinterpret_cast<uint32_t*>(rowp) = o;
-          rowp += step4;
+        for (int i = 0; i < 16; ++i) w[i] = 0xFFFFFFFFu;  // padding column: x = 0
+      }
+      // the previous unit's MMAs must be done reading the tiles
+      if (!tiles_free(grp_empty, it, lane, err)) break;
+      store_entries(at, w);
+      *reinterpret_cast<uint4*>(bt) = make_uint4(x, 0, 0, 0);
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(grp_full);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bsum[i] += (x >> (8 * i)) & 0xFFu;
+      if constexpr (kFlat) {
+        // word s of keystream word g: rows 16 g + 4 j + s (j = 0 .. 3) of this lane's
+        // polynomial; after the transpose row 16 g + 4 (lane & 3) + s of
+        // polynomials jj - (lane & 3) .. + 3
+        int8_t* rowp = flat + ((unsigned long long)part * d + kk) * npoly + (jj - (lane & 3)) +
+                       (unsigned long long)(4 * (lane & 3)) * plane;
+#pragma unroll
+        for (int g = 0; g < 16; ++g) {
+          const uint32_t m = packed_entries(w[g]);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            const uint32_t v = (m >> (2 * s)) & 0x03030303u;
+            const uint32_t e = (v + 0x7F7F7F7Fu) ^ 0x80808080u;  // M = M' - 1 per byte
+            const uint32_t a = __byte_perm(e, __shfl_xor_sync(0xffffffffu, e, 1), sel1);
+            const uint32_t o = __byte_perm(a, __shfl_xor_sync(0xffffffffu, a, 2), sel2);
+            if (16 * g + 4 * (lane & 3) + s < rows) *reinterpret_cast<uint32_t*>(rowp) = o;
+            rowp += plane;
+          }
+          rowp += 12 * plane;
         }
       }
+      part += step_part;
+      ci += step_ci;
+      if (ci >= per_part) {
+        ci -= per_part;
+        ++part;
+      }
     }
-    *reinterpret_cast<uint4*>(sm + kTcA + (tid >> 3) * 128 + (tid & 7) * 16) =
-        make_uint4(x, 0, 0, 0);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) bsum[i] += (x >> (8 * i)) & 0xFFu;
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc::fence_after_sync();
+    for (int i = 0; i < 4; ++i) {
+      uint32_t v = bsum[i];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int ks = 0; ks < kTcCols / 32; ++ks)
-          tc::mma_u8(tbase + 16 * h, tc::smem_desc(s0 + h * 1024 + ks * 8192, 2048, 128),
-                     tc::smem_desc(s0 + kTcA + ks * 512, 128, 256), idesc,
-                     (it | (uint32_t)ks) != 0);
-      tc::mma_commit(bar);
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) atomicAdd(&colsum[i], v);
     }
   }
-  if (ok && it > 0) ok = mbar_wait(bar, (it - 1) & 1, err);
-  ok = __syncthreads_and(ok);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t v = bsum[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) atomicAdd(&colsum[i], v);
-  }
-  __syncthreads();
+  __syncthreads();  // every MMA is done, the byte sums are complete
   tc::fence_after_sync();
-  if (ok && it > 0 && warp < 4) {
-    uint32_t d0[4], d1[4];
-    tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 0), d0);
-    tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 16), d1);
+  if (warp < 4 && first(0) < nunits) {  // a CTA without units accumulated nothing
+    uint32_t dv[2][4];
+    tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 0), dv[0]);
+    tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 16), dv[1]);
     tc::tmem_ld_wait();
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int row = 128 * h + 32 * warp + lane;
-      const uint32_t* dv = h ? d1 : d0;
-      long long v = 0;
+      const int row = tile_row_to_row(128 * h + 32 * warp + lane);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v += ((long long)dv[i] - (long long)colsum[i]) << (8 * i);
-      long long r = v % (long long)q;
-      if (r < 0) r += q;
-      if (row < rows) atomicAdd(&gsum_pos[row], (unsigned long long)r);
+      for (int i = 0; i < 4; ++i) dv[h][i] = unscale(dv[h][i], lane);
+      const long long v = weigh(dv[h], colsum);
+      if (row < rows)
+        atomicAdd(&gsum[row], (unsigned long long)(fold ? (long long)residue(v, q) : v));
     }
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, 32);
+  if (warp == WARPS) tc::tmem_dealloc(tbase, 32);
+}
+
+// out[i] = the signed sum gsum[i] mod q.
+__global__ void jl_finish_kernel(const unsigned long long* __restrict__ gsum,
+                                 uint32_t* __restrict__ out, int n, uint32_t q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = residue((long long)gsum[i], q);
 }
 
 // Entry -> int8 table for one keystream byte: 4 rows, 2 bits each.
@@ -427,124 +505,150 @@ __global__ void __launch_bounds__(kJlThreads) jl_flat_kernel(unsigned long long 
 // columns (two 128-row halves). The M' = M + 1 correction
 // S[t][i] = sum_c byte_i(s'[u_c + t]) comes from per-position byte sums of each
 // coefficient and its negation: sum_{v >= t} P_i[v] + sum_{v < t} N_i[v].
+//
+// A unit is 32 coefficients (half a polynomial) of one part. The B tile is a
+// Hankel matrix, word (u, t) = s'[u + t]: core matrix (k-group kg, t-group g) depends
+// on 2 kg + g alone, so the tile is 22 overlapping core matrices (128 bytes each)
+// instead of 64, and the descriptor's strides are 2 and 1 of them. Bound and
+// hand-over as in the projection (20 producer warps: 11 KB of tiles each); the
+// tensor pipe is the second resource, 256 cycles per unit of about 400.
+// Measured at 64 x 131072 columns: 0.78 ms before (one chunk of 256 columns per CTA
+// at a time, table lookups, every rotation written out), 0.47 ms now.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kEvB = 256u * kTcCols;                  // B tile: 256 bytes x 256 columns
-// M' table in 32 bank-rotated copies (entry e of copy c at word 32 e + c; lane
-// l reads copy l), so the 32 random lookups of a warp never share a bank
-constexpr uint32_t kEvOffLut = kTcA + kEvB;
-constexpr uint32_t kEvOffPoly = kEvOffLut + 32 * 1024;     // the chunk's 4 polys (1 KB)
-constexpr uint32_t kEvOffSums = kEvOffPoly + 1024;         // P[64][4], N[64][4] (2 KB)
-constexpr uint32_t kEvOffS = kEvOffSums + 2048;            // S[64][4] (1 KB)
-constexpr uint32_t kEvOffBar = kEvOffS + 1024;
-constexpr uint32_t kEvSmem = kEvOffBar + 64 + 1024;        // + alignment slack
 constexpr int kEvD = 64, kEvRows = 256;
+constexpr int kEvWarps = 20;
+constexpr int kEvThreads = (kEvWarps + 1) * 32;
+constexpr uint32_t kEvCores = 22;                       // 2 kg + g, kg < 4, g < 16
+constexpr uint32_t kEvB = kEvCores * 128;
+constexpr uint32_t kEvOffB = kEvWarps * kUnitA;
+constexpr uint32_t kEvOffExt = kEvOffB + kEvWarps * kEvB;  // s', 128 words per warp
+constexpr uint32_t kEvOffBar = kEvOffExt + kEvWarps * 512;
+constexpr uint32_t kEvSmem = kEvOffBar + (2 * kEvWarps / kGroup + 1) * 8 + 16 + 128;
+static_assert(kEvSmem <= 232448, "shared memory budget");
+// after the last MMA the tiles hold the corrections: P[64][4], N[64][4], S[64][4]
+constexpr uint32_t kEvOffSums = 0, kEvOffS = 2048;
 
-__global__ void __launch_bounds__(kTcThreads, 1) jl_eval_tc_kernel(
-    const uint32_t* __restrict__ parts, unsigned long long cols, ChachaKey key,
-    unsigned long long nchunks, unsigned long long* __restrict__ gsum, uint32_t q,
+__global__ void __launch_bounds__(kEvThreads, 1) jl_eval_tc_kernel(
+    const uint32_t* __restrict__ parts, unsigned long long cols, ChachaKey key, uint32_t nunits,
+    uint32_t per_part, unsigned long long* __restrict__ gsum, uint32_t q, bool fold,
     int* __restrict__ err) {
-  extern __shared__ __align__(1024) unsigned char sm_raw[];
+  extern __shared__ __align__(128) unsigned char sm_raw[];
   const uint32_t raw = smem_addr(sm_raw);
-  unsigned char* sm = sm_raw + (((raw + 1023u) & ~1023u) - raw);
+  unsigned char* sm = sm_raw + (((raw + 127u) & ~127u) - raw);
   const uint32_t s0 = smem_addr(sm);
-  uint32_t* lut = reinterpret_cast<uint32_t*>(sm + kEvOffLut);
-  uint32_t* poly = reinterpret_cast<uint32_t*>(sm + kEvOffPoly);
   uint32_t* sums = reinterpret_cast<uint32_t*>(sm + kEvOffSums);  // [0,256): P, [256,512): N
   uint32_t* corr = reinterpret_cast<uint32_t*>(sm + kEvOffS);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kEvOffBar);
-  uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(bar + 1);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + kEvOffBar);
+  uint64_t* empty = full + kEvWarps / kGroup;
+  uint64_t* done = empty + kEvWarps / kGroup;
+  uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(done + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  for (int i = tid; i < 256 * 32; i += kTcThreads) lut[i] = shifted_entries_of_byte(i >> 5);
-  for (int i = tid; i < 512; i += kTcThreads) sums[i] = 0;
-  if (warp == 0) {
+  if (warp == kEvWarps) {
     tc::tmem_alloc(taddr_slot, 512);
     tc::tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(bar, 1);
+    for (int i = 0; i < kEvWarps / kGroup; ++i) {
+      mbar_init(&full[i], kGroup);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
     fence_mbar_init();
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *taddr_slot;
-  // kind::i8, u8 x u8 -> s32, A and B MN-major, M = 128, N = 256
-  const uint32_t idesc = tc::idesc_u8(128, 256) | (1u << 15) | (1u << 16);
+  const uint32_t stride = gridDim.x * kEvWarps;  // even: a warp keeps its half polynomial
+  auto first = [&](int w) -> uint32_t { return (uint32_t)w * gridDim.x + blockIdx.x; };
 
-  const unsigned long long per_part = (cols + kTcCols - 1) / kTcCols;
-  const uint32_t u = tid & (kEvD - 1);  // this thread's coefficient position in its poly
   uint32_t psum[4] = {0, 0, 0, 0}, nsum[4] = {0, 0, 0, 0};
-  bool ok = true;
-  uint32_t it = 0;
-  for (unsigned long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x, ++it) {
-    const uint32_t part = (uint32_t)(ch / per_part);
-    const unsigned long long c = (ch % per_part) * kTcCols + tid;
-    uint32_t w[16];
-    uint32_t x = 0;
-    if (c < cols) {
-      chacha20_block<kEvFmaAdds>(key, (uint32_t)c, part, w);  // 256 rows: column c is block c
-      x = parts[(unsigned long long)part * cols + c];
-    } else {
+  uint32_t u0 = 0;
+  if (warp == kEvWarps) {
+    if (lane == 0) {
+      // kind::i8, u8 x u8 -> s32, A and B MN-major, M = 128, N = 256
+      const uint32_t idesc = tc::idesc_u8(128, 256) | (1u << 15) | (1u << 16);
+      const uint64_t da = tc::smem_desc(s0, 2048, 128);
+      const uint64_t db = tc::smem_desc(s0 + kEvOffB, 256, 128);
+      mma_loop<kEvWarps>(
+          full, empty, done, nunits, stride, first,
+          [&](int w, uint32_t acc) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) w[i] = 0xFFFFFFFFu;  // padding column: x = 0
+            for (int h = 0; h < 2; ++h)
+              tc::mma_u8(tbase + 256 * h, desc_plus(da, w * kUnitA + h * 1024),
+                         desc_plus(db, w * kEvB), idesc, acc);
+          },
+          err);
     }
-    const uint32_t xn = x == 0 ? 0u : q - x;
+    __syncwarp();
+  } else {
+    unsigned char* at = sm + warp * kUnitA + unit_a_off(0, lane);
+    unsigned char* bt = sm + kEvOffB + warp * kEvB;
+    uint32_t* ext = reinterpret_cast<uint32_t*>(sm + kEvOffExt + warp * 512);
+    uint32_t unit = first(warp);
+    uint32_t part = unit / per_part, ci = unit % per_part;
+    const uint32_t step_part = stride / per_part, step_ci = stride % per_part;
+    u0 = (unit & 1) * kUnitCols;  // per_part is even: the unit's half polynomial
+    uint64_t* grp_full = &full[warp / kGroup];
+    uint64_t* grp_empty = &empty[warp / kGroup];
+    // a warp whose group still has a unit arrives with it
+    uint32_t lead = first(warp / kGroup * kGroup);
+    for (uint32_t it = 0; lead < nunits; ++it, unit += stride, lead += stride) {
+      if (unit >= nunits) {
+        if (tiles_free(grp_empty, it, lane, err) && lane == 0) mbar_arrive(grp_full);
+        break;
+      }
+      const unsigned long long c = (unsigned long long)ci * kUnitCols + lane;
+      const uint32_t* poly = parts + (unsigned long long)part * cols + (c & ~(kEvD - 1ull));
+      const uint32_t x0 = __ldg(poly + lane), x1 = __ldg(poly + kUnitCols + lane);
+      uint32_t w[16];
+      chacha20_block(key, (uint32_t)c, part, w);  // 256 rows: column c is block c
+      const uint32_t n0 = x0 == 0 ? 0u : q - x0, n1 = x1 == 0 ? 0u : q - x1;
+      const uint32_t x = u0 ? x1 : x0, xn = u0 ? n1 : n0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        psum[i] += (x >> (8 * i)) & 0xFFu;
+        nsum[i] += (xn >> (8 * i)) & 0xFFu;
+      }
+      // the previous unit's MMAs must be done reading the tiles
+      if (!tiles_free(grp_empty, it, lane, err)) break;
+      ext[lane] = x0;
+      ext[32 + lane] = x1;
+      ext[64 + lane] = n0;
+      ext[96 + lane] = n1;
+      store_entries(at, w);
+      __syncwarp();
+      // row r of core matrix cm: words s'[u0 + 4 cm + r .. + 3]
+#pragma unroll
+      for (uint32_t i = lane; i < kEvCores * 8; i += 32) {
+        const uint32_t* src = ext + u0 + 4 * (i >> 3) + (i & 7);
+        *reinterpret_cast<uint4*>(bt + 16 * i) = make_uint4(src[0], src[1], src[2], src[3]);
+      }
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(grp_full);
+      part += step_part;
+      ci += step_ci;
+      if (ci >= per_part) {
+        ci -= per_part;
+        ++part;
+      }
+    }
+  }
+  __syncthreads();  // every MMA is done: the tiles' shared memory is free
+  // per-position byte sums of the coefficients and of their negations
+  for (int i = tid; i < 512; i += kEvThreads) sums[i] = 0;
+  __syncthreads();
+  if (warp < kEvWarps) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      psum[i] += (x >> (8 * i)) & 0xFFu;
-      nsum[i] += (xn >> (8 * i)) & 0xFFu;
+      atomicAdd(&sums[4 * (u0 + lane) + i], psum[i]);
+      atomicAdd(&sums[256 + 4 * (u0 + lane) + i], nsum[i]);
     }
-    // the previous chunk's MMAs must be done reading the tiles
-    if (it > 0) ok = __syncthreads_and(mbar_wait(bar, (it - 1) & 1, err));
-    if (!ok) break;
-    poly[tid] = x;
-    const uint32_t* lt = lut + lane;
-#pragma unroll
-    for (int g = 0; g < 16; ++g)
-      *reinterpret_cast<uint4*>(sm + jl_a_off(16 * g, tid)) =
-          make_uint4(lt[(w[g] & 0xFFu) << 5], lt[((w[g] >> 8) & 0xFFu) << 5],
-                     lt[((w[g] >> 16) & 0xFFu) << 5], lt[(w[g] >> 24) << 5]);
-    __syncthreads();  // the chunk's polys are staged
-    // B column tid: s'[u + t] for t = 0 .. 63, 16 bytes per group of 4 t
-    const uint32_t* pw = poly + (tid & ~(kEvD - 1));
-#pragma unroll
-    for (int g = 0; g < 16; ++g) {
-      uint32_t v4[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t pos = u + 4 * g + k;
-        const uint32_t s = pw[pos & (kEvD - 1)];
-        v4[k] = pos < (uint32_t)kEvD ? s : (s == 0 ? 0u : q - s);
-      }
-      *reinterpret_cast<uint4*>(sm + kTcA + (tid >> 3) * 2048 + g * 128 + (tid & 7) * 16) =
-          make_uint4(v4[0], v4[1], v4[2], v4[3]);
-    }
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc::fence_after_sync();
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int ks = 0; ks < kTcCols / 32; ++ks)
-          tc::mma_u8(tbase + 256 * h, tc::smem_desc(s0 + h * 1024 + ks * 8192, 2048, 128),
-                     tc::smem_desc(s0 + kTcA + ks * 8192, 2048, 128), idesc,
-                     (it | (uint32_t)ks) != 0);
-      tc::mma_commit(bar);
-    }
-  }
-  if (ok && it > 0) ok = mbar_wait(bar, (it - 1) & 1, err);
-  ok = __syncthreads_and(ok);
-  // per-position byte sums of the coefficients and of their negations
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    atomicAdd(&sums[4 * u + i], psum[i]);
-    atomicAdd(&sums[256 + 4 * u + i], nsum[i]);
   }
   __syncthreads();
-  {
+  if (tid < 4 * kEvD) {
     // S[t][i] = sum_{v >= t} P[v][i] + sum_{v < t} N[v][i], thread (t, i) = (tid / 4, tid % 4)
     const int t = tid >> 2, i = tid & 3;
     uint32_t acc = 0;
@@ -553,39 +657,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) jl_eval_tc_kernel(
   }
   __syncthreads();
   tc::fence_after_sync();
-  if (ok && it > 0) {
-    const int h = warp >> 2, wl = warp & 3;
-    const int row = 128 * h + 32 * wl + lane;
+  if (warp < 16 && first(0) < nunits) {
+    // warp: lane quarter warp % 4 of half (warp / 4) % 2, 32 of the 64 coefficients
+    const int h = (warp >> 2) & 1, wl = warp & 3, tbeg = 32 * (warp >> 3);
+    const int row = tile_row_to_row(128 * h + 32 * wl + lane);
     const uint32_t base = tc::tmem_addr(tbase, 32 * wl, 256 * h);
 #pragma unroll 1
-    for (int t0 = 0; t0 < kEvD; t0 += 2) {
+    for (int t0 = tbeg; t0 < tbeg + 32; t0 += 2) {
       uint32_t dv[8];
       tc::tmem_ld8(base + 4 * t0, dv);
       tc::tmem_ld_wait();
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int t = t0 + k;
-        long long v = 0;
+      for (int i = 0; i < 8; ++i) dv[i] = unscale(dv[i], lane);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          v += ((long long)dv[4 * k + i] - (long long)corr[4 * t + i]) << (8 * i);
-        long long r = v % (long long)q;
-        if (r < 0) r += q;
-        atomicAdd(&gsum[(size_t)row * kEvD + t], (unsigned long long)r);
+      for (int k = 0; k < 2; ++k) {
+        const long long v = weigh(dv + 4 * k, corr + 4 * (t0 + k));
+        atomicAdd(&gsum[(size_t)row * kEvD + t0 + k],
+                  (unsigned long long)(fold ? (long long)residue(v, q) : v));
       }
     }
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, 512);
+  if (warp == kEvWarps) tc::tmem_dealloc(tbase, 512);
 }
 
-__global__ void jl_eval_finish_kernel(const unsigned long long* __restrict__ gsum,
-                                      uint32_t* __restrict__ evals, size_t n, uint32_t q) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    evals[i] = (uint32_t)(gsum[i] % q);
+// Grid of a unit kernel: every SM (or every unit, if fewer), and more CTAs (they
+// queue) where one would accumulate past its bound. False if the units do not fit
+// 32-bit indices.
+bool unit_grid(unsigned long long nunits, int warps, int num_sms, unsigned* grid) {
+  const unsigned long long per_cta = kMaxUnitsPerCta / warps * warps;
+  unsigned long long g =
+      std::max((unsigned long long)num_sms, (nunits + per_cta - 1) / per_cta);
+  g = std::min(g, nunits);
+  if (nunits + g * warps >= (1ull << 32)) return false;
+  *grid = (unsigned)g;
+  return true;
 }
+
+// Signed 64-bit sums over all columns stay exact without a reduction per CTA while
+// columns * 255 * (1 + 2^8 + 2^16 + 2^24) < 2^63.
+bool must_fold(unsigned long long columns) { return columns >= (1ull << 30); }
 
 }  // namespace
 
@@ -599,90 +711,49 @@ int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
       num_parts > 0xFFFFFFFFull)
     return GRID_ERR_INVALID_PARAMETERS;
   if (scratch_bytes < jl_scratch_bytes(rows, num_parts, num_sms)) return GRID_ERR_INVALID_PARAMETERS;
-  ChachaKey key;
-  for (int i = 0; i < 8; ++i)
-    key.k[i] = (uint32_t)seed[4 * i] | ((uint32_t)seed[4 * i + 1] << 8) |
-               ((uint32_t)seed[4 * i + 2] << 16) | ((uint32_t)seed[4 * i + 3] << 24);
+  const ChachaKey key = chacha::make_key(seed);
   const int packed_len = (int)((rows + 3) / 4);
-  unsigned long long* gpos = static_cast<unsigned long long*>(scratch);
-  unsigned long long* gneg = gpos + rows;
-  cudaError_t e = cudaMemsetAsync(gpos, 0, 2 * rows * sizeof(unsigned long long), s);
+  unsigned long long* gsum = static_cast<unsigned long long*>(scratch);
+  cudaError_t e = cudaMemsetAsync(gsum, 0, rows * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return cuda_status(e);
-  static int tc_bps_whole[kMaxDevices] = {}, tc_bps_part[kMaxDevices] = {},
-             tc_bps_flat[kMaxDevices] = {};
-  int dev = 0, bps = 0;
   // the int8 entries come out of the projection kernel itself when the
-  // columns split into 32 polynomials x 8 coefficients and rows fill the blocks
+  // columns split into 32 polynomials per coefficient and rows fill the blocks
   const unsigned long long npoly = cols / d;
   const bool fused_flat = flat_out && packed_len == 64 && d % 8 == 0 && npoly % 32 == 0 &&
                           (reinterpret_cast<uintptr_t>(flat_out) & 3u) == 0;
-  const unsigned long long tc_per_part =
-      fused_flat ? npoly / 32 * (d / 8) : (cols + kTcCols - 1) / kTcCols;
-  const unsigned long long tc_chunks = tc_per_part * num_parts;
-  bool use_tc = cols > 0 && cudaGetDevice(&dev) == cudaSuccess &&
-                (fused_flat ? prepare_kernel(jl_tc_kernel<true, true>, kTcSmem, kTcThreads, dev,
-                                             tc_bps_flat, &bps)
-                 : packed_len == 64
-                     ? prepare_kernel(jl_tc_kernel<true>, kTcSmem, kTcThreads, dev, tc_bps_whole,
-                                      &bps)
-                     : prepare_kernel(jl_tc_kernel<false>, kTcSmem, kTcThreads, dev, tc_bps_part,
-                                      &bps)) == GRID_OK;
-  // Resident CTAs per SM: the occupancy query has reported 1 for this kernel
-  // where shared memory admits 3 (measured 20 % slower), so take the larger of
-  // it and what the SM's shared memory holds. The grid-stride chunk loop makes
-  // any count correct.
-  static int smem_bps[kMaxDevices] = {};
-  if (use_tc && smem_bps[dev] == 0) {
-    int per_sm = 0, reserved = 0;
-    if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
-            cudaSuccess ||
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) !=
-            cudaSuccess)
-      per_sm = 0;
-    const int fit = per_sm / (int)(kTcSmem + (uint32_t)reserved);
-    smem_bps[dev] = std::max(1, std::min(fit, 2048 / kTcThreads));
-  }
-  if (use_tc) bps = std::max(bps, smem_bps[dev]);
-  unsigned long long tc_grid = (unsigned long long)num_sms * (unsigned long long)(bps > 0 ? bps : 1);
-  if (tc_grid > tc_chunks) tc_grid = tc_chunks;
-  // exactness bound of the int32 accumulators: columns per CTA
-  if (use_tc && tc_grid > 0 &&
-      (tc_chunks + tc_grid - 1) / tc_grid * (unsigned long long)kTcCols > kTcMaxColsPerCta)
-    use_tc = false;
+  const unsigned long long per_part =
+      fused_flat ? npoly / 32 * d : (cols + kUnitCols - 1) / kUnitCols;
   const unsigned long long plane = (unsigned long long)num_parts * cols;  // flat bytes per row
-  if (use_tc) {
-    if (fused_flat)
-      jl_tc_kernel<true, true><<<(unsigned)tc_grid, kTcThreads, kTcSmem, s>>>(
-          parts, cols, (int)rows, packed_len, key, tc_chunks, tc_per_part, (int)d, plane,
-          flat_out, gpos, f.q, err);
-    else if (packed_len == 64)
-      jl_tc_kernel<true><<<(unsigned)tc_grid, kTcThreads, kTcSmem, s>>>(
-          parts, cols, (int)rows, packed_len, key, tc_chunks, tc_per_part, (int)d, plane,
-          nullptr, gpos, f.q, err);
-    else
-      jl_tc_kernel<false><<<(unsigned)tc_grid, kTcThreads, kTcSmem, s>>>(
-          parts, cols, (int)rows, packed_len, key, tc_chunks, tc_per_part, (int)d, plane,
-          nullptr, gpos, f.q, err);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e);
-  } else if (cols > 0) {
-    const unsigned long long chunks = (cols + 31) / 32 * num_parts;
-    unsigned long long blocks = (chunks + kJlWarps - 1) / kJlWarps;
-    const unsigned long long cap = (unsigned long long)num_sms * 8;
-    if (blocks > cap) blocks = cap;
-    if (packed_len == 64)
-      jl_project_kernel<true><<<(unsigned)blocks, kJlThreads, 0, s>>>(
-          parts, cols, (int)num_parts, (int)rows, packed_len, key, gpos, gneg, f.q);
-    else
-      jl_project_kernel<false><<<(unsigned)blocks, kJlThreads, 0, s>>>(
-          parts, cols, (int)num_parts, (int)rows, packed_len, key, gpos, gneg, f.q);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e);
+  if (cols > 0) {
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
+    auto run = [&](auto kernel, auto shape, int* cache) -> int {
+      using S = decltype(shape);
+      unsigned grid = 0;
+      if (per_part > (0xFFFFFFFFull / num_parts) ||
+          !unit_grid(per_part * num_parts, S::WARPS, num_sms, &grid))
+        return GRID_ERR_INVALID_PARAMETERS;
+      int bps = 0;
+      const int rc = prepare_kernel(kernel, S::SMEM, S::THREADS, dev, cache, &bps);
+      if (rc) return rc;
+      kernel<<<grid, S::THREADS, S::SMEM, s>>>(
+          parts, cols, (int)rows, packed_len, key, (uint32_t)(per_part * num_parts),
+          (uint32_t)per_part, (uint32_t)d, plane, fused_flat ? flat_out : nullptr, gsum, f.q,
+          must_fold(plane), err);
+      return cuda_status(cudaGetLastError());
+    };
+    static int cache_whole[kMaxDevices] = {}, cache_part[kMaxDevices] = {},
+               cache_flat[kMaxDevices] = {};
+    const int rc = fused_flat ? run(jl_tc_kernel<true, true>, PjShape<true>(), cache_flat)
+                   : packed_len == 64
+                       ? run(jl_tc_kernel<true>, PjShape<false>(), cache_whole)
+                       : run(jl_tc_kernel<false>, PjShape<false>(), cache_part);
+    if (rc) return rc;
   }
-  jl_finish_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(gpos, gneg, p_out, (int)rows, f.q);
+  jl_finish_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(gsum, p_out, (int)rows, f.q);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_status(e);
-  if (flat_out && cols > 0 && !(use_tc && fused_flat)) {
+  if (flat_out && cols > 0 && !fused_flat) {
     const unsigned long long n = cols / d;
     const unsigned long long work = (unsigned long long)num_parts * d * ((n + 127) / 128);
     unsigned long long blocks = (work + kJlWarps - 1) / kJlWarps;
@@ -713,32 +784,27 @@ int launch_jl_evals(const FieldParams& f, const uint8_t seed[32], size_t rows,
   if (cols == 0 || cols % d != 0 || num_parts == 0 || num_parts > 0xFFFFFFFFull)
     return GRID_ERR_INVALID_PARAMETERS;
   if (scratch_bytes < jl_evals_scratch_bytes()) return GRID_ERR_INVALID_PARAMETERS;
-  ChachaKey key;
-  for (int i = 0; i < 8; ++i)
-    key.k[i] = (uint32_t)seed[4 * i] | ((uint32_t)seed[4 * i + 1] << 8) |
-               ((uint32_t)seed[4 * i + 2] << 16) | ((uint32_t)seed[4 * i + 3] << 24);
+  const ChachaKey key = chacha::make_key(seed);
   unsigned long long* gsum = static_cast<unsigned long long*>(scratch);
   cudaError_t e = cudaMemsetAsync(gsum, 0, jl_evals_scratch_bytes(), s);
   if (e != cudaSuccess) return cuda_status(e);
-  const unsigned long long nchunks = (cols + kTcCols - 1) / kTcCols * num_parts;
-  // one CTA per SM (all 512 tensor-memory columns); more CTAs only where a CTA
-  // would see more than kTcMaxColsPerCta columns (they queue for an SM)
-  unsigned long long grid = (unsigned long long)num_sms;
-  const unsigned long long need = (nchunks * kTcCols + kTcMaxColsPerCta - 1) / kTcMaxColsPerCta;
-  if (grid < need) grid = need;
-  if (grid > nchunks) grid = nchunks;
-  if (grid > 0x7FFFFFFFull) return GRID_ERR_INVALID_PARAMETERS;
+  const unsigned long long per_part = cols / kUnitCols;  // d = 64: a whole, even number
+  unsigned grid = 0;
+  if (per_part > (0xFFFFFFFFull / num_parts) ||
+      !unit_grid(per_part * num_parts, kEvWarps, num_sms, &grid))
+    return GRID_ERR_INVALID_PARAMETERS;
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
   static int bps_cache[kMaxDevices] = {};
   int bps = 0;
-  int rc = prepare_kernel(jl_eval_tc_kernel, kEvSmem, kTcThreads, dev, bps_cache, &bps);
+  int rc = prepare_kernel(jl_eval_tc_kernel, kEvSmem, kEvThreads, dev, bps_cache, &bps);
   if (rc) return rc;
-  jl_eval_tc_kernel<<<(unsigned)grid, kTcThreads, kEvSmem, s>>>(parts, cols, key, nchunks, gsum,
-                                                               f.q, err);
+  jl_eval_tc_kernel<<<grid, kEvThreads, kEvSmem, s>>>(
+      parts, cols, key, (uint32_t)(per_part * num_parts), (uint32_t)per_part, gsum, f.q,
+      must_fold((unsigned long long)num_parts * cols), err);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
-  const size_t n = (size_t)kEvRows * kEvD;
-  jl_eval_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gsum, evals, n, f.q);
+  const int n = kEvRows * kEvD;
+  jl_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gsum, evals, n, f.q);
   return cuda_status(cudaGetLastError());
 }
 
