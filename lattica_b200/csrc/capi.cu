@@ -21,14 +21,13 @@ bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, size_t ldy, i
   return ntt_tc_available(p) && emm_pm_geometry(p, (int)M, (int)N, (int)K, (int)ldy, mode, &g);
 }
 
-// Workspace layouts. On a ring plan without an NTT for q (is_crt) a call
-// lifts its inputs into one residue buffer per auxiliary prime in turn (reused),
-// keeps the three residue results, and runs the prime's own call in the rest of
-// the workspace (reused across the primes); the reconstruction writes the output.
+// Workspace layouts. On a ring plan without an NTT for q (is_crt) a call runs the
+// prime's own call for each auxiliary prime in turn, on the inputs as they are (the
+// forward transforms reduce any 32-bit words, ring_crt.cu) and in the same workspace,
+// and keeps the three residue results; the reconstruction writes the output.
 size_t commit_ws_bytes(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
   if (is_crt(p))
-    return words_bytes(batch * cols * p->d) + 3 * words_bytes(batch * rows * p->d) +
-           commit_ws_bytes(p->crt[0], rows, cols, batch);
+    return 3 * words_bytes(batch * rows * p->d) + commit_ws_bytes(p->crt[0], rows, cols, batch);
   return words_bytes(batch * cols * p->d) +
          words_bytes(emm_workspace_words(p, (int)batch, (int)rows, (int)cols, EMM_DENSE));
 }
@@ -64,13 +63,6 @@ size_t round_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa, 
                    : base;
 }
 
-// x mod p_j into dst (the j-th auxiliary prime only)
-int lift_one(const grid_gpu_plan* p, int j, const uint32_t* x, size_t words, uint32_t* dst,
-             cudaStream_t st) {
-  return crt_lift(p, x, words, j == 0 ? dst : nullptr, j == 1 ? dst : nullptr,
-                  j == 2 ? dst : nullptr, st);
-}
-
 bool dims_ok(size_t a, size_t b, size_t c) {
   // all kernels index rows/cols/K with int
   return a > 0 && b > 0 && c > 0 && a < (1u << 30) && b < (1u << 30) && c < (1u << 30);
@@ -88,20 +80,40 @@ bool square_dims_ok(const grid_gpu_plan* p, size_t r, size_t n) {
   return dims_ok(r, n, 1) && words_fit(r, n, p->d) && words_fit(r, r, p->d);
 }
 
+// The evaluations of matrix m (plan, shape and ld set) from A, and, where products on
+// the TMA-fed tensor-core kernel apply, their point-major copy in the same allocation.
+int prepare_evals(grid_gpu_matrix* m, const uint32_t* A, bool a_is_evals, cudaStream_t st) {
+  const grid_gpu_plan* p = m->plan;
+  const size_t polys = m->rows * m->cols, words = polys * p->d;
+  EmmPmGeometry pg;
+  const bool pm = ntt_tc_available(p) && emm_pm_geometry(p, 1, (int)m->rows, (int)m->cols,
+                                                         (int)m->cols, EMM_DENSE, &pg);
+  const size_t part = words_bytes(words);
+  int rc = cuda_status(cudaMalloc(&m->d_evals, pm ? part + words * 4 : words * 4));
+  if (rc) return rc;
+  if (a_is_evals)
+    rc = cuda_status(cudaMemcpyAsync(m->d_evals, A, words * 4, cudaMemcpyDeviceToDevice, st));
+  else
+    rc = launch_ntt(p, MODE_FWD, A, nullptr, m->d_evals, polys, st);
+  if (!rc && pm) {
+    m->d_evals_pm = m->d_evals + part / 4;
+    rc = launch_to_point_major(m->d_evals, m->d_evals_pm, polys, (int)p->d, st);
+  }
+  return rc;
+}
+
 // t = A * s for `batch` vectors, into t (coefficients). ws from a Carver.
 int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint32_t* t,
                 Carver& cv, cudaStream_t st) {
   const grid_gpu_plan* p = A->plan;
   if (is_crt(p)) {
     if (!crt_bound_ok(p, A->cols)) return GRID_ERR_INVALID_PARAMETERS;
-    const size_t sw = batch * A->cols * p->d, tw = batch * A->rows * p->d;
-    uint32_t* sj = cv.take<uint32_t>(sw);
+    const size_t tw = batch * A->rows * p->d;
     uint32_t* tj[3] = {cv.take<uint32_t>(tw), cv.take<uint32_t>(tw), cv.take<uint32_t>(tw)};
     if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
     const size_t mark = cv.used;
     for (int j = 0; j < 3; ++j) {
-      int rc = lift_one(p, j, s, sw, sj, st);
-      if (!rc) rc = commit_core(A->crt[j], sj, batch, tj[j], cv, st);
+      const int rc = commit_core(A->crt[j], s, batch, tj[j], cv, st);
       if (rc) return rc;
       cv.used = mark;  // the next prime reuses the same workspace
     }
@@ -150,10 +162,9 @@ int grid_gpu_matrix_create_dev(grid_gpu_plan* p, const uint32_t* A, size_t rows,
   m->cols = cols;
   m->ld = cols;
   cudaStream_t st = (cudaStream_t)stream;
+  int rc = GRID_OK;
   if (is_crt(p)) {
-    // residues mod each auxiliary prime, prepared (transformed) on its plan
-    const size_t words = rows * cols * p->d;
-    int rc = GRID_OK;
+    // the matrix mod each auxiliary prime, prepared (transformed) on its plan
     for (int j = 0; j < 3 && !rc; ++j) {
       grid_gpu_matrix* sub = new (std::nothrow) grid_gpu_matrix();
       if (!sub) {
@@ -165,36 +176,10 @@ int grid_gpu_matrix_create_dev(grid_gpu_plan* p, const uint32_t* A, size_t rows,
       sub->rows = rows;
       sub->cols = cols;
       sub->ld = cols;
-      rc = cuda_status(cudaMalloc(&sub->d_evals, words * 4));
-      if (!rc) rc = lift_one(p, j, A, words, sub->d_evals, st);
-      if (!rc) rc = launch_ntt(sub->plan, MODE_FWD, sub->d_evals, nullptr, sub->d_evals,
-                               rows * cols, st);
+      rc = prepare_evals(sub, A, false, st);
     }
-    if (rc) {
-      grid_gpu_matrix_destroy(m);
-      return rc;
-    }
-    *out = m;
-    return GRID_OK;
-  }
-  cudaError_t e = cudaMalloc(&m->d_evals, rows * cols * p->d * 4);
-  if (e != cudaSuccess) {
-    delete m;
-    return cuda_status(e);
-  }
-  int rc;
-  if (a_is_evals) {
-    rc = cuda_status(cudaMemcpyAsync(m->d_evals, A, rows * cols * p->d * 4,
-                                     cudaMemcpyDeviceToDevice, st));
   } else {
-    rc = launch_ntt(p, MODE_FWD, A, nullptr, m->d_evals, rows * cols, st);
-  }
-  // a point-major copy for products on the TMA-fed tensor-core kernel
-  EmmPmGeometry pg;
-  if (!rc && ntt_tc_available(p) &&
-      emm_pm_geometry(p, 1, (int)rows, (int)cols, (int)cols, EMM_DENSE, &pg)) {
-    rc = cuda_status(cudaMalloc(&m->d_evals_pm, rows * cols * p->d * 4));
-    if (!rc) rc = launch_to_point_major(m->d_evals, m->d_evals_pm, rows * cols, (int)p->d, st);
+    rc = prepare_evals(m, A, a_is_evals != 0, st);
   }
   if (rc) {
     grid_gpu_matrix_destroy(m);
@@ -231,7 +216,6 @@ int grid_gpu_matrix_destroy(grid_gpu_matrix* m) {
   for (grid_gpu_matrix* sub : m->crt)
     if (sub) grid_gpu_matrix_destroy(sub);
   if (m->owned && m->d_evals) cudaFree(m->d_evals);
-  if (m->owned && m->d_evals_pm) cudaFree(m->d_evals_pm);
   delete m;
   return GRID_OK;
 }
@@ -500,10 +484,7 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
   for (int j = 0; j < (is_crt(p) ? 3 : 1) && !rc; ++j) {
     const grid_gpu_plan* q = is_crt(p) ? p->crt[j] : p;
     uint32_t* out = is_crt(p) ? gj[j] : G;
-    if (is_crt(p)) {
-      rc = lift_one(p, j, S, r * n * p->d, s_hat, st);
-      if (!rc) rc = launch_ntt(q, MODE_FWD, s_hat, nullptr, s_hat, r * n, st);
-    } else if (pm_fits(q, r, r, n, n, EMM_UPPER)) {
+    if (pm_fits(q, r, r, n, n, EMM_UPPER)) {
       rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, st);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_UPPER, out, work,
@@ -566,44 +547,42 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
   const size_t ew = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_DENSE);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
+  uint32_t* cj[3] = {};
+  if (is_crt(p)) {
+    if (!crt_bound_ok(p, n)) return GRID_ERR_INVALID_PARAMETERS;
+    for (auto& x : cj) x = cv.take<uint32_t>(r * r * p->d);
+  }
+  if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+  // out[i][j] = <phi_i, s_j> in plan q's evaluation domain
+  auto cross_products = [&](const grid_gpu_plan* q, uint32_t* out) {
+    if (pm_fits(q, r, r, n, n, EMM_DENSE)) {
+      int rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, st);
+      if (!rc) rc = launch_ntt_tc(q, MODE_FWD_PM, Phi, nullptr, phi_hat, r * n, st);
+      if (!rc)
+        rc = launch_emm_pm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, out, work,
+                           st);
+      return rc;
+    }
+    int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
+    if (!rc) rc = launch_ntt(q, MODE_FWD, Phi, nullptr, phi_hat, r * n, st);
+    if (!rc)
+      rc = launch_emm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, out, work, st);
+    return rc;
+  };
   if (!is_crt(p)) {
-    if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-    // cross[i][j] = <phi_i, s_j>
-    const bool pm = pm_fits(p, r, r, n, n, EMM_DENSE);
-    const int fwd = pm ? MODE_FWD_PM : MODE_FWD;
-    int rc = pm ? launch_ntt_tc(p, fwd, S, nullptr, s_hat, r * n, st)
-                : launch_ntt(p, fwd, S, nullptr, s_hat, r * n, st);
-    if (!rc)
-      rc = pm ? launch_ntt_tc(p, fwd, Phi, nullptr, phi_hat, r * n, st)
-              : launch_ntt(p, fwd, Phi, nullptr, phi_hat, r * n, st);
-    if (!rc)
-      rc = pm ? launch_emm_pm(p, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, cross,
-                              work, st)
-              : launch_emm(p, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, cross,
-                           work, st);
+    int rc = cross_products(p, cross);
     if (!rc) rc = launch_symmetrize_half(p, cross, (int)r, H, st);
     if (rc) return rc;
     return launch_ntt(p, MODE_INV, H, nullptr, H, r * (r + 1) / 2, st);
   }
   // ring plan without an NTT for q: the cross products per auxiliary prime,
   // back to coefficients, reconstructed mod q; then the (linear) symmetrisation
-  if (!crt_bound_ok(p, n)) return GRID_ERR_INVALID_PARAMETERS;
-  const size_t cw = r * r * p->d;
-  uint32_t* cj[3] = {cv.take<uint32_t>(cw), cv.take<uint32_t>(cw), cv.take<uint32_t>(cw)};
-  if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
   int rc = GRID_OK;
   for (int j = 0; j < 3 && !rc; ++j) {
-    const grid_gpu_plan* q = p->crt[j];
-    rc = lift_one(p, j, S, r * n * p->d, s_hat, st);
-    if (!rc) rc = lift_one(p, j, Phi, r * n * p->d, phi_hat, st);
-    if (!rc) rc = launch_ntt(q, MODE_FWD, s_hat, nullptr, s_hat, r * n, st);
-    if (!rc) rc = launch_ntt(q, MODE_FWD, phi_hat, nullptr, phi_hat, r * n, st);
-    if (!rc)
-      rc = launch_emm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, cj[j], work,
-                      st);
-    if (!rc) rc = launch_ntt(q, MODE_INV, cj[j], nullptr, cj[j], r * r, st);
+    rc = cross_products(p->crt[j], cj[j]);
+    if (!rc) rc = launch_ntt(p->crt[j], MODE_INV, cj[j], nullptr, cj[j], r * r, st);
   }
-  if (!rc) rc = crt_combine(p, cj[0], cj[1], cj[2], cw, cross, st);
+  if (!rc) rc = crt_combine(p, cj[0], cj[1], cj[2], r * r * p->d, cross, st);
   if (!rc) rc = launch_symmetrize_half(p, cross, (int)r, H, st);
   return rc;
 }
@@ -668,10 +647,8 @@ int grid_gpu_amortize_dev(const grid_gpu_plan* p, const uint32_t* S, const uint3
   int rc = GRID_OK;
   for (int j = 0; j < 3 && !rc; ++j) {
     const grid_gpu_plan* q = p->crt[j];
-    rc = lift_one(p, j, S, r * n * p->d, s_hat, st);
-    if (!rc) rc = lift_one(p, j, c, r * p->d, c_hat, st);
-    if (!rc) rc = launch_ntt(q, MODE_FWD, s_hat, nullptr, s_hat, r * n, st);
-    if (!rc) rc = launch_ntt(q, MODE_FWD, c_hat, nullptr, c_hat, r, st);
+    rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
+    if (!rc) rc = launch_ntt(q, MODE_FWD, c, nullptr, c_hat, r, st);
     if (!rc) rc = launch_amortize(q, c_hat, s_hat, (int)r, n, zj[j], st);
     if (!rc) rc = launch_ntt(q, MODE_INV, zj[j], nullptr, zj[j], n, st);
   }
@@ -946,12 +923,12 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
   // inner commitments and the Gram over the witness's evaluations (one
   // transform shared by both) on plan q into tt / gg
-  auto contract = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq, const uint32_t* src,
-                      uint32_t* tt, uint32_t* gg, cudaStream_t cs) {
-    if (src != s_hat && Aq->d_evals_pm && pm_fits(q, r, kappa, n, Aq->ld, EMM_DENSE) &&
+  auto contract = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq, uint32_t* tt,
+                      uint32_t* gg, cudaStream_t cs) {
+    if (Aq->d_evals_pm && pm_fits(q, r, kappa, n, Aq->ld, EMM_DENSE) &&
         pm_fits(q, r, r, n, n, EMM_UPPER)) {
       // point-major evaluations: both products load their operands with TMA
-      int rc = launch_ntt_tc(q, MODE_FWD_PM, src, nullptr, s_hat, r * n, cs);
+      int rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, cs);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, Aq->d_evals_pm, (int)r, (int)kappa, (int)n, (int)Aq->ld,
                            EMM_DENSE, tt, work, cs);
@@ -962,7 +939,7 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
       if (!rc) rc = launch_ntt(q, MODE_INV, gg, nullptr, gg, r * (r + 1) / 2, cs);
       return rc;
     }
-    int rc = launch_ntt(q, MODE_FWD, src, nullptr, s_hat, r * n, cs);
+    int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, cs);
     if (!rc)
       rc = launch_emm(q, s_hat, Aq->d_evals, (int)r, (int)kappa, (int)n, (int)Aq->ld, EMM_DENSE,
                       tt, work, cs);
@@ -993,12 +970,10 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
                                 jl_scratch_bytes(jl_rows, 0, 0), p->num_sms, p->d_err, lo);
     // 1. inner commitments t_i = A s_i and 2. garbage g_ij = <s_i, s_j>, i <= j
     if (!is_crt(p)) {
-      rc_chain = contract(p, A, S, t, g, hi);
+      rc_chain = contract(p, A, t, g, hi);
     } else {
-      for (int j = 0; j < 3 && !rc_chain; ++j) {
-        rc_chain = lift_one(p, j, S, r * n * d, s_hat, hi);
-        if (!rc_chain) rc_chain = contract(p->crt[j], A->crt[j], s_hat, tj[j], gj[j], hi);
-      }
+      for (int j = 0; j < 3 && !rc_chain; ++j)
+        rc_chain = contract(p->crt[j], A->crt[j], tj[j], gj[j], hi);
       if (!rc_chain) rc_chain = crt_combine(p, tj[0], tj[1], tj[2], tw, t, hi);
       if (!rc_chain) rc_chain = crt_combine(p, gj[0], gj[1], gj[2], gw, g, hi);
     }

@@ -102,7 +102,8 @@ struct grid_gpu_matrix {
   size_t ld = 0;                // row stride in polys (cols of the owning matrix)
   uint32_t* d_evals = nullptr;  // rows x ld polys in the twisted evaluation domain
   // The same evaluations point-major, [d][rows][ld], for the tensor-core
-  // contraction over TMA-loaded operands (null where that path does not apply).
+  // contraction over TMA-loaded operands (null where that path does not apply; in
+  // d_evals' allocation).
   uint32_t* d_evals_pm = nullptr;
   bool owned = true;            // false for views sharing another matrix's evaluations
   // On a ring plan without an NTT for q: the matrix's residues mod each
@@ -218,9 +219,6 @@ void crt_consts(uint32_t q, CrtConsts* c);
 // terms * d * (q - 1)^2 < 2^93: every output coefficient sums at most terms * d
 // word products, within the reconstruction's range
 bool crt_bound_ok(const grid_gpu_plan* p, size_t terms);
-// o_j = x mod p_j (null outputs skipped); words % 4 == 0, 16-byte aligned buffers
-int crt_lift(const grid_gpu_plan* p, const uint32_t* x, size_t words, uint32_t* o0, uint32_t* o1,
-             uint32_t* o2, cudaStream_t s);
 // out = Montgomery word mod q of the integer whose words mod p_j are w_j
 int crt_combine(const grid_gpu_plan* p, const uint32_t* w0, const uint32_t* w1,
                 const uint32_t* w2, size_t words, uint32_t* out, cudaStream_t s);

@@ -292,7 +292,7 @@ size_t crt_poly_words(const grid_gpu_plan* p, size_t npolys) {
 }
 
 // Negacyclic products on a ring plan without an NTT for q: per auxiliary
-// prime, lift a and b, transform b, multiply and invert; then reconstruct.
+// prime, transform b, multiply by a's transform and invert; then reconstruct.
 // scratch: 4 * crt_poly_words words.
 int crt_poly_mul(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_t* out,
                  uint32_t* scratch, size_t npolys, cudaStream_t s) {
@@ -303,13 +303,8 @@ int crt_poly_mul(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, u
   int rc = GRID_OK;
   for (int j = 0; j < 3 && !rc; ++j) {
     const grid_gpu_plan* sub = p->crt[j];
-    rc = crt_lift(p, a, w, j == 0 ? aj[0] : nullptr, j == 1 ? aj[1] : nullptr,
-                  j == 2 ? aj[2] : nullptr, s);
-    if (!rc)
-      rc = crt_lift(p, b, w, j == 0 ? bt : nullptr, j == 1 ? bt : nullptr, j == 2 ? bt : nullptr,
-                    s);
-    if (!rc) rc = launch_ntt(sub, MODE_FWD, bt, nullptr, bt, npolys, s);
-    if (!rc) rc = launch_ntt(sub, MODE_MULINV, aj[j], bt, aj[j], npolys, s);
+    rc = launch_ntt(sub, MODE_FWD, b, nullptr, bt, npolys, s);
+    if (!rc) rc = launch_ntt(sub, MODE_MULINV, a, bt, aj[j], npolys, s);
   }
   if (rc) return rc;
   return crt_combine(p, aj[0], aj[1], aj[2], w, out, s);

@@ -10,11 +10,13 @@
 //
 // A ring plan for such a q computes every contraction (commitments, Gram,
 // garbage h, amortization, single products) exactly over the integers:
-//  * input words x < q are lifted to residues modulo three auxiliary primes
-//    p_j = 1 (mod 512) just below 2^32 (x mod p_j is one conditional
-//    subtraction, since p_j > 2^31);
-//  * each residue problem runs on the NTT kernels of an ordinary plan for p_j,
-//    with the lifted words read as Montgomery words: its output words are
+//  * each residue problem, modulo three auxiliary primes p_j = 1 (mod 512) just
+//    below 2^32, runs on the NTT kernels of an ordinary plan for p_j, with the input
+//    words x < q read as Montgomery words as they are: every forward transform takes
+//    any 32-bit words (the tensor-core ones sum bytes times residues, below 2^16 p_j;
+//    the CUDA-core ones work on lazy words), so x need not be reduced mod p_j first
+//    (a reducing pass before each transform, and the gathering products it forced,
+//    cost the round of r = 64, n = 2048 at q = 2^32 - 5 868 us against 753). Its output words are
 //    w_j = V * 2^-32 mod p_j, where V is the exact integer sum of the word
 //    products with the negacyclic signs;
 //  * Garner's mixed-radix reconstruction x1 + p0 x2 + p0 p1 x3 recovers V in
@@ -59,21 +61,6 @@ uint32_t neg_inv32(uint32_t q) {  // q^-1 mod 2^32 (positive inverse, grid_field
   uint32_t x = 1;
   for (int i = 0; i < 5; ++i) x *= 2u - q * x;
   return x;
-}
-
-__global__ void crt_lift_kernel(const uint4* __restrict__ x, size_t n4, uint4* __restrict__ o0,
-                                uint4* __restrict__ o1, uint4* __restrict__ o2, uint3 p) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const uint4 v = x[i];
-    auto lift = [](uint4 w, uint32_t m) {
-      return make_uint4(w.x >= m ? w.x - m : w.x, w.y >= m ? w.y - m : w.y,
-                        w.z >= m ? w.z - m : w.z, w.w >= m ? w.w - m : w.w);
-    };
-    if (o0) o0[i] = lift(v, p.x);
-    if (o1) o1[i] = lift(v, p.y);
-    if (o2) o2[i] = lift(v, p.z);
-  }
 }
 
 __device__ __forceinline__ uint32_t crt_word(uint32_t w0, uint32_t w1, uint32_t w2,
@@ -151,18 +138,6 @@ bool crt_bound_ok(const grid_gpu_plan* p, size_t terms) {
   if (terms == 0) return true;
   if (t >> 40) return false;
   return t * q1 * q1 < ((unsigned __int128)1 << 93);
-}
-
-int crt_lift(const grid_gpu_plan* p, const uint32_t* x, size_t words, uint32_t* o0, uint32_t* o1,
-             uint32_t* o2, cudaStream_t s) {
-  if (words == 0) return GRID_OK;
-  if (words % 4) return GRID_ERR_INVALID_PARAMETERS;  // whole polynomials of d >= 8 words
-  const size_t n4 = words / 4;
-  crt_lift_kernel<<<grid_for(p, n4), 256, 0, s>>>(
-      reinterpret_cast<const uint4*>(x), n4, reinterpret_cast<uint4*>(o0),
-      reinterpret_cast<uint4*>(o1), reinterpret_cast<uint4*>(o2),
-      make_uint3(kAux[0], kAux[1], kAux[2]));
-  return cuda_status(cudaGetLastError());
 }
 
 int crt_combine(const grid_gpu_plan* p, const uint32_t* w0, const uint32_t* w1,
