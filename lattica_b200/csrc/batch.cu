@@ -325,7 +325,7 @@ int build_tables(const grid_gpu_plan* plan, grid_gpu_matrix* const* mats, size_t
     if (mats[i]->plan != plan) return GRID_ERR_INVALID_PARAMETERS;
     if (mats[i]->rows > (size_t)TN) return GRID_ERR_INVALID_PARAMETERS;  // ranks up to 32
     tb.mats.push_back(MatDev{mats[i]->d_evals, mats[i]->d_evals_pm, (uint32_t)mats[i]->rows,
-                             (uint32_t)mats[i]->ld});
+                             (uint32_t)mats[i]->ld, (uint32_t)mats[i]->ld_pm});
   }
   std::vector<std::pair<uint32_t, uint32_t>> order;  // (matrix, index)
   order.reserve(nitems);
@@ -339,12 +339,13 @@ int build_tables(const grid_gpu_plan* plan, grid_gpu_matrix* const* mats, size_t
     order.emplace_back(it.matrix, (uint32_t)i);
   }
   // The point-major engine needs the point-major forward transform (d = 64,
-  // tensor cores), every matrix's point-major evaluations, K ranges of whole
-  // chunks, and transform tiles whose source rows and destination columns
-  // stay below 2^31; AUTO takes it where those hold.
+  // tensor cores), every matrix's point-major evaluations over a multiple of four
+  // columns, K ranges of whole chunks, and transform tiles whose source rows and
+  // destination columns stay below 2^31; AUTO takes it where those hold.
   bool pm_ok = plan->pm_emm && ntt_tc_available(plan) && k_split % 32 == 0 &&
                tb.s_polys <= (uint64_t)INT32_MAX - 128 && tb.pm_polys <= (uint64_t)INT32_MAX - 128;
-  for (size_t i = 0; pm_ok && i < nmats; ++i) pm_ok = mats[i]->d_evals_pm != nullptr;
+  for (size_t i = 0; pm_ok && i < nmats; ++i)
+    pm_ok = mats[i]->d_evals_pm != nullptr && mats[i]->ld % 4 == 0;
   if (engine == GRID_GPU_ENGINE_POINT_MAJOR && !pm_ok) return GRID_ERR_UNSUPPORTED_DEGREE;
   tb.pm = engine == GRID_GPU_ENGINE_POINT_MAJOR || (engine == GRID_GPU_ENGINE_AUTO && pm_ok);
   tb.tc = tb.pm || engine_uses_tc(plan, engine);

@@ -19,8 +19,8 @@ constexpr uint32_t kUpperTile = 0xFFFFFFFFu;  // TileDev::matrix of a Gram tile
 
 struct MatDev {
   const uint32_t* evals;
-  const uint32_t* evals_pm;  // [point][row][ld] (point-major engine), or null
-  uint32_t rows, ld;         // ld: row stride in polys
+  const uint32_t* evals_pm;  // [point][row][ld_pm] (point-major engine), or null
+  uint32_t rows, ld, ld_pm;  // row strides in polys
 };
 struct ItemDev {
   unsigned long long s_off, t_off;

@@ -14,11 +14,11 @@ namespace {
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 // The forward transform stores the evaluations of M x K witness polys
-// point-major and the product with Y (N rows of row stride ldy) runs on the
-// TMA-fed tensor-core kernel (emm_pm.cu).
-bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, size_t ldy, int mode) {
+// point-major and the product with Y (N rows) runs on the TMA-fed tensor-core
+// kernel (emm_pm.cu).
+bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, int mode) {
   EmmPmGeometry g;
-  return ntt_tc_available(p) && emm_pm_geometry(p, (int)M, (int)N, (int)K, (int)ldy, mode, &g);
+  return ntt_tc_available(p) && emm_pm_geometry(p, (int)M, (int)N, (int)K, mode, &g);
 }
 
 // Workspace layouts. On a ring plan without an NTT for q (is_crt) a call runs the
@@ -28,20 +28,22 @@ bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, size_t ldy, i
 size_t commit_ws_bytes(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
   if (is_crt(p))
     return 3 * words_bytes(batch * rows * p->d) + commit_ws_bytes(p->crt[0], rows, cols, batch);
-  return words_bytes(batch * cols * p->d) +
+  return words_bytes(batch * pm_stride(cols) * p->d) +
          words_bytes(emm_workspace_words(p, (int)batch, (int)rows, (int)cols, EMM_DENSE));
 }
 
-size_t gram_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n) {
+// stride: polys per witness row of the evaluations (pm_stride(n), or n where only the
+// gathering products are to fit)
+size_t gram_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t stride) {
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
-  const size_t base = words_bytes(r * n * p->d) +
+  const size_t base = words_bytes(r * stride * p->d) +
                       words_bytes(emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER));
   return is_crt(p) ? base + 3 * words_bytes(r * (r + 1) / 2 * p->d) : base;
 }
 
 size_t garbage_h_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n) {
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
-  const size_t base = 2 * words_bytes(r * n * p->d) + words_bytes(r * r * p->d) +
+  const size_t base = 2 * words_bytes(r * pm_stride(n) * p->d) + words_bytes(r * r * p->d) +
                       words_bytes(emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_DENSE));
   return is_crt(p) ? base + 3 * words_bytes(r * r * p->d) : base;
 }
@@ -56,7 +58,7 @@ size_t round_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa, 
   const size_t d = p->d;
   const size_t e1 = emm_workspace_words(e, (int)r, (int)kappa, (int)n, EMM_DENSE);
   const size_t e2 = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
-  const size_t base = words_bytes(r * n * d) + words_bytes(e1 > e2 ? e1 : e2) +
+  const size_t base = words_bytes(r * pm_stride(n) * d) + words_bytes(e1 > e2 ? e1 : e2) +
                       words_bytes(r * kappa * d) +
                       round_up(jl_scratch_bytes(jl_rows ? jl_rows : 1, 0, 0), 256);
   return is_crt(p) ? base + 3 * (words_bytes(r * kappa * d) + words_bytes(r * (r + 1) / 2 * d))
@@ -85,11 +87,9 @@ bool square_dims_ok(const grid_gpu_plan* p, size_t r, size_t n) {
 int prepare_evals(grid_gpu_matrix* m, const uint32_t* A, bool a_is_evals, cudaStream_t st) {
   const grid_gpu_plan* p = m->plan;
   const size_t polys = m->rows * m->cols, words = polys * p->d;
-  EmmPmGeometry pg;
-  const bool pm = ntt_tc_available(p) && emm_pm_geometry(p, 1, (int)m->rows, (int)m->cols,
-                                                         (int)m->cols, EMM_DENSE, &pg);
-  const size_t part = words_bytes(words);
-  int rc = cuda_status(cudaMalloc(&m->d_evals, pm ? part + words * 4 : words * 4));
+  const bool pm = pm_fits(p, 1, m->rows, m->cols, EMM_DENSE);
+  const size_t part = words_bytes(words), ld = pm_stride(m->cols);
+  int rc = cuda_status(cudaMalloc(&m->d_evals, pm ? part + m->rows * ld * p->d * 4 : words * 4));
   if (rc) return rc;
   if (a_is_evals)
     rc = cuda_status(cudaMemcpyAsync(m->d_evals, A, words * 4, cudaMemcpyDeviceToDevice, st));
@@ -97,7 +97,8 @@ int prepare_evals(grid_gpu_matrix* m, const uint32_t* A, bool a_is_evals, cudaSt
     rc = launch_ntt(p, MODE_FWD, A, nullptr, m->d_evals, polys, st);
   if (!rc && pm) {
     m->d_evals_pm = m->d_evals + part / 4;
-    rc = launch_to_point_major(m->d_evals, m->d_evals_pm, polys, (int)p->d, st);
+    m->ld_pm = ld;
+    rc = launch_to_point_major(m->d_evals, m->d_evals_pm, m->rows, m->cols, ld, (int)p->d, st);
   }
   return rc;
 }
@@ -121,27 +122,34 @@ int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint3
   }
   if (commit_small_fits(p, A->rows, A->cols, batch))
     return launch_commit_small(p, A->d_evals, A->rows, A->cols, A->ld, s, batch, t, st);
-  uint32_t* s_hat = cv.take<uint32_t>(batch * A->cols * p->d);
+  const size_t ldx = pm_stride(A->cols);
+  uint32_t* s_hat = cv.take<uint32_t>(batch * ldx * p->d);
   const size_t ew = emm_workspace_words(p, (int)batch, (int)A->rows, (int)A->cols, EMM_DENSE);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
   int rc;
-  if (A->d_evals_pm && pm_fits(p, batch, A->rows, A->cols, A->ld, EMM_DENSE)) {
-    rc = launch_ntt_tc(p, MODE_FWD_PM, s, nullptr, s_hat, batch * A->cols, st);
-    if (!rc)
-      rc = launch_emm_pm(p, s_hat, A->d_evals_pm, (int)batch, (int)A->rows, (int)A->cols,
-                         (int)A->ld, EMM_DENSE, t, work, st);
-  } else {
-    rc = launch_ntt(p, MODE_FWD, s, nullptr, s_hat, batch * A->cols, st);
-    if (!rc)
-      rc = launch_emm(p, s_hat, A->d_evals, (int)batch, (int)A->rows, (int)A->cols, (int)A->ld,
-                      EMM_DENSE, t, work, st);
+  if (A->d_evals_pm && pm_fits(p, batch, A->rows, A->cols, EMM_DENSE)) {
+    rc = launch_ntt_tc_pm(p, s, batch, A->cols, s_hat, st);
+    if (rc) return rc;
+    return launch_emm_pm(p, s_hat, A->d_evals_pm, (int)batch, (int)A->rows, (int)A->cols, (int)ldx,
+                         (int)A->ld_pm, EMM_DENSE, false, t, work, st);
   }
+  rc = launch_ntt(p, MODE_FWD, s, nullptr, s_hat, batch * A->cols, st);
+  if (!rc)
+    rc = launch_emm(p, s_hat, A->d_evals, (int)batch, (int)A->rows, (int)A->cols, (int)A->ld,
+                    EMM_DENSE, t, work, st);
   if (rc) return rc;
   return launch_ntt(p, MODE_INV, t, nullptr, t, batch * A->rows, st);
 }
 
 }  // namespace
+
+int grid::gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes) {
+  if (!p || !bytes) return GRID_ERR_NULL_POINTER;
+  if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
+  *bytes = gram_ws_bytes(p, r, n, n);
+  return GRID_OK;
+}
 
 extern "C" {
 
@@ -232,6 +240,7 @@ int grid_gpu_matrix_view(const grid_gpu_matrix* parent, size_t cols, grid_gpu_ma
   m->ld = parent->ld;
   m->d_evals = parent->d_evals;
   m->d_evals_pm = parent->d_evals_pm;
+  m->ld_pm = parent->ld_pm;
   m->owned = false;
   for (int j = 0; j < 3; ++j)
     if (parent->crt[j]) {
@@ -459,7 +468,7 @@ int grid_gpu_bdlop_commit(grid_gpu_matrix* A_mask, grid_gpu_matrix* A_msg, grid_
 int grid_gpu_gram_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes) {
   if (!p || !bytes) return GRID_ERR_NULL_POINTER;
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
-  *bytes = gram_ws_bytes(p, r, n);
+  *bytes = gram_ws_bytes(p, r, n, pm_stride(n));
   return GRID_OK;
 }
 
@@ -472,8 +481,12 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
   if (is_crt(p) && !crt_bound_ok(p, n)) return GRID_ERR_INVALID_PARAMETERS;
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
   const size_t gw = r * (r + 1) / 2 * p->d;
+  // rows of whole 16-byte units where they fit the workspace (a caller with a fixed
+  // buffer may have room for the gathering products' layout only)
+  const bool padded = workspace_bytes >= gram_ws_bytes(p, r, n, pm_stride(n));
+  const size_t ldx = padded ? pm_stride(n) : n;
   Carver cv(workspace, workspace_bytes);
-  uint32_t* s_hat = cv.take<uint32_t>(r * n * p->d);
+  uint32_t* s_hat = cv.take<uint32_t>(r * ldx * p->d);
   const size_t ew = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   uint32_t* gj[3] = {};
@@ -484,16 +497,14 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
   for (int j = 0; j < (is_crt(p) ? 3 : 1) && !rc; ++j) {
     const grid_gpu_plan* q = is_crt(p) ? p->crt[j] : p;
     uint32_t* out = is_crt(p) ? gj[j] : G;
-    if (pm_fits(q, r, r, n, n, EMM_UPPER)) {
-      rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, st);
+    if (ldx % 4 == 0 && pm_fits(q, r, r, n, EMM_UPPER)) {
+      rc = launch_ntt_tc_pm(q, S, r, n, s_hat, st);
       if (!rc)
-        rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_UPPER, out, work,
-                           st);
-      if (!rc) rc = launch_ntt(q, MODE_INV, out, nullptr, out, r * (r + 1) / 2, st);
+        rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
+                           false, out, work, st);
       continue;
-    } else {
-      rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
     }
+    rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
     if (!rc)
       rc = launch_emm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_UPPER, out, work, st);
     if (!rc) rc = launch_ntt(q, MODE_INV, out, nullptr, out, r * (r + 1) / 2, st);
@@ -507,7 +518,7 @@ int grid_gpu_gram(grid_gpu_plan* p, const uint32_t* S, size_t r, size_t n, uint3
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
   std::lock_guard<std::mutex> lk(p->mu);
   const size_t s_bytes = r * n * p->d * 4, g_bytes = r * (r + 1) / 2 * p->d * 4;
-  const size_t ws = gram_ws_bytes(p, r, n);
+  const size_t ws = gram_ws_bytes(p, r, n, pm_stride(n));
   int rc;
   if ((rc = ensure_scratch(p, 6, s_bytes)) || (rc = ensure_scratch(p, 7, g_bytes)) ||
       (rc = ensure_scratch(p, 8, ws)))
@@ -541,8 +552,9 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     return GRID_ERR_MISALIGNED;
   cudaStream_t st = (cudaStream_t)stream;
   Carver cv(workspace, workspace_bytes);
-  uint32_t* s_hat = cv.take<uint32_t>(r * n * p->d);
-  uint32_t* phi_hat = cv.take<uint32_t>(r * n * p->d);
+  const size_t ldx = pm_stride(n);
+  uint32_t* s_hat = cv.take<uint32_t>(r * ldx * p->d);
+  uint32_t* phi_hat = cv.take<uint32_t>(r * ldx * p->d);
   uint32_t* cross = cv.take<uint32_t>(r * r * p->d);
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
   const size_t ew = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_DENSE);
@@ -553,16 +565,18 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     for (auto& x : cj) x = cv.take<uint32_t>(r * r * p->d);
   }
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-  // out[i][j] = <phi_i, s_j> in plan q's evaluation domain
-  auto cross_products = [&](const grid_gpu_plan* q, uint32_t* out) {
-    if (pm_fits(q, r, r, n, n, EMM_DENSE)) {
-      int rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, st);
-      if (!rc) rc = launch_ntt_tc(q, MODE_FWD_PM, Phi, nullptr, phi_hat, r * n, st);
-      if (!rc)
-        rc = launch_emm_pm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_DENSE, out, work,
-                           st);
-      return rc;
-    }
+  const bool pm = pm_fits(e, r, r, n, EMM_DENSE);
+  // point-major: <phi_i, s_j> through to coefficients, symmetrised if sym
+  auto cross_pm = [&](const grid_gpu_plan* q, bool sym, uint32_t* out) {
+    int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, st);
+    if (!rc) rc = launch_ntt_tc_pm(q, Phi, r, n, phi_hat, st);
+    if (!rc)
+      rc = launch_emm_pm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_DENSE,
+                         sym, out, work, st);
+    return rc;
+  };
+  // poly-major: out[i][j] = <phi_i, s_j> in plan q's evaluation domain
+  auto cross_evals = [&](const grid_gpu_plan* q, uint32_t* out) {
     int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
     if (!rc) rc = launch_ntt(q, MODE_FWD, Phi, nullptr, phi_hat, r * n, st);
     if (!rc)
@@ -570,7 +584,8 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     return rc;
   };
   if (!is_crt(p)) {
-    int rc = cross_products(p, cross);
+    if (pm) return cross_pm(p, true, H);
+    int rc = cross_evals(p, cross);
     if (!rc) rc = launch_symmetrize_half(p, cross, (int)r, H, st);
     if (rc) return rc;
     return launch_ntt(p, MODE_INV, H, nullptr, H, r * (r + 1) / 2, st);
@@ -579,8 +594,12 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
   // back to coefficients, reconstructed mod q; then the (linear) symmetrisation
   int rc = GRID_OK;
   for (int j = 0; j < 3 && !rc; ++j) {
-    rc = cross_products(p->crt[j], cj[j]);
-    if (!rc) rc = launch_ntt(p->crt[j], MODE_INV, cj[j], nullptr, cj[j], r * r, st);
+    if (pm) {
+      rc = cross_pm(p->crt[j], false, cj[j]);
+    } else {
+      rc = cross_evals(p->crt[j], cj[j]);
+      if (!rc) rc = launch_ntt(p->crt[j], MODE_INV, cj[j], nullptr, cj[j], r * r, st);
+    }
   }
   if (!rc) rc = crt_combine(p, cj[0], cj[1], cj[2], r * r * p->d, cross, st);
   if (!rc) rc = launch_symmetrize_half(p, cross, (int)r, H, st);
@@ -905,7 +924,8 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
   cudaStream_t st = (cudaStream_t)stream;
   const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
   Carver cv(workspace, workspace_bytes);
-  uint32_t* s_hat = cv.take<uint32_t>(r * n * d);
+  const size_t ldx = pm_stride(n);
+  uint32_t* s_hat = cv.take<uint32_t>(r * ldx * d);
   const size_t e1 = emm_workspace_words(e, (int)r, (int)kappa, (int)n, EMM_DENSE);
   const size_t e2 = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
   const size_t ew = e1 > e2 ? e1 : e2;
@@ -925,18 +945,15 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
   // transform shared by both) on plan q into tt / gg
   auto contract = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq, uint32_t* tt,
                       uint32_t* gg, cudaStream_t cs) {
-    if (Aq->d_evals_pm && pm_fits(q, r, kappa, n, Aq->ld, EMM_DENSE) &&
-        pm_fits(q, r, r, n, n, EMM_UPPER)) {
+    if (Aq->d_evals_pm && pm_fits(q, r, kappa, n, EMM_DENSE) && pm_fits(q, r, r, n, EMM_UPPER)) {
       // point-major evaluations: both products load their operands with TMA
-      int rc = launch_ntt_tc(q, MODE_FWD_PM, S, nullptr, s_hat, r * n, cs);
+      int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, cs);
       if (!rc)
-        rc = launch_emm_pm(q, s_hat, Aq->d_evals_pm, (int)r, (int)kappa, (int)n, (int)Aq->ld,
-                           EMM_DENSE, tt, work, cs);
-      if (!rc) rc = launch_ntt(q, MODE_INV, tt, nullptr, tt, r * kappa, cs);
+        rc = launch_emm_pm(q, s_hat, Aq->d_evals_pm, (int)r, (int)kappa, (int)n, (int)ldx,
+                           (int)Aq->ld_pm, EMM_DENSE, false, tt, work, cs);
       if (!rc)
-        rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)n, EMM_UPPER, gg, work,
-                           cs);
-      if (!rc) rc = launch_ntt(q, MODE_INV, gg, nullptr, gg, r * (r + 1) / 2, cs);
+        rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
+                           false, gg, work, cs);
       return rc;
     }
     int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, cs);

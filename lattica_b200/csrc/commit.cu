@@ -335,34 +335,39 @@ int launch_sum_splits(const grid_gpu_plan* p, const uint32_t* work, uint32_t* ou
 
 namespace {
 
-// out[e][i] = in[i][e]: 32 x 32 tiles through shared memory.
+// out[e][row][k] = in[row][k][e] for k < cols, 0 for cols <= k < ld: 32 x 32 tiles
+// (k, e) of one row through shared memory.
 __global__ void to_point_major_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                      size_t npolys, int d) {
+                                      size_t rows, size_t cols, size_t ld, int d) {
   __shared__ uint32_t t[32][33];
-  const size_t i0 = (size_t)blockIdx.x * 32;
+  const size_t k0 = (size_t)blockIdx.x * 32;
   const int e0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const size_t i = i0 + r;
-    const int e = e0 + threadIdx.x;
-    if (i < npolys && e < d) t[r][threadIdx.x] = in[i * d + e];
-  }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int e = e0 + r;
-    const size_t i = i0 + threadIdx.x;
-    if (i < npolys && e < d) out[(size_t)e * npolys + i] = t[threadIdx.x][r];
+  for (size_t row = blockIdx.z; row < rows; row += gridDim.z) {
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+      const size_t k = k0 + r;
+      const int e = e0 + threadIdx.x;
+      if (e < d) t[r][threadIdx.x] = k < cols ? in[(row * cols + k) * d + e] : 0u;
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+      const int e = e0 + r;
+      const size_t k = k0 + threadIdx.x;
+      if (k < ld && e < d) out[((size_t)e * rows + row) * ld + k] = t[threadIdx.x][r];
+    }
+    __syncthreads();
   }
 }
 
 }  // namespace
 
-int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t npolys, int d,
-                          cudaStream_t s) {
-  if (npolys == 0) return GRID_OK;
-  const size_t bx = (npolys + 31) / 32;
+int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t rows, size_t cols, size_t ld,
+                          int d, cudaStream_t s) {
+  const size_t bx = (ld + 31) / 32;
+  if (bx == 0 || rows == 0) return GRID_OK;
   if (bx > 0x7fffffffu) return GRID_ERR_INVALID_PARAMETERS;
-  to_point_major_kernel<<<dim3((unsigned)bx, (d + 31) / 32), dim3(32, 8), 0, s>>>(in, out, npolys,
-                                                                                   d);
+  const unsigned bz = rows < 65535 ? (unsigned)rows : 65535u;
+  to_point_major_kernel<<<dim3((unsigned)bx, (d + 31) / 32, bz), dim3(32, 8), 0, s>>>(
+      in, out, rows, cols, ld, d);
   return cuda_status(cudaGetLastError());
 }
 

@@ -41,8 +41,7 @@ enum NttMode : int {
   MODE_INV = 1,     // twisted evaluations -> coefficients
   MODE_MULINV = 2,  // out = INTT(NTT(a) (.) b_evals)
   MODE_POLYMUL = 3, // out = INTT(NTT(a) (.) NTT(b))  (negacyclic product)
-  MODE_FWD_PM = 4,  // MODE_FWD stored point-major: out[e * ps + poly], ps = npolys rounded
-                    // up to a multiple of 4, pad polys zero (d = 64 tensor cores)
+  MODE_FWD_PM = 4,  // MODE_FWD stored point-major (launch_ntt_tc_pm, d = 64 tensor cores)
 };
 
 struct DeviceScratch {
@@ -101,10 +100,11 @@ struct grid_gpu_matrix {
   size_t rows = 0, cols = 0;
   size_t ld = 0;                // row stride in polys (cols of the owning matrix)
   uint32_t* d_evals = nullptr;  // rows x ld polys in the twisted evaluation domain
-  // The same evaluations point-major, [d][rows][ld], for the tensor-core
+  // The same evaluations point-major, [d][rows][ld_pm], for the tensor-core
   // contraction over TMA-loaded operands (null where that path does not apply; in
   // d_evals' allocation).
   uint32_t* d_evals_pm = nullptr;
+  size_t ld_pm = 0;             // pm_stride of the owning matrix's cols
   bool owned = true;            // false for views sharing another matrix's evaluations
   // On a ring plan without an NTT for q: the matrix's residues mod each
   // auxiliary prime, prepared on that prime's plan (d_evals stays null).
@@ -129,6 +129,9 @@ int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, const uin
                   uint32_t* out, size_t npolys, cudaStream_t s);
 void build_tc_tables(uint32_t q, uint32_t d, uint64_t psi, uint64_t ninv,
                      std::vector<unsigned char>& out);
+// a [rows][n] polys -> out [64 points][rows][pm_stride(n)] (pad words undefined).
+int launch_ntt_tc_pm(const grid_gpu_plan* p, const uint32_t* a, size_t rows, size_t n,
+                     uint32_t* out, cudaStream_t s);
 // MODE_FWD_PM over a tile list: tile t transforms the 128 polys from source
 // row ptiles[t].x of a (npolys polys) into columns ptiles[t].y .. + 127 of
 // out [64][ps_out], polys from ptiles[t].z of the tile on as zeros. Columns
@@ -162,21 +165,34 @@ int launch_emm_tc(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, 
 // out[i] = sum over splits s of work[s * stride + i] (mod q)
 int launch_sum_splits(const grid_gpu_plan* p, const uint32_t* work, uint32_t* out, size_t stride,
                       int splits, cudaStream_t s);
-// emm_pm.cu: the same products over point-major operands, X [d][M][K] and
-// Y [d][N][ldy] (tensor cores, TMA; X rows <= 128, Y rows <= 64, K and ldy
-// multiples of 4, 16-byte aligned bases). Split partials go to `work`.
+// emm_pm.cu: the same products over point-major operands, X [d][M][ldx] and
+// Y [d][N][ldy] (tensor cores, TMA; d = 64, X rows <= 128, Y rows <= 64, any K, row
+// strides multiples of 4, 16-byte aligned bases), through to coefficients: K-range
+// partials go to `work`, are summed and inverse transformed into out [output][d].
+// symmetrize: out = the packed upper triangle of (C_ij + C_ji) / 2 for the dense
+// M x M product C.
 struct EmmPmGeometry {
   int np;  // Y rows padded to 16, 32, 48 or 64
   int splits, k_per_split;
 };
-bool emm_pm_geometry(const grid_gpu_plan* p, int M, int N, int K, int ldy, int mode,
-                     EmmPmGeometry* g);
+bool emm_pm_geometry(const grid_gpu_plan* p, int M, int N, int K, int mode, EmmPmGeometry* g);
 size_t emm_pm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode);
 int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N,
-                  int K, int ldy, int mode, uint32_t* out_evals, uint32_t* work, cudaStream_t s);
-// in [npolys][d] -> out [d][npolys] (point-major copy of evaluations)
-int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t npolys, int d,
-                          cudaStream_t s);
+                  int K, int ldx, int ldy, int mode, bool symmetrize, uint32_t* out,
+                  uint32_t* work, cudaStream_t s);
+// Row stride of point-major evaluations of rows of n polys: whole 16-byte units.
+inline size_t pm_stride(size_t n) { return (n + 3) / 4 * 4; }
+// in [rows][cols][d] -> out [d][rows][ld], words past cols zero
+int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t rows, size_t cols, size_t ld,
+                          int d, cudaStream_t s);
+// ntt.cu (d = 64): part [split][e][output] summed over the splits (mod q), inverse
+// transformed, out [output][64]. sym_r > 0: part holds the dense sym_r x sym_r product C
+// and the outputs are the packed upper triangle of (C_ij + C_ji) / 2.
+int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
+                       int sym_r, uint32_t* out, cudaStream_t s);
+// The least workspace grid_gpu_gram_dev runs in (grid_gpu_gram_workspace: what it runs
+// best in).
+int gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes);
 // garbage.cu: (C_ij + C_ji) * 2^-1 on the upper triangle; z_hat = sum_i c_hat_i (.) s_hat_i.
 int launch_symmetrize_half(const grid_gpu_plan* p, const uint32_t* C, int r, uint32_t* H,
                            cudaStream_t s);

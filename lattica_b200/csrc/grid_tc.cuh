@@ -74,6 +74,13 @@ __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Descriptor `off` bytes after one whose address field cannot carry out of its word.
+__device__ __forceinline__ uint64_t desc_plus(uint64_t desc, uint32_t off) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"((uint32_t)desc + (off >> 4)), "r"((uint32_t)(desc >> 32)));
+  return r;
+}
+
 // One thread: D[tmem] (+)= A * B^T, M = 128 rows, N columns, K = 32 bytes.
 __device__ __forceinline__ void mma_u8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                        uint32_t idesc, uint32_t accumulate) {
@@ -117,6 +124,34 @@ __device__ __forceinline__ void tmem_ld_wait32(uint32_t (&r)[4][8]) {
                  "+r"(r[1][0]), "+r"(r[1][1]), "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]), "+r"(r[1][7]),
                  "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]), "+r"(r[2][4]), "+r"(r[2][5]), "+r"(r[2][6]), "+r"(r[2][7]),
                  "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]), "+r"(r[3][3]), "+r"(r[3][4]), "+r"(r[3][5]), "+r"(r[3][6]), "+r"(r[3][7])
+               :
+               : "memory");
+}
+
+// Whole warp: zeros into 16 consecutive columns of the warp's 32 lanes.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1};" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
+}
+
+// This thread's tensor-memory stores are done (then fence_before_sync and a barrier
+// order them before another thread's MMAs).
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld_wait7(uint32_t (&r)[7][8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[0][4]), "+r"(r[0][5]), "+r"(r[0][6]), "+r"(r[0][7]),
+                 "+r"(r[1][0]), "+r"(r[1][1]), "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[1][4]), "+r"(r[1][5]), "+r"(r[1][6]), "+r"(r[1][7]),
+                 "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]), "+r"(r[2][4]), "+r"(r[2][5]), "+r"(r[2][6]), "+r"(r[2][7]),
+                 "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]), "+r"(r[3][3]), "+r"(r[3][4]), "+r"(r[3][5]), "+r"(r[3][6]), "+r"(r[3][7]),
+                 "+r"(r[4][0]), "+r"(r[4][1]), "+r"(r[4][2]), "+r"(r[4][3]), "+r"(r[4][4]), "+r"(r[4][5]), "+r"(r[4][6]), "+r"(r[4][7]),
+                 "+r"(r[5][0]), "+r"(r[5][1]), "+r"(r[5][2]), "+r"(r[5][3]), "+r"(r[5][4]), "+r"(r[5][5]), "+r"(r[5][6]), "+r"(r[5][7]),
+                 "+r"(r[6][0]), "+r"(r[6][1]), "+r"(r[6][2]), "+r"(r[6][3]), "+r"(r[6][4]), "+r"(r[6][5]), "+r"(r[6][6]), "+r"(r[6][7])
                :
                : "memory");
 }

@@ -168,7 +168,7 @@ __global__ void __maxnreg__(64)
       const TileDev tl = tiles[w.tile];
       const MatDev mt = mats[tl.matrix];
       const uint32_t* se = s_pm + (unsigned long long)w.eg * ps;
-      const uint32_t* ye = mt.evals_pm + (unsigned long long)w.eg * mt.rows * mt.ld;
+      const uint32_t* ye = mt.evals_pm + (unsigned long long)w.eg * mt.rows * mt.ld_pm;
       const uint32_t row0 = 32u * lw;
       const uint32_t cw = tl.count > row0 ? min(tl.count - row0, 32u) : 0u;  // this warp's rows
       // this lane's row: point-major column (a multiple of 128) and length
@@ -213,9 +213,9 @@ __global__ void __maxnreg__(64)
         for (uint32_t u = lw * 32 + lane; u < mt.rows * 8; u += kGpLoaders) {
           const uint32_t yr = u >> 3, yq = u & 7;
           const uint32_t kw = kc + 4 * yq;
-          const bool valid = kw < mt.ld;
+          const bool valid = kw < mt.ld_pm;
           cp_async16s(sa + S::XSLOT + sw128(yr, 0, yq, 0),
-                      valid ? ye + (unsigned long long)yr * mt.ld + kw : ye, valid ? 16u : 0u);
+                      valid ? ye + (unsigned long long)yr * mt.ld_pm + kw : ye, valid ? 16u : 0u);
         }
         cp_async_arrive_noinc(&full[sl]);
       }

@@ -157,13 +157,6 @@ __device__ __forceinline__ uint32_t residue(long long v, uint32_t q) {
   return (uint32_t)(r < 0 ? r + q : r);
 }
 
-// Descriptor `off` bytes after one whose address field cannot carry out of its word.
-__device__ __forceinline__ uint64_t desc_plus(uint64_t desc, uint32_t off) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"((uint32_t)desc + (off >> 4)), "r"((uint32_t)(desc >> 32)));
-  return r;
-}
-
 // The MMA warp's loop (one lane): warp w's units are first(w), first(w) + stride, ...
 // below nunits, first() ascending; issue(w, accumulate) issues one unit's MMAs. A group
 // of kGroup warps is handed over through one barrier and released by one commit, and the
@@ -284,8 +277,8 @@ __global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
           [&](int w, uint32_t acc) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-              tc::mma_u8(tbase + 16 * h, desc_plus(da, w * kUnitA + h * 1024),
-                         desc_plus(db, w * kPjB), idesc, acc);
+              tc::mma_u8(tbase + 16 * h, tc::desc_plus(da, w * kUnitA + h * 1024),
+                         tc::desc_plus(db, w * kPjB), idesc, acc);
           },
           err);
     }
@@ -576,8 +569,8 @@ __global__ void __launch_bounds__(kEvThreads, 1) jl_eval_tc_kernel(
           [&](int w, uint32_t acc) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-              tc::mma_u8(tbase + 256 * h, desc_plus(da, w * kUnitA + h * 1024),
-                         desc_plus(db, w * kEvB), idesc, acc);
+              tc::mma_u8(tbase + 256 * h, tc::desc_plus(da, w * kUnitA + h * 1024),
+                         tc::desc_plus(db, w * kEvB), idesc, acc);
           },
           err);
     }

@@ -67,7 +67,7 @@ int grid_gpu_gram_noalloc_dev(const grid_gpu_plan* plan, const uint32_t* S, size
   const size_t max_polys = kNoAllocScratchBytes / (4 * (size_t)plan->d);
   if (r > max_polys || n > max_polys / r) return GRID_ERR_SCRATCH_LIMIT;
   size_t need = 0;
-  int st = grid_gpu_gram_workspace(plan, r, n, &need);
+  int st = grid::gram_min_workspace(plan, r, n, &need);
   if (st) return st;
   if (need > kNoAllocScratchBytes) return GRID_ERR_SCRATCH_LIMIT;
   // The buffer's address is per device: the launches go to the current device,

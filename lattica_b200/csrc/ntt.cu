@@ -610,6 +610,83 @@ __global__ void __launch_bounds__(D * kSmallSlots) commit_small_kernel(
 }
 
 // ---------------------------------------------------------------------------
+// The end of a point-major contraction (emm_pm.cu): a CTA sums the K-range partials of
+// 32 outputs point by point (reads along the outputs, 128 bytes per point and
+// split), and eight threads per output run its inverse transform from shared memory.
+// One launch instead of a transposing sum and a transform of its own, whose 64 KB
+// matrix copy a few hundred polynomials do not pay for (the Gram of r = 30, n = 1021 went
+// from 41 to 27 us a call with this and the products' byte planes, u1 and u2 of the outer
+// commitment at r = 64 from 204 to 130).
+// kSym: output (i, j) is (C_ij + C_ji) / 2 of a dense r x r product (garbage h).
+// ---------------------------------------------------------------------------
+constexpr int kSiPolys = 32;
+constexpr int kSiThreads = kSiPolys * kSmallT;
+
+template <bool kSym>
+__global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
+    const uint32_t* __restrict__ part, int outputs, int splits, int r, uint32_t two_inv,
+    uint32_t* __restrict__ out, const uint2* __restrict__ gtw, FieldParams f) {
+  constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2;
+  constexpr int PS = D + 1;  // the 32 outputs of a point fall in distinct banks
+  __shared__ uint2 tws[TWN];
+  __shared__ uint32_t sh[kSiPolys * PS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < TWN; i += kSiThreads) tws[i] = gtw[i];
+  const int o = blockIdx.x * kSiPolys + lane;
+  const bool valid = o < outputs;
+  int at = o, mirror = 0;
+  const int width = kSym ? r * r : outputs;  // words per (split, point) of part
+  if (kSym) {  // packed upper triangle: row i starts at i r - i (i - 1) / 2
+    int i = (int)((2 * r + 1 - sqrtf((float)((2 * r + 1) * (2 * r + 1)) - 8.0f * (float)o)) * 0.5f);
+    i = max(0, min(i, r - 1));
+    while (i > 0 && i * r - i * (i - 1) / 2 > o) --i;
+    while (i + 1 < r && (i + 1) * r - (i + 1) * i / 2 <= o) ++i;
+    const int j = i + o - (i * r - i * (i - 1) / 2);
+    at = i * r + j;
+    mirror = j * r + i;
+  }
+  const size_t stride = (size_t)D * width;
+  // this warp's points warp, warp + 8, ...: the loads of one split are independent
+  constexpr int PTS = D / (kSiThreads / 32);
+  uint32_t v[PTS] = {};
+  if (valid) {
+    const uint32_t* src = part + (size_t)warp * width;
+#pragma unroll 2
+    for (int s = 0; s < splits; ++s, src += stride) {
+#pragma unroll
+      for (int k = 0; k < PTS; ++k) {
+        const uint32_t* row = src + (size_t)(k * (kSiThreads / 32)) * width;
+        uint32_t w = row[at];
+        if (kSym) w = add_mod(w, row[mirror], f.q);
+        v[k] = add_mod(v[k], w, f.q);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < PTS; ++k)
+    sh[lane * PS + warp + k * (kSiThreads / 32)] =
+        kSym ? mont_mul(v[k], two_inv, f.q, f.qinv) : v[k];
+  __syncthreads();
+  const int pl = tid / T, t = tid % T;
+  const int bt_t = brv(4 * t, LOGD);
+  const Consts c = consts_of(f);
+  uint32_t x[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = 4 * T * (e >> 2) + (e & 3);
+    x[e] = sh[pl * PS + (brv(i, LOGD) | bt_t)];
+  }
+  invT_stages<D, T, 1>(x, tws, t, c);
+  const int po = blockIdx.x * kSiPolys + pl;
+  if (po < outputs) {
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)po * D);
+#pragma unroll
+    for (int m = 0; m < E / 4; ++m)
+      dst[T * m + t] = make_uint4(x[4 * m + 0], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
 template <int D>
@@ -701,6 +778,24 @@ int launch_ntt(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32
     case MODE_MULINV: return dispatch<MODE_MULINV>(p, a, b, out, npolys, s);
     default: return GRID_ERR_INVALID_PARAMETERS;
   }
+}
+
+int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
+                       int sym_r, uint32_t* out, cudaStream_t s) {
+  if (p->d != 64) return GRID_ERR_UNSUPPORTED_DEGREE;
+  if (sym_r) outputs = sym_r * (sym_r + 1) / 2;
+  if (outputs <= 0) return GRID_OK;
+  // (q + 1) / 2 in Montgomery form
+  const uint32_t two_inv =
+      (uint32_t)(((unsigned __int128)((p->f.q + 1ull) / 2) << 32) % p->f.q);
+  const unsigned grid = (unsigned)((outputs + kSiPolys - 1) / kSiPolys);
+  if (sym_r)
+    sum_inverse_kernel<true><<<grid, kSiThreads, 0, s>>>(part, outputs, splits, sym_r, two_inv, out,
+                                                         p->d_tw, p->f);
+  else
+    sum_inverse_kernel<false><<<grid, kSiThreads, 0, s>>>(part, outputs, splits, 0, two_inv, out,
+                                                          p->d_tw, p->f);
+  return cuda_status(cudaGetLastError());
 }
 
 bool commit_small_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {

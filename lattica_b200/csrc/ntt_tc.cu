@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                   const __grid_constant__ CUtensorMap tmap_out, const uint32_t* __restrict__ a,
                   const uint32_t* __restrict__ b, unsigned long long npolys,
                   const uint4* __restrict__ wtab, const TcConsts k, int* __restrict__ err,
-                  const uint4* __restrict__ ptiles, unsigned long long nptiles) {
+                  const uint4* __restrict__ ptiles, unsigned long long nptiles,
+                  uint32_t row_polys) {
   constexpr bool kTwo = MODE == MODE_MULINV;
   constexpr bool kPm = MODE == MODE_FWD_PM;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
@@ -120,8 +121,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   // Point-major mode with a tile list (ptiles): tile t reads 128 polys from
   // row x, stores them at column y, and rows from z on (past an instance) as 0.
+  // With row_polys the tiles stay within rows of that many polys: a tile's result box
+  // ends at its row's end (the 3D output map clips it), tile t / row_tiles being the row.
   const bool listed = kPm && ptiles != nullptr;
-  const unsigned long long ntiles = listed ? nptiles : (npolys + ROWS - 1) / ROWS;
+  const bool by_row = kPm && row_polys != 0;
+  const uint32_t row_tiles = by_row ? (row_polys + ROWS - 1) / ROWS : 1u;
+  const unsigned long long ntiles =
+      listed || by_row ? nptiles : (npolys + ROWS - 1) / ROWS;
   const uint32_t n = blockIdx.x < ntiles
                          ? (uint32_t)((ntiles - 1 - blockIdx.x) / gridDim.x + 1)
                          : 0u;  // tiles of this CTA
@@ -130,6 +136,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   };
   // first source row / destination row (point-major: column) of tile j
   auto tile_row0 = [&](uint32_t j) -> unsigned long long {
+    if (by_row) {
+      const uint32_t t = (uint32_t)tile_index(j);
+      return (unsigned long long)(t / row_tiles) * row_polys + (t % row_tiles) * ROWS;
+    }
     return listed ? (unsigned long long)ptiles[tile_index(j)].x : tile_index(j) * ROWS;
   };
   auto tile_out0 = [&](uint32_t j) -> unsigned long long {
@@ -171,7 +181,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint32_t js = t - lag;
         ok = warp_wait_fast(&bars[STAGED0 + buf], staged_seen[buf]++ & 1, err);
         if (ok && lane == 0) {
-          if constexpr (kPm) {  // [64 points][128 polys] -> columns row0.. of the [d][npolys] output
+          if (by_row) {
+            const uint32_t tr = (uint32_t)tile_index(js);
+            tma_store_3d(&tmap_out, (int)((tr % row_tiles) * ROWS), (int)(tr / row_tiles), 0, dst);
+          } else if constexpr (kPm) {  // [64 points][128 polys] -> columns row0.. of the [d][npolys] output
             tma_store_2d(&tmap_out, (int)tile_out0(js), 0, dst);
           } else {
             tma_store_2d(&tmap_out, 0, (int)tile_row0(js), dst);
@@ -331,12 +344,15 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-// ptiles / nptiles / ps_out: the point-major mode's tile list and row length
-// (defaults: consecutive tiles, npolys rounded up to a multiple of 4).
+// The point-major mode's layout: ptiles / nptiles / ps_out, a tile list over
+// [64][ps_out]; row_polys, rows of that many polys, npolys / row_polys of them, at
+// [64][rows][pm_stride(row_polys)]; neither, consecutive tiles over [64][npolys]
+// (npolys a multiple of 4).
 template <int MODE>
 int run_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_t* out,
            size_t npolys, cudaStream_t s, const uint4* ptiles = nullptr,
-           unsigned long long nptiles = 0, unsigned long long ps_out = 0) {
+           unsigned long long nptiles = 0, unsigned long long ps_out = 0,
+           uint32_t row_polys = 0) {
   EncodeTiled enc = encoder();
   if (!enc) return GRID_ERR_CUDA;
   // Rows of 64 words, boxes of 32 words x 128 rows with 128-byte swizzle.
@@ -351,11 +367,21 @@ int run_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return GRID_ERR_CUDA;
-  if (MODE == MODE_FWD_PM) {
-    // output [64 points][ps], ps = npolys rounded up to a multiple of 4 (rows
-    // of whole 16-byte units); one box of 128 polys x 64 points per tile, the
-    // pad polys transformed from the zero fill past the input
-    const cuuint64_t ps = ps_out ? ps_out : ((cuuint64_t)npolys + 3) / 4 * 4;
+  if (MODE == MODE_FWD_PM && row_polys) {
+    const cuuint64_t rows = npolys / row_polys, ld = pm_stride(row_polys);
+    const cuuint64_t rdims[3] = {row_polys, rows, 64};
+    const cuuint64_t rstrides[2] = {ld * 4, rows * ld * 4};
+    const cuuint32_t rbox[3] = {ROWS, 1, 64};
+    const cuuint32_t rstr[3] = {1, 1, 1};
+    if (enc(&map_out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, (void*)out, rdims, rstrides, rbox, rstr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return GRID_ERR_CUDA;
+    nptiles = rows * ((row_polys + ROWS - 1) / ROWS);
+  } else if (MODE == MODE_FWD_PM) {
+    // output [64 points][ps], ps a multiple of 4 (rows of whole 16-byte units); one
+    // box of 128 polys x 64 points per tile
+    const cuuint64_t ps = ps_out ? ps_out : (cuuint64_t)npolys;
     const cuuint64_t pdims[2] = {ps, 64};
     const cuuint64_t pstrides[1] = {ps * 4};
     const cuuint32_t pbox[2] = {ROWS, 64};
@@ -369,7 +395,7 @@ int run_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_
   const int st =
       prepare_kernel(ntt_tc_kernel<MODE>, SMEM_BYTES, THREADS, p->device, bps_cache, &bps);
   if (st) return st;
-  const unsigned long long tiles = ptiles ? nptiles : (npolys + ROWS - 1) / ROWS;
+  const unsigned long long tiles = nptiles ? nptiles : (npolys + ROWS - 1) / ROWS;
   const unsigned long long grid =
       tiles < (unsigned long long)p->num_sms ? tiles : (unsigned long long)p->num_sms;
   TcConsts k;
@@ -377,7 +403,7 @@ int run_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_
   k.qinv = p->f.qinv;
   ntt_tc_kernel<MODE><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(
       map_a, map_out, a, b, (unsigned long long)npolys, reinterpret_cast<const uint4*>(p->d_tcw), k,
-      p->d_err, ptiles, nptiles);
+      p->d_err, ptiles, nptiles, row_polys);
   return cuda_status(cudaGetLastError());
 }
 
@@ -414,6 +440,19 @@ int launch_ntt_tc_pm_tiles(const grid_gpu_plan* p, const uint32_t* a, size_t npo
   return run_tc<MODE_FWD_PM>(p, a, nullptr, out, npolys, s, ptiles, nptiles, ps_out);
 }
 
+int launch_ntt_tc_pm(const grid_gpu_plan* p, const uint32_t* a, size_t rows, size_t n,
+                     uint32_t* out, cudaStream_t s) {
+  const size_t npolys = rows * n;
+  if (npolys == 0) return GRID_OK;
+  // tiles of other CTAs still read the input while a tile's columns land
+  if (a == out) return GRID_ERR_INVALID_PARAMETERS;
+  if (npolys > (size_t)INT32_MAX - ROWS) return GRID_ERR_INVALID_PARAMETERS;  // TMA coordinates
+  // rows of whole 16-byte units follow one another without a gap: one long row, whose
+  // tiles need not end with each of them
+  return run_tc<MODE_FWD_PM>(p, a, nullptr, out, npolys, s, nullptr, 0, 0,
+                             n % 4 ? (uint32_t)n : 0u);
+}
+
 int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32_t* b,
                   uint32_t* out, size_t npolys, cudaStream_t s) {
   if (npolys == 0) return GRID_OK;
@@ -422,10 +461,6 @@ int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, const uin
     case MODE_FWD: return run_tc<MODE_FWD>(p, a, nullptr, out, npolys, s);
     case MODE_INV: return run_tc<MODE_INV>(p, a, nullptr, out, npolys, s);
     case MODE_MULINV: return run_tc<MODE_MULINV>(p, a, b, out, npolys, s);
-    case MODE_FWD_PM:
-      // tiles of other CTAs still read the input while a tile's columns land
-      if (a == out) return GRID_ERR_INVALID_PARAMETERS;
-      return run_tc<MODE_FWD_PM>(p, a, nullptr, out, npolys, s);
     default: return GRID_ERR_INVALID_PARAMETERS;
   }
 }

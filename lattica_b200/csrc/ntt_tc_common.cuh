@@ -133,6 +133,18 @@ __device__ __forceinline__ void reduce16(uint32_t taddr, const TcConsts& k, uint
   reduce16(taddr, k, out, [] {});
 }
 
+// (sum_s 2^(8s) d_s) * 2^-32 mod q for the seven byte classes of a sum of word
+// products (each below 2^32, the sum below 2^80), canonical.
+__device__ __forceinline__ uint32_t reduce_classes(uint32_t d0, uint32_t d1, uint32_t d2,
+                                                   uint32_t d3, uint32_t d4, uint32_t d5,
+                                                   uint32_t d6, const FieldParams& f) {
+  const uint64_t lo = mad_wide(d3, 16777216u, mad_wide(d2, 65536u, mad_wide(d1, 256u, d0)));
+  const uint64_t hi = mad_wide(d6, 65536u, mad_wide(d5, 256u, d4));
+  const uint64_t mid = (lo >> 32) + (uint32_t)hi;
+  return acc96_reduce(Acc96{(uint32_t)lo, (uint32_t)mid, (uint32_t)(hi >> 32) + (uint32_t)(mid >> 32)},
+                      f);
+}
+
 // One transform of a 128-row tile (A at `a`, B at `w`) into 256 columns.
 __device__ __forceinline__ void issue_transform(uint32_t dcol, uint32_t a, uint32_t w) {
 #pragma unroll
@@ -166,6 +178,14 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
                    map),
                "r"(x), "r"(y), "r"(src)
                : "memory");
+}
+
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z,
+                                             uint32_t src) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map),
+      "r"(x), "r"(y), "r"(z), "r"(src)
+      : "memory");
 }
 
 // Contiguous global bytes -> L2 (no shared memory, no completion tracking).
