@@ -132,7 +132,7 @@ int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint3
     rc = launch_ntt_tc_pm(p, s, batch, A->cols, s_hat, st);
     if (rc) return rc;
     return launch_emm_pm(p, s_hat, A->d_evals_pm, (int)batch, (int)A->rows, (int)A->cols, (int)ldx,
-                         (int)A->ld_pm, EMM_DENSE, false, t, work, st);
+                         (int)A->ld_pm, EMM_DENSE, false, t, LimbSpec(), work, st);
   }
   rc = launch_ntt(p, MODE_FWD, s, nullptr, s_hat, batch * A->cols, st);
   if (!rc)
@@ -501,7 +501,7 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
       rc = launch_ntt_tc_pm(q, S, r, n, s_hat, st);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
-                           false, out, work, st);
+                           false, out, LimbSpec(), work, st);
       continue;
     }
     rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
@@ -572,7 +572,7 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     if (!rc) rc = launch_ntt_tc_pm(q, Phi, r, n, phi_hat, st);
     if (!rc)
       rc = launch_emm_pm(q, phi_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_DENSE,
-                         sym, out, work, st);
+                         sym, out, LimbSpec(), work, st);
     return rc;
   };
   // poly-major: out[i][j] = <phi_i, s_j> in plan q's evaluation domain
@@ -941,19 +941,22 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
       gj[j] = cv.take<uint32_t>(gw);
     }
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+  auto round_pm = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq) {
+    return Aq->d_evals_pm && pm_fits(q, r, kappa, n, EMM_DENSE) && pm_fits(q, r, r, n, EMM_UPPER);
+  };
   // inner commitments and the Gram over the witness's evaluations (one
-  // transform shared by both) on plan q into tt / gg
+  // transform shared by both) on plan q into tt / gg, or their limbs (tt unwritten then)
   auto contract = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq, uint32_t* tt,
-                      uint32_t* gg, cudaStream_t cs) {
-    if (Aq->d_evals_pm && pm_fits(q, r, kappa, n, EMM_DENSE) && pm_fits(q, r, r, n, EMM_UPPER)) {
+                      uint32_t* gg, const LimbSpec& tl, const LimbSpec& gl, cudaStream_t cs) {
+    if (round_pm(q, Aq)) {
       // point-major evaluations: both products load their operands with TMA
       int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, cs);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, Aq->d_evals_pm, (int)r, (int)kappa, (int)n, (int)ldx,
-                           (int)Aq->ld_pm, EMM_DENSE, false, tt, work, cs);
+                           (int)Aq->ld_pm, EMM_DENSE, false, tl.out ? nullptr : tt, tl, work, cs);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
-                           false, gg, work, cs);
+                           false, gg, gl, work, cs);
       return rc;
     }
     int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, cs);
@@ -985,18 +988,26 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
     if (jl)
       rc_jl = launch_jl_project(p->f, jl_seed, jl_rows, S, r, n * d, d, p_out, jl_flat, jl_ws,
                                 jl_scratch_bytes(jl_rows, 0, 0), p->num_sms, p->d_err, lo);
-    // 1. inner commitments t_i = A s_i and 2. garbage g_ij = <s_i, s_j>, i <= j
+    // 1. inner commitments t_i = A s_i and 2. garbage g_ij = <s_i, s_j>, i <= j, with
+    // the balanced limbs of both (inner_commit_decomposed, decompose_polys)
+    auto spec = [](uint32_t* out, uint64_t base, size_t limbs) {
+      return out && aligned16(out) && limbs_ok(base, limbs) ? limb_spec(out, base, limbs)
+                                                            : LimbSpec();
+    };
+    LimbSpec tl = spec(t_limbs, b1, t1), gl = spec(g_limbs, b2, t2);
     if (!is_crt(p)) {
-      rc_chain = contract(p, A, t, g, hi);
+      if (!round_pm(p, A)) tl = gl = LimbSpec();  // the poly-major products leave them to a pass
+      rc_chain = contract(p, A, t, g, tl, gl, hi);
     } else {
       for (int j = 0; j < 3 && !rc_chain; ++j)
-        rc_chain = contract(p->crt[j], A->crt[j], tj[j], gj[j], hi);
-      if (!rc_chain) rc_chain = crt_combine(p, tj[0], tj[1], tj[2], tw, t, hi);
-      if (!rc_chain) rc_chain = crt_combine(p, gj[0], gj[1], gj[2], gw, g, hi);
+        rc_chain = contract(p->crt[j], A->crt[j], tj[j], gj[j], LimbSpec(), LimbSpec(), hi);
+      if (!rc_chain)
+        rc_chain = crt_combine(p, tj[0], tj[1], tj[2], tw, tl.out ? nullptr : t, hi, tl);
+      if (!rc_chain) rc_chain = crt_combine(p, gj[0], gj[1], gj[2], gw, g, hi, gl);
     }
-    // balanced limbs of both (inner_commit_decomposed, decompose_polys)
-    if (!rc_chain) rc_chain = launch_decompose_balanced(p, t, r * kappa, b1, t1, t_limbs, hi);
-    if (!rc_chain && g_limbs)
+    if (!rc_chain && !tl.out)
+      rc_chain = launch_decompose_balanced(p, t, r * kappa, b1, t1, t_limbs, hi);
+    if (!rc_chain && g_limbs && !gl.out)
       rc_chain = launch_decompose_balanced(p, g, r * (r + 1) / 2, b2, t2, g_limbs, hi);
     // join: the caller's stream waits for both forks (also after a failed launch)
     int rj = cuda_status(cudaEventRecord(ev[1], hi));

@@ -13,38 +13,32 @@
 // digit = value % base, value /= base, k = #digits(q - 1) times.
 #include <cuda_runtime.h>
 
+#include "balanced.cuh"
 #include "grid_field.cuh"
 #include "grid_internal.h"
 
 namespace grid {
 namespace {
 
-__device__ __forceinline__ long long centered_mod(long long v, long long base) {
-  const long long half = base / 2;
-  const long long r = v % base;  // truncating, like Rust's %
-  if (r > half) return r - base;
-  if (r < -half) return r + base;
-  return r;
-}
-
-__global__ void balanced_kernel(const uint32_t* __restrict__ in, size_t npolys, int d,
-                                long long base, int num_limbs, uint32_t* __restrict__ out,
-                                FieldParams f) {
-  const size_t total = npolys * (size_t)d;
+// kVec: four coefficients per thread (16-byte aligned buffers, d a multiple of 4).
+template <bool kVec>
+__global__ void balanced_kernel(const uint32_t* __restrict__ in, size_t npolys, uint32_t d,
+                                LimbSpec l, FieldParams f) {
+  constexpr int W = kVec ? 4 : 1;
+  const size_t total = npolys * (size_t)d / W;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const long long q = f.q;
-  const long long half_q = q / 2;
+  const uint32_t per_poly = d / W;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-    const size_t poly = idx / d;
-    const int i = (int)(idx % d);
-    long long carry = (long long)from_mont(in[idx], f);
-    if (carry > half_q) carry -= q;
-    uint32_t* dst = out + poly * (size_t)num_limbs * d + i;
-    for (int k = 0; k < num_limbs; ++k) {
-      const long long limb = centered_mod(carry, base);
-      const long long u = limb >= 0 ? limb : q + limb;  // q - |limb|
-      dst[(size_t)k * d] = to_mont((uint32_t)(u % q), f);
-      carry = (carry - limb) / base;
+    const size_t poly = idx / per_poly;
+    const uint32_t i = (uint32_t)(idx % per_poly) * W;
+    uint32_t* dst = l.out + poly * (size_t)l.limbs * d + i;
+    if constexpr (kVec) {
+      store_limbs4(reinterpret_cast<const uint4*>(in)[idx], dst, (int)d, l, f);
+    } else {
+      uint32_t a = from_mont(in[idx], f);
+      const bool neg = a > f.q / 2;
+      if (neg) a = f.q - a;
+      for (int k = 0; k < l.limbs; ++k, dst += d) *dst = next_limb(a, neg, l, f);
     }
   }
 }
@@ -76,13 +70,23 @@ unsigned blocks_for(size_t n, int num_sms) {
 
 }  // namespace
 
+bool limbs_ok(uint64_t base, size_t num_limbs) {
+  return base >= 2 && base <= (1ull << 32) && num_limbs > 0 && num_limbs <= 64;
+}
+
 int launch_decompose_balanced(const grid_gpu_plan* p, const uint32_t* polys, size_t npolys,
                               uint64_t base, size_t num_limbs, uint32_t* out, cudaStream_t s) {
-  if (base < 2 || base > (1ull << 32) || num_limbs == 0 || num_limbs > 64)
-    return GRID_ERR_INVALID_PARAMETERS;
+  if (!limbs_ok(base, num_limbs)) return GRID_ERR_INVALID_PARAMETERS;
   if (npolys == 0) return GRID_OK;
-  balanced_kernel<<<blocks_for(npolys * p->d, p->num_sms), 256, 0, s>>>(
-      polys, npolys, (int)p->d, (long long)base, (int)num_limbs, out, p->f);
+  const LimbSpec l = limb_spec(out, base, num_limbs);
+  const size_t words = npolys * p->d;
+  if (((reinterpret_cast<uintptr_t>(polys) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 &&
+      p->d % 4 == 0)
+    balanced_kernel<true><<<blocks_for(words / 4, p->num_sms), 256, 0, s>>>(polys, npolys, p->d, l,
+                                                                            p->f);
+  else
+    balanced_kernel<false><<<blocks_for(words, p->num_sms), 256, 0, s>>>(polys, npolys, p->d, l,
+                                                                         p->f);
   return cuda_status(cudaGetLastError());
 }
 

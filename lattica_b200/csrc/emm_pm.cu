@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(kPmThreads)
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  grid_dep_wait();
+  grid_dep_launch();
 
   if (warp == kPmLoadWarp) {
     // ------------------------------------------------------------ TMA loads
@@ -313,9 +315,8 @@ int launch_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int 
   else if (!make_pm_map(&my, Y, K, N, ldy, (int)p->d))
     return GRID_ERR_CUDA;
   const uint32_t box_bytes = (uint32_t)(KCH * 4) * (uint32_t)(UPPER ? M : M + N);
-  emm_pm_kernel<NP, MX, UPPER><<<dim3(p->d, g.splits), kPmThreads, S::SMEM, s>>>(
-      mx, my, part, M, N, K, g.k_per_split, box_bytes, p->f, p->d_err);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(emm_pm_kernel<NP, MX, UPPER>, dim3(p->d, g.splits), kPmThreads, S::SMEM, s,
+                        mx, my, part, M, N, K, g.k_per_split, box_bytes, p->f, p->d_err);
 }
 
 template <int NP>
@@ -372,7 +373,7 @@ size_t emm_pm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int m
 
 int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N,
                   int K, int ldx, int ldy, int mode, bool symmetrize, uint32_t* out,
-                  uint32_t* work, cudaStream_t s) {
+                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s) {
   EmmPmGeometry g;
   if (!emm_pm_geometry(p, M, N, K, mode, &g) || ldx < K || ldx % 4) return GRID_ERR_INVALID_PARAMETERS;
   if (mode != EMM_UPPER && (ldy < K || ldy % 4)) return GRID_ERR_INVALID_PARAMETERS;
@@ -390,7 +391,7 @@ int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, 
   if (rc) return rc;
   // point-major partials [split][e][output] -> coefficients [output][64]
   const int outputs = mode == EMM_UPPER ? M * (M + 1) / 2 : M * N;
-  return launch_sum_inverse(p, work, outputs, g.splits, symmetrize ? M : 0, out, s);
+  return launch_sum_inverse(p, work, outputs, g.splits, symmetrize ? M : 0, out, limbs, s);
 }
 
 }  // namespace grid

@@ -38,6 +38,19 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                : "memory");
 }
 
+// Programmatic dependent launch. A kernel launched with it (launch_chained) may start
+// while its predecessor in the stream still runs: everything before grid_dep_wait()
+// must touch only constants and its own shared and tensor memory. grid_dep_launch()
+// lets the successor start; it comes after this CTA's tensor memory is allocated, so
+// that a successor's CTA can never take columns its predecessor still has to get.
+__device__ __forceinline__ void grid_dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ void grid_dep_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Plain arrive (release semantics, shared::cta).
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");

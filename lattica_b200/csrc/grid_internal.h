@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/grid_gpu.h"
+#include "balanced.cuh"
 #include "grid_field.cuh"
 
 namespace grid {
@@ -177,9 +178,10 @@ struct EmmPmGeometry {
 };
 bool emm_pm_geometry(const grid_gpu_plan* p, int M, int N, int K, int mode, EmmPmGeometry* g);
 size_t emm_pm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode);
+// limbs: the outputs' balanced limbs as well (out may then be null).
 int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N,
                   int K, int ldx, int ldy, int mode, bool symmetrize, uint32_t* out,
-                  uint32_t* work, cudaStream_t s);
+                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s);
 // Row stride of point-major evaluations of rows of n polys: whole 16-byte units.
 inline size_t pm_stride(size_t n) { return (n + 3) / 4 * 4; }
 // in [rows][cols][d] -> out [d][rows][ld], words past cols zero
@@ -189,7 +191,7 @@ int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t rows, size_t
 // transformed, out [output][64]. sym_r > 0: part holds the dense sym_r x sym_r product C
 // and the outputs are the packed upper triangle of (C_ij + C_ji) / 2.
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
-                       int sym_r, uint32_t* out, cudaStream_t s);
+                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s);
 // The least workspace grid_gpu_gram_dev runs in (grid_gpu_gram_workspace: what it runs
 // best in).
 int gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes);
@@ -204,6 +206,7 @@ int launch_add(const grid_gpu_plan* p, uint32_t* dst, const uint32_t* rhs, size_
 // decompose.cu
 int launch_decompose_balanced(const grid_gpu_plan* p, const uint32_t* polys, size_t npolys,
                               uint64_t base, size_t num_limbs, uint32_t* out, cudaStream_t s);
+bool limbs_ok(uint64_t base, size_t num_limbs);  // what launch_decompose_balanced takes
 int launch_gadget_decompose(const grid_gpu_plan* p, const uint32_t* x, size_t len, uint64_t base,
                             size_t digits, int digit_major, uint32_t* out, cudaStream_t s);
 size_t gadget_digit_count(uint64_t q, uint64_t base);
@@ -235,9 +238,11 @@ void crt_consts(uint32_t q, CrtConsts* c);
 // terms * d * (q - 1)^2 < 2^93: every output coefficient sums at most terms * d
 // word products, within the reconstruction's range
 bool crt_bound_ok(const grid_gpu_plan* p, size_t terms);
-// out = Montgomery word mod q of the integer whose words mod p_j are w_j
+// out = Montgomery word mod q of the integer whose words mod p_j are w_j; limbs: the
+// balanced limbs of the polynomials as well (out may then be null)
 int crt_combine(const grid_gpu_plan* p, const uint32_t* w0, const uint32_t* w1,
-                const uint32_t* w2, size_t words, uint32_t* out, cudaStream_t s);
+                const uint32_t* w2, size_t words, uint32_t* out, cudaStream_t s,
+                const LimbSpec& limbs = LimbSpec());
 
 // plan.cu
 int host_pipeline(grid_gpu_plan* p, const uint32_t* const* ins, int nin, uint32_t* out,
@@ -279,6 +284,25 @@ struct Carver {
     return p;
   }
 };
+
+// A launch that may overlap its predecessor's tail in the stream (grid_dep_wait in the
+// kernel): barriers, tensor memory and constant tables are set up while the predecessor
+// finishes.
+template <typename... P, typename... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                   A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
 
 // Sets the dynamic shared-memory limit of `kernel` once per device and caches
 // its resident blocks per SM (idempotent; benign if two threads race).

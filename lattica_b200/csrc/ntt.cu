@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(D * kSmallSlots) commit_small_kernel(
 // 32 outputs point by point (reads along the outputs, 128 bytes per point and
 // split), and eight threads per output run its inverse transform from shared memory.
 // One launch instead of a transposing sum and a transform of its own, whose 64 KB
-// matrix copy a few hundred polynomials do not pay for (the Gram of r = 30, n = 1021 went
+// matrix copy a few hundred polynomials do not pay for; the prover round's balanced
+// limbs come out of the same registers (the Gram of r = 30, n = 1021 went
 // from 41 to 27 us a call with this and the products' byte planes, u1 and u2 of the outer
 // commitment at r = 64 from 204 to 130).
 // kSym: output (i, j) is (C_ij + C_ji) / 2 of a dense r x r product (garbage h).
@@ -625,13 +626,15 @@ constexpr int kSiThreads = kSiPolys * kSmallT;
 template <bool kSym>
 __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
     const uint32_t* __restrict__ part, int outputs, int splits, int r, uint32_t two_inv,
-    uint32_t* __restrict__ out, const uint2* __restrict__ gtw, FieldParams f) {
+    uint32_t* __restrict__ out, LimbSpec limbs, const uint2* __restrict__ gtw, FieldParams f) {
   constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2;
   constexpr int PS = D + 1;  // the 32 outputs of a point fall in distinct banks
   __shared__ uint2 tws[TWN];
   __shared__ uint32_t sh[kSiPolys * PS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < TWN; i += kSiThreads) tws[i] = gtw[i];
+  grid_dep_wait();
+  grid_dep_launch();
   const int o = blockIdx.x * kSiPolys + lane;
   const bool valid = o < outputs;
   int at = o, mirror = 0;
@@ -679,10 +682,13 @@ __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
   invT_stages<D, T, 1>(x, tws, t, c);
   const int po = blockIdx.x * kSiPolys + pl;
   if (po < outputs) {
-    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)po * D);
 #pragma unroll
-    for (int m = 0; m < E / 4; ++m)
-      dst[T * m + t] = make_uint4(x[4 * m + 0], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]);
+    for (int m = 0; m < E / 4; ++m) {
+      const uint4 v = make_uint4(x[4 * m + 0], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]);
+      if (out) reinterpret_cast<uint4*>(out + (size_t)po * D)[T * m + t] = v;
+      if (limbs.out)
+        store_limbs4(v, limbs.out + (size_t)po * limbs.limbs * D + 4 * (T * m + t), D, limbs, f);
+    }
   }
 }
 
@@ -781,7 +787,7 @@ int launch_ntt(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32
 }
 
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
-                       int sym_r, uint32_t* out, cudaStream_t s) {
+                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s) {
   if (p->d != 64) return GRID_ERR_UNSUPPORTED_DEGREE;
   if (sym_r) outputs = sym_r * (sym_r + 1) / 2;
   if (outputs <= 0) return GRID_OK;
@@ -789,13 +795,10 @@ int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs
   const uint32_t two_inv =
       (uint32_t)(((unsigned __int128)((p->f.q + 1ull) / 2) << 32) % p->f.q);
   const unsigned grid = (unsigned)((outputs + kSiPolys - 1) / kSiPolys);
-  if (sym_r)
-    sum_inverse_kernel<true><<<grid, kSiThreads, 0, s>>>(part, outputs, splits, sym_r, two_inv, out,
-                                                         p->d_tw, p->f);
-  else
-    sum_inverse_kernel<false><<<grid, kSiThreads, 0, s>>>(part, outputs, splits, 0, two_inv, out,
-                                                          p->d_tw, p->f);
-  return cuda_status(cudaGetLastError());
+  return sym_r ? launch_chained(sum_inverse_kernel<true>, dim3(grid), kSiThreads, 0, s, part, outputs,
+                                splits, sym_r, two_inv, out, limbs, p->d_tw, p->f)
+               : launch_chained(sum_inverse_kernel<false>, dim3(grid), kSiThreads, 0, s, part,
+                                outputs, splits, 0, two_inv, out, limbs, p->d_tw, p->f);
 }
 
 bool commit_small_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {

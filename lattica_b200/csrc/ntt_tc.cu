@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc::fence_after_sync();
   const uint32_t tbase = *taddr_slot;
   const uint32_t R0 = tbase, R1 = tbase + 256;
+  grid_dep_wait();
+  grid_dep_launch();
 
   // Point-major mode with a tile list (ptiles): tile t reads 128 polys from
   // row x, stores them at column y, and rows from z on (past an instance) as 0.
@@ -401,10 +403,10 @@ int run_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_
   TcConsts k;
   k.q = p->f.q;
   k.qinv = p->f.qinv;
-  ntt_tc_kernel<MODE><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(
-      map_a, map_out, a, b, (unsigned long long)npolys, reinterpret_cast<const uint4*>(p->d_tcw), k,
-      p->d_err, ptiles, nptiles, row_polys);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(ntt_tc_kernel<MODE>, dim3((unsigned)grid), THREADS, SMEM_BYTES, s, map_a,
+                        map_out, a, b, (unsigned long long)npolys,
+                        reinterpret_cast<const uint4*>(p->d_tcw), k, p->d_err, ptiles, nptiles,
+                        row_polys);
 }
 
 }  // namespace

@@ -84,12 +84,18 @@ __device__ __forceinline__ uint32_t crt_word(uint32_t w0, uint32_t w1, uint32_t 
 
 __global__ void crt_combine_kernel(const uint4* __restrict__ w0, const uint4* __restrict__ w1,
                                    const uint4* __restrict__ w2, size_t n4,
-                                   uint4* __restrict__ out, CrtConsts c) {
+                                   uint4* __restrict__ out, CrtConsts c, LimbSpec l,
+                                   uint32_t d) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
     const uint4 a = w0[i], b = w1[i], e = w2[i];
-    out[i] = make_uint4(crt_word(a.x, b.x, e.x, c), crt_word(a.y, b.y, e.y, c),
-                        crt_word(a.z, b.z, e.z, c), crt_word(a.w, b.w, e.w, c));
+    const uint4 v = make_uint4(crt_word(a.x, b.x, e.x, c), crt_word(a.y, b.y, e.y, c),
+                               crt_word(a.z, b.z, e.z, c), crt_word(a.w, b.w, e.w, c));
+    if (out) out[i] = v;
+    if (l.out) {
+      const size_t poly = i / (d / 4);
+      store_limbs4(v, l.out + poly * (size_t)l.limbs * d + 4 * (i % (d / 4)), (int)d, l, c.fq);
+    }
   }
 }
 
@@ -141,13 +147,14 @@ bool crt_bound_ok(const grid_gpu_plan* p, size_t terms) {
 }
 
 int crt_combine(const grid_gpu_plan* p, const uint32_t* w0, const uint32_t* w1,
-                const uint32_t* w2, size_t words, uint32_t* out, cudaStream_t s) {
+                const uint32_t* w2, size_t words, uint32_t* out, cudaStream_t s,
+                const LimbSpec& limbs) {
   if (words == 0) return GRID_OK;
   if (words % 4) return GRID_ERR_INVALID_PARAMETERS;
   const size_t n4 = words / 4;
   crt_combine_kernel<<<grid_for(p, n4), 256, 0, s>>>(
       reinterpret_cast<const uint4*>(w0), reinterpret_cast<const uint4*>(w1),
-      reinterpret_cast<const uint4*>(w2), n4, reinterpret_cast<uint4*>(out), p->crt_c);
+      reinterpret_cast<const uint4*>(w2), n4, reinterpret_cast<uint4*>(out), p->crt_c, limbs, p->d);
   return cuda_status(cudaGetLastError());
 }
 
