@@ -88,16 +88,6 @@ struct PmShape {
   static_assert(PLANES >= (UPPER ? (uint32_t)NP * (NP + 1) / 2 : (uint32_t)MX * NP) * 4, "staging");
 };
 
-// Bounded wait by lane 0 alone (mbarrier operations of a whole warp on one
-// barrier serialise over its lanes); __syncwarp then orders what lane 0
-// acquired before every lane's later accesses.
-__device__ __forceinline__ bool lane0_wait(uint64_t* bar, uint32_t parity, int lane, int* err) {
-  bool ok = true;
-  if (lane == 0) ok = mbar_wait(bar, parity, err);
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0);
-}
-
 // The builder warps' own barrier (named barrier 1; the CTA's is 0).
 __device__ __forceinline__ void builders_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(kPmBuilders) : "memory");

@@ -74,7 +74,7 @@ struct grid_gpu_plan {
   // Device copy of the twiddle table as uint2 {w, wq}: fw[d], iw[d], {ninv}, {izeta1*ninv}.
   uint2* d_tw = nullptr;
   // Tensor-core tables. d = 64: byte planes of the Montgomery-form forward /
-  // inverse matrices (2 x 64 KB). d = 256: the 64-point matrix (64 KB) and the
+  // inverse matrices (2 x 64 KB) and of the products' inverse (32 KB). d = 256: the 64-point matrix (64 KB) and the
   // twist constants of the products. Null selects the CUDA-core kernels.
   void* d_tcw = nullptr;
   bool tc_emm = false;  // evaluation-domain products on the tensor cores where the shape allows
@@ -126,10 +126,14 @@ int launch_commit_small(const grid_gpu_plan* p, const uint32_t* A_evals, size_t 
                         cudaStream_t st);
 // ntt_tc.cu (d = 64, tcgen05)
 bool ntt_tc_available(const grid_gpu_plan* p);
-int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32_t* b,
-                  uint32_t* out, size_t npolys, cudaStream_t s);
+int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, uint32_t* out,
+                  size_t npolys, cudaStream_t s);  // MODE_FWD or MODE_INV
 void build_tc_tables(uint32_t q, uint32_t d, uint64_t psi, uint64_t ninv,
                      std::vector<unsigned char>& out);
+// ntt_mul_tc.cu (d = 64 products, tcgen05): out = INTT(NTT(a) (.) b); out may be a or b
+int launch_ntt_mul_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* b, uint32_t* out,
+                      size_t npolys, cudaStream_t s);
+void build_tc_mul_table(uint32_t q, uint64_t psi, uint64_t ninv, std::vector<unsigned char>& out);
 // a [rows][n] polys -> out [64 points][rows][pm_stride(n)] (pad words undefined).
 int launch_ntt_tc_pm(const grid_gpu_plan* p, const uint32_t* a, size_t rows, size_t n,
                      uint32_t* out, cudaStream_t s);

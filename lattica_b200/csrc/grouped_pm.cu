@@ -90,15 +90,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Bounded wait by lane 0; __syncwarp orders what lane 0 acquired before every
-// lane's later accesses.
-__device__ __forceinline__ bool lane0_wait(uint64_t* bar, uint32_t parity, int lane, int* err) {
-  bool ok = true;
-  if (lane == 0) ok = mbar_wait(bar, parity, err);
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0);
-}
-
 __device__ __forceinline__ uint32_t item_chunks(const WorkDev& w) {
   return (w.k1 - w.k0 + KCH - 1) / KCH;
 }

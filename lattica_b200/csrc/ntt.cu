@@ -775,7 +775,9 @@ int launch_ntt(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32
                uint32_t* out, size_t npolys, cudaStream_t s) {
   if (is_crt(p)) return p->ntt_status;  // q has no 2d-th root: no transform exists
   if (npolys == 0) return GRID_OK;
-  if (ntt_tc_available(p)) return launch_ntt_tc(p, mode, a, b, out, npolys, s);
+  if (ntt_tc_available(p))
+    return mode == MODE_MULINV ? launch_ntt_mul_tc(p, a, b, out, npolys, s)
+                               : launch_ntt_tc(p, mode, a, out, npolys, s);
   if (mode == MODE_MULINV && ntt256_tc_available(p))
     return launch_ntt256_tc(p, a, b, out, npolys, s);
   switch (mode) {

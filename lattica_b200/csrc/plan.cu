@@ -481,10 +481,12 @@ int grid_gpu_plan_create(uint64_t q, uint64_t d, grid_gpu_plan** out) {
     p->pm_emm = p->tc_emm && use_point_major();
     if ((d == 64 || d == 256) && use_tensor_cores()) {
       std::vector<unsigned char> tcw;
-      if (d == 64)
+      if (d == 64) {
         build_tc_tables(p->q, p->d, p->psi_value, p->n_inv_value, tcw);
-      else
+        build_tc_mul_table(p->q, p->psi_value, p->n_inv_value, tcw);
+      } else {
         build_tc256_tables(p->q, p->psi_value, tcw);
+      }
       if ((e = cudaMalloc(&p->d_tcw, tcw.size())) != cudaSuccess) break;
       if ((e = cudaMemcpy(p->d_tcw, tcw.data(), tcw.size(), cudaMemcpyHostToDevice)) !=
           cudaSuccess)
