@@ -11,6 +11,7 @@ of Montgomery words shaped (..., len, d) on the host, or CUDA int32 tensors.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from dataclasses import dataclass
 
 import numpy as np
@@ -54,6 +55,7 @@ class PreparedMatrix:
         raise_status(st, "grid_gpu_matrix_create")
         self._h, self._lib, self.plan = h, lib, plan
         self.rows, self.cols = rows, cols
+        self._ws_bytes = {}  # batch -> workspace bytes, the few batch sizes of a program
 
     @property
     def handle(self):
@@ -71,25 +73,34 @@ class PreparedMatrix:
             pass
 
     def workspace_bytes(self, batch: int) -> int:
+        known = self._ws_bytes.get(batch)
+        if known is not None:
+            return known
         n = C.c_size_t()
         raise_status(self._lib.grid_gpu_commit_workspace(self._h, batch, C.byref(n)),
                      "grid_gpu_commit_workspace")
+        if len(self._ws_bytes) >= 64:
+            self._ws_bytes.clear()
+        self._ws_bytes[batch] = n.value
         return n.value
 
     def mul_vec(self, s):
         """t[b] = A * s[b] for s shaped (batch, cols, d) (RingMat::mul_slice /
         mul_matrix_vector_runtime)."""
         d = self.plan.d
-        if tuple(s.shape[-2:]) != (self.cols, d):
+        shape = tuple(s.shape)
+        if shape[-2:] != (self.cols, d):
             raise CommitmentError("DimensionMismatch")
-        batch = int(np.prod(s.shape[:-2])) if len(s.shape) > 2 else 1
+        lead = shape[:-2]
+        batch = math.prod(lead)
         if _is_torch(s):
             import torch
-            t = torch.empty((*s.shape[:-2], self.rows, d), dtype=s.dtype, device=s.device)
-            ws = torch.empty(max(16, self.workspace_bytes(batch)), dtype=torch.uint8,
-                             device=s.device)
+            t = s.new_empty((*lead, self.rows, d))
+            need = self.workspace_bytes(batch)  # 0: one launch does without
+            ws = s.new_empty(need, dtype=torch.uint8) if need else None
             st = self._lib.grid_gpu_commit_dev(self._h, s.data_ptr(), batch, t.data_ptr(),
-                                               ws.data_ptr(), ws.numel(), _stream_ptr(s))
+                                               ws.data_ptr() if need else None, need,
+                                               _stream_ptr(s))
         else:
             s = np.ascontiguousarray(s, dtype=np.uint32)
             t = np.empty((*s.shape[:-2], self.rows, d), dtype=np.uint32)

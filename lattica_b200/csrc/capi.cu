@@ -28,6 +28,7 @@ bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, int mode) {
 size_t commit_ws_bytes(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
   if (is_crt(p))
     return 3 * words_bytes(batch * rows * p->d) + commit_ws_bytes(p->crt[0], rows, cols, batch);
+  if (commit_small_fits(p, rows, cols, batch)) return 0;  // one launch, no intermediate
   return words_bytes(batch * pm_stride(cols) * p->d) +
          words_bytes(emm_workspace_words(p, (int)batch, (int)rows, (int)cols, EMM_DENSE));
 }

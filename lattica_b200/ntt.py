@@ -65,8 +65,10 @@ def _is_torch(x) -> bool:
 
 
 def _stream_ptr(t) -> int:
+    """The current stream of t's device as an integer, without building a Stream
+    object (0.2 us against 2.5 us, a seventh of a small commitment's call)."""
     import torch
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 def _host_u32(a: np.ndarray) -> np.ndarray:
