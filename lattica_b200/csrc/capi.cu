@@ -29,6 +29,8 @@ size_t commit_ws_bytes(const grid_gpu_plan* p, size_t rows, size_t cols, size_t 
   if (is_crt(p))
     return 3 * words_bytes(batch * rows * p->d) + commit_ws_bytes(p->crt[0], rows, cols, batch);
   if (commit_small_fits(p, rows, cols, batch)) return 0;  // one launch, no intermediate
+  if (commit_vec_fits(p, rows, cols, batch))
+    return words_bytes(commit_vec_words(p, rows, cols, 0, batch));
   return words_bytes(batch * pm_stride(cols) * p->d) +
          words_bytes(emm_workspace_words(p, (int)batch, (int)rows, (int)cols, EMM_DENSE));
 }
@@ -104,6 +106,14 @@ int prepare_evals(grid_gpu_matrix* m, const uint32_t* A, bool a_is_evals, cudaSt
   return rc;
 }
 
+// Two products of a few vectors as one (both too long for the one-launch kernel).
+bool linear_vec_fits(const grid_gpu_matrix* A, const grid_gpu_matrix* B, size_t batch) {
+  const grid_gpu_plan* p = A->plan;
+  return commit_vec_fits(p, A->rows, A->cols + B->cols, batch) &&
+         !commit_small_fits(p, A->rows, A->cols, batch) &&
+         !commit_small_fits(p, B->rows, B->cols, batch);
+}
+
 // t = A * s for `batch` vectors, into t (coefficients). ws from a Carver.
 int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint32_t* t,
                 Carver& cv, cudaStream_t st) {
@@ -123,6 +133,12 @@ int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint3
   }
   if (commit_small_fits(p, A->rows, A->cols, batch))
     return launch_commit_small(p, A->d_evals, A->rows, A->cols, A->ld, s, batch, t, st);
+  if (commit_vec_fits(p, A->rows, A->cols, batch)) {
+    uint32_t* part = cv.take<uint32_t>(commit_vec_words(p, A->rows, A->cols, 0, batch));
+    if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+    return launch_commit_vec(p, VecOperand{A->d_evals, s, A->cols, A->ld}, nullptr, A->rows, batch,
+                             t, part, st);
+  }
   const size_t ldx = pm_stride(A->cols);
   uint32_t* s_hat = cv.take<uint32_t>(batch * ldx * p->d);
   const size_t ew = emm_workspace_words(p, (int)batch, (int)A->rows, (int)A->cols, EMM_DENSE);
@@ -141,6 +157,32 @@ int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint3
                     EMM_DENSE, t, work, st);
   if (rc) return rc;
   return launch_ntt(p, MODE_INV, t, nullptr, t, batch * A->rows, st);
+}
+
+// t = A m + B r, t2: scratch of t's size (coefficients).
+int linear_core(const grid_gpu_matrix* A, const grid_gpu_matrix* B, const uint32_t* m,
+                const uint32_t* r, size_t batch, uint32_t* t, uint32_t* t2, Carver& cv,
+                cudaStream_t st) {
+  const grid_gpu_plan* p = A->plan;
+  if (linear_vec_fits(A, B, batch)) {
+    uint32_t* part = cv.take<uint32_t>(commit_vec_words(p, A->rows, A->cols, B->cols, batch));
+    if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+    const VecOperand second{B->d_evals, r, B->cols, B->ld};
+    return launch_commit_vec(p, VecOperand{A->d_evals, m, A->cols, A->ld}, &second, A->rows, batch,
+                             t, part, st);
+  }
+  int rc = commit_core(A, m, batch, t, cv, st);
+  if (!rc) rc = commit_core(B, r, batch, t2, cv, st);
+  // A_msg*m + A_open*r: INTT is linear, so adding the coefficient forms is exact.
+  if (!rc) rc = launch_add(p, t, t2, batch * B->rows * p->d, st);
+  return rc;
+}
+
+size_t linear_ws_bytes(const grid_gpu_matrix* A, const grid_gpu_matrix* B, size_t batch) {
+  const grid_gpu_plan* p = A->plan;
+  if (linear_vec_fits(A, B, batch))
+    return words_bytes(commit_vec_words(p, A->rows, A->cols, B->cols, batch));
+  return commit_ws_bytes(p, A->rows, A->cols, batch) + commit_ws_bytes(p, B->rows, B->cols, batch);
 }
 
 }  // namespace
@@ -316,9 +358,7 @@ int grid_gpu_linear_commit_workspace(const grid_gpu_matrix* A_msg, const grid_gp
                                      size_t batch, size_t* bytes) {
   if (!A_msg || !A_open || !bytes) return GRID_ERR_NULL_POINTER;
   const grid_gpu_plan* p = A_msg->plan;
-  *bytes = commit_ws_bytes(p, A_msg->rows, A_msg->cols, batch) +
-           commit_ws_bytes(p, A_open->rows, A_open->cols, batch) +
-           words_bytes(batch * A_open->rows * p->d);
+  *bytes = linear_ws_bytes(A_msg, A_open, batch) + words_bytes(batch * A_open->rows * p->d);
   return GRID_OK;
 }
 
@@ -338,11 +378,7 @@ int grid_gpu_linear_commit_dev(const grid_gpu_matrix* A_msg, const grid_gpu_matr
   Carver cv(workspace, workspace_bytes);
   uint32_t* t2 = cv.take<uint32_t>(batch * A_open->rows * p->d);
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-  int rc = commit_core(A_msg, m, batch, t, cv, st);
-  if (!rc) rc = commit_core(A_open, r, batch, t2, cv, st);
-  // A_msg*m + A_open*r: INTT is linear, so adding the coefficient forms is exact.
-  if (!rc) rc = launch_add(p, t, t2, batch * A_open->rows * p->d, st);
-  return rc;
+  return linear_core(A_msg, A_open, m, r, batch, t, t2, cv, st);
 }
 
 int grid_gpu_linear_commit(grid_gpu_matrix* A_msg, grid_gpu_matrix* A_open, const uint32_t* m,
@@ -356,8 +392,7 @@ int grid_gpu_linear_commit(grid_gpu_matrix* A_msg, grid_gpu_matrix* A_open, cons
   const size_t rows = A_msg->rows, d = p->d;
   const size_t m_bytes = batch * A_msg->cols * d * 4, r_bytes = batch * A_open->cols * d * 4;
   const size_t t_bytes = batch * rows * d * 4;
-  const size_t ws = commit_ws_bytes(p, rows, A_msg->cols, batch) +
-                    commit_ws_bytes(p, rows, A_open->cols, batch);
+  const size_t ws = linear_ws_bytes(A_msg, A_open, batch);
   int rc;
   if ((rc = ensure_scratch(p, 6, m_bytes)) || (rc = ensure_scratch(p, 7, r_bytes)) ||
       (rc = ensure_scratch(p, 9, t_bytes)) || (rc = ensure_scratch(p, 10, t_bytes)) ||
@@ -372,11 +407,8 @@ int grid_gpu_linear_commit(grid_gpu_matrix* A_msg, grid_gpu_matrix* A_open, cons
   if (!rc) rc = cuda_status(cudaMemcpyAsync(dr, r, r_bytes, cudaMemcpyHostToDevice, st));
   if (!rc) {
     Carver cv(p->scratch[8].ptr, ws);
-    rc = commit_core(A_msg, dm, batch, t1, cv, st);
-    if (!rc) rc = commit_core(A_open, dr, batch, t2, cv, st);
+    rc = linear_core(A_msg, A_open, dm, dr, batch, t1, t2, cv, st);
   }
-  // A_msg*m + A_open*r: INTT is linear, so adding the coefficient forms is exact.
-  if (!rc) rc = launch_add(p, t1, t2, batch * rows * d, st);
   if (!rc) rc = cuda_status(cudaMemcpyAsync(t, t1, t_bytes, cudaMemcpyDeviceToHost, st));
   const int fin = finish_host_call(p, st);
   return rc ? rc : fin;
@@ -389,9 +421,7 @@ int grid_gpu_bdlop_workspace(const grid_gpu_matrix* A_mask, const grid_gpu_matri
   if (!A_mask || !A_msg || !A_open || !bytes) return GRID_ERR_NULL_POINTER;
   const grid_gpu_plan* p = A_msg->plan;
   *bytes = commit_ws_bytes(p, A_mask->rows, A_mask->cols, batch) +
-           commit_ws_bytes(p, A_msg->rows, A_msg->cols, batch) +
-           commit_ws_bytes(p, A_open->rows, A_open->cols, batch) +
-           words_bytes(batch * A_open->rows * p->d);
+           linear_ws_bytes(A_msg, A_open, batch) + words_bytes(batch * A_open->rows * p->d);
   return GRID_OK;
 }
 
@@ -417,10 +447,7 @@ int grid_gpu_bdlop_commit_dev(const grid_gpu_matrix* A_mask, const grid_gpu_matr
   uint32_t* t2 = cv.take<uint32_t>(batch * A_open->rows * p->d);
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
   int rc = commit_core(A_mask, r, batch, u, cv, st);
-  if (!rc) rc = commit_core(A_msg, m, batch, v, cv, st);
-  if (!rc) rc = commit_core(A_open, r, batch, t2, cv, st);
-  // A_msg*m + A_open*r: INTT is linear, so adding the coefficient forms is exact.
-  if (!rc) rc = launch_add(p, v, t2, batch * A_open->rows * p->d, st);
+  if (!rc) rc = linear_core(A_msg, A_open, m, r, batch, v, t2, cv, st);
   return rc;
 }
 

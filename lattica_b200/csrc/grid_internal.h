@@ -124,6 +124,17 @@ bool commit_small_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t 
 int launch_commit_small(const grid_gpu_plan* p, const uint32_t* A_evals, size_t rows,
                         size_t cols, size_t ld, const uint32_t* s, size_t batch, uint32_t* t,
                         cudaStream_t st);
+// A matrix times one to four vectors, or the sum of two such products, in two launches
+// (d = 64, rows <= 64): t = A0 s0 (+ A1 s1) for `batch` vectors. part: >= commit_vec_words.
+struct VecOperand {
+  const uint32_t *A, *s;  // evaluations [rows][ld][d], vectors [batch][cols][d]
+  size_t cols, ld;
+};
+bool commit_vec_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch);
+size_t commit_vec_words(const grid_gpu_plan* p, size_t rows, size_t cols0, size_t cols1,
+                        size_t batch);
+int launch_commit_vec(const grid_gpu_plan* p, const VecOperand& o0, const VecOperand* o1,
+                      size_t rows, size_t batch, uint32_t* t, uint32_t* part, cudaStream_t s);
 // ntt_tc.cu (d = 64, tcgen05)
 bool ntt_tc_available(const grid_gpu_plan* p);
 int launch_ntt_tc(const grid_gpu_plan* p, int mode, const uint32_t* a, uint32_t* out,

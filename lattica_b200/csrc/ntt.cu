@@ -610,6 +610,145 @@ __global__ void __launch_bounds__(D * kSmallSlots) commit_small_kernel(
 }
 
 // ---------------------------------------------------------------------------
+// A matrix times a few vectors (outer commitments, single commits): t = A s, up to
+// 64 outputs (rows times vectors) of any length, or the sum of two such products
+// (A_msg m + A_open r). The matrix's evaluations are read once from HBM and bound it
+// (16 x 8320 polys: 34 MB, 5.2 us at the measured rate); a tensor-core product would
+// spend 44 cycles on every MMA for one useful row of 128.
+//  * vec_partial_kernel: a CTA takes up to 64 columns at a time of one product: eight
+//    threads transform each polynomial (as in commit_small_kernel), thread (e, slot)
+//    accumulates evaluation point e of rows slot, slot + 8, ... over the columns; the
+//    canonical sums go to part [cta][row][e].
+//  * vec_finish_kernel: a CTA per output polynomial sums the partials and inverts.
+// Two launches for the sum of two products, where each took a transform, a product and
+// an inverse of its own and an addition. u1 = B t + C g and u2 = D h of the LaBRADOR level
+// at r = 64, kappa = 16: 119 us before, 45 us now.
+// ---------------------------------------------------------------------------
+constexpr int kVecMaxRows = 64, kVecMaxBatch = 4, kVecCols = 64;
+constexpr int kVecThreads = 512;
+
+struct VecProduct {
+  const uint32_t *A, *s;  // evaluations [rows][ld][64]; vectors [batch][cols][64]
+  int cols, ld;
+  int ctas;               // CTAs of this product, each `span` columns
+  int span;
+};
+
+template <int RPT>
+__global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
+    const VecProduct p0, const VecProduct p1, int rows, uint32_t* __restrict__ part,
+    const uint2* __restrict__ gtw, FieldParams f) {
+  constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, PS = D + 4 * T, TWN = 2 * D + 2;
+  __shared__ uint2 tws[TWN];
+  __shared__ __align__(16) uint32_t sh[kVecCols * PS];
+  const int tid = threadIdx.x;
+  for (int i = tid; i < TWN; i += kVecThreads) tws[i] = gtw[i];
+  __syncthreads();
+  grid_dep_wait();
+  grid_dep_launch();
+  const bool second = (int)blockIdx.x >= p0.ctas;
+  const VecProduct& p = second ? p1 : p0;
+  const int c0 = ((int)blockIdx.x - (second ? p0.ctas : 0)) * p.span;
+  const int c1 = min(p.cols, c0 + p.span);
+  const uint32_t* s = p.s + (size_t)blockIdx.y * p.cols * D;
+  const int pl = tid / T, t = tid % T;
+  const int bt_t = brv(4 * t, LOGD);
+  const Consts c = consts_of(f);
+  const int e = tid % D, slot = tid / D;
+  Acc96 acc[RPT];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) acc96_zero(acc[i]);
+  for (int k0 = c0; k0 < c1; k0 += kVecCols) {  // uniform over the CTA
+    const int n = min(kVecCols, c1 - k0);
+    {  // groups past the last polynomial transform zeros
+      uint32_t x[E];
+#pragma unroll
+      for (int m = 0; m < E / 4; ++m) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (pl < n) v = __ldg(reinterpret_cast<const uint4*>(s + (size_t)(k0 + pl) * D) + T * m + t);
+        x[4 * m + 0] = v.x;
+        x[4 * m + 1] = v.y;
+        x[4 * m + 2] = v.z;
+        x[4 * m + 3] = v.w;
+      }
+      fwdT_stages<D, T, D / 2>(x, tws, t, c);  // ends with a CTA barrier
+#pragma unroll
+      for (int i = 0; i < E; ++i)  // lazy words -> canonical, slot order
+        sh[pl * PS + (brv(4 * T * (i >> 2) + (i & 3), LOGD) | bt_t)] =
+            mont_v(x[i], c.r1, c.q, c.qinv);
+    }
+    __syncthreads();
+    // a group of columns' matrix loads are issued before the first is used
+    constexpr int KB = 16 / RPT;
+    for (int kk = 0; kk < n; kk += KB) {
+      uint32_t av[RPT][KB], sv[KB];
+#pragma unroll
+      for (int j = 0; j < KB; ++j) {
+        sv[j] = kk + j < n ? sh[(kk + j) * PS + e] : 0u;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const int r = slot + kSmallSlots * i;
+          av[i][j] = kk + j < n && r < rows
+                         ? __ldg(p.A + ((size_t)r * p.ld + k0 + kk + j) * D + e)
+                         : 0u;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < KB; ++j)
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) acc96_mad(acc[i], av[i][j], sv[j]);
+    }
+    __syncthreads();
+  }
+  uint32_t* o = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * rows * D;
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = slot + kSmallSlots * i;
+    if (r < rows) o[r * D + e] = acc96_reduce(acc[i], f);
+  }
+}
+
+constexpr int kVfThreads = 256;
+
+__global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
+    const uint32_t* __restrict__ part, int count, int rows, uint32_t* __restrict__ t_out,
+    const uint2* __restrict__ gtw, FieldParams f) {
+  constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2, G = kVfThreads / D;
+  __shared__ uint2 tws[TWN];
+  __shared__ unsigned long long sums[G][D];
+  __shared__ uint32_t sh[D];
+  const int tid = threadIdx.x, e = tid % D, g = tid / D;
+  for (int i = tid; i < TWN; i += kVfThreads) tws[i] = gtw[i];
+  grid_dep_wait();
+  grid_dep_launch();
+  const uint32_t* src = part + ((size_t)blockIdx.y * count * rows + blockIdx.x) * D + e;
+  unsigned long long v = 0;  // count canonical words stay below 2^64
+#pragma unroll 8
+  for (int i = g; i < count; i += G) v += __ldg(src + (size_t)i * rows * D);
+  sums[g][e] = v;
+  __syncthreads();
+  if (g == 0) {
+#pragma unroll
+    for (int i = 1; i < G; ++i) v += sums[i][e];
+    sh[e] = (uint32_t)(v % f.q);
+  }
+  __syncthreads();
+  // eight threads invert; the others repeat them (the stages hold CTA barriers)
+  const int t = tid % T, bt_t = brv(4 * t, LOGD);
+  const Consts c = consts_of(f);
+  uint32_t x[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) x[i] = sh[brv(4 * T * (i >> 2) + (i & 3), LOGD) | bt_t];
+  invT_stages<D, T, 1>(x, tws, t, c);
+  if (tid < T) {
+    uint4* dst = reinterpret_cast<uint4*>(t_out + ((size_t)blockIdx.y * rows + blockIdx.x) * D);
+#pragma unroll
+    for (int m = 0; m < E / 4; ++m)
+      dst[T * m + t] = make_uint4(x[4 * m + 0], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // The end of a point-major contraction (emm_pm.cu): a CTA sums the K-range partials of
 // 32 outputs point by point (reads along the outputs, 128 bytes per point and
 // split), and eight threads per output run its inverse transform from shared memory.
@@ -786,6 +925,57 @@ int launch_ntt(const grid_gpu_plan* p, int mode, const uint32_t* a, const uint32
     case MODE_MULINV: return dispatch<MODE_MULINV>(p, a, b, out, npolys, s);
     default: return GRID_ERR_INVALID_PARAMETERS;
   }
+}
+
+// Every vector reads the matrix again (from L2) and its products run on the integer
+// pipe, where the tensor-core product costs the same for one vector as for eight: 16 x
+// 8320 takes 18.8, 26.9, 34.8, 42.7 us for 1 to 4 vectors (42.4 for 5 there), 32 x 8192 23,
+// 36, 49 (45), 64 x 2048 19, 28 (26), 8 x 4096 30 for 4 (31). So rows * batch <= 64.
+bool commit_vec_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
+  return !is_crt(p) && p->d == 64 && rows >= 1 && rows <= (size_t)kVecMaxRows && cols >= 1 &&
+         cols < (1u << 30) && batch >= 1 && batch <= (size_t)kVecMaxBatch &&
+         rows * batch <= (size_t)kVecMaxRows;
+}
+
+namespace {
+
+// Columns per CTA: two CTAs' worth of SMs in all, 16 to 64 columns each, or several
+// blocks of 64 for longer vectors.
+VecProduct vec_product(const grid_gpu_plan* p, const VecOperand& o, size_t all_cols) {
+  const size_t slots = 2 * (size_t)p->num_sms;
+  size_t span = (all_cols + slots - 1) / slots;
+  span = span < 16 ? 16 : span <= (size_t)kVecCols ? span : round_up(span, kVecCols);
+  VecProduct v{o.A, o.s, (int)o.cols, (int)o.ld, (int)((o.cols + span - 1) / span), (int)span};
+  return v;
+}
+
+}  // namespace
+
+size_t commit_vec_words(const grid_gpu_plan* p, size_t rows, size_t cols0, size_t cols1,
+                        size_t batch) {
+  const VecOperand a{nullptr, nullptr, cols0, 0}, b{nullptr, nullptr, cols1, 0};
+  const size_t all = cols0 + cols1;
+  return (size_t)(vec_product(p, a, all).ctas + (cols1 ? vec_product(p, b, all).ctas : 0)) * rows *
+         64 * batch;
+}
+
+int launch_commit_vec(const grid_gpu_plan* p, const VecOperand& o0, const VecOperand* o1,
+                      size_t rows, size_t batch, uint32_t* t, uint32_t* part, cudaStream_t s) {
+  const size_t all = o0.cols + (o1 ? o1->cols : 0);
+  if (!commit_vec_fits(p, rows, all, batch) || !part) return GRID_ERR_INVALID_PARAMETERS;
+  const VecProduct p0 = vec_product(p, o0, all);
+  const VecProduct p1 = o1 ? vec_product(p, *o1, all) : VecProduct{nullptr, nullptr, 0, 0, 0, 1};
+  const dim3 grid((unsigned)(p0.ctas + p1.ctas), (unsigned)batch);
+  auto run = [&](auto kernel) {
+    return launch_chained(kernel, grid, kVecThreads, 0, s, p0, p1, (int)rows, part, p->d_tw, p->f);
+  };
+  const int rc = rows <= 8    ? run(vec_partial_kernel<1>)
+                 : rows <= 16 ? run(vec_partial_kernel<2>)
+                 : rows <= 32 ? run(vec_partial_kernel<4>)
+                              : run(vec_partial_kernel<8>);
+  if (rc) return rc;
+  return launch_chained(vec_finish_kernel, dim3((unsigned)rows, (unsigned)batch), kVfThreads, 0, s,
+                        part, p0.ctas + p1.ctas, (int)rows, t, p->d_tw, p->f);
 }
 
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
