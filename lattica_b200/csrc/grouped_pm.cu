@@ -359,7 +359,9 @@ int launch_np(const grid_gpu_plan* p, const WorkDev* work, unsigned nwork, const
   TcConsts k;
   k.q = p->f.q;
   k.qinv = p->f.qinv;
-  const unsigned grid = std::min<unsigned>(nwork, (unsigned)(p->num_sms * bps));
+  // Two CTAs per SM (GpShape, 64 registers). The occupancy query answers 1 for any kernel
+  // that allocates tensor memory, whatever its registers and shared memory.
+  const unsigned grid = std::min<unsigned>(nwork, 2u * (unsigned)p->num_sms);
   batch_pm_kernel<NP><<<grid, kGpThreads, S::SMEM, s>>>(
       work, nwork, tiles, items, mats, s_pm, (unsigned long long)ps, acc, (int)p->d,
       make_uint4(c[0], c[1], c[2], 0), make_uint4(cq[0], cq[1], cq[2], 0), k, p->d_err);
