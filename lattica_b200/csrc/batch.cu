@@ -236,8 +236,8 @@ struct Tables {
   bool tc = false;
   bool pm = false;
   unsigned class_begin[TC_CLASSES + 1] = {};
-  // Point-major layout: instance i's polys at a column of a multiple of 128
-  // (ItemDev::s_off of the point-major tables), the transform's tile list.
+  // Point-major layout: a tile's polys in blocks of 128 columns from ItemDev::s_off of
+  // its instances on, and the transform's tile list, one entry per block.
   uint64_t pm_polys = 0;
   std::vector<uint4> xtiles;
 };
@@ -354,7 +354,6 @@ int build_tables(const grid_gpu_plan* plan, grid_gpu_matrix* const* mats, size_t
     if (x.first != y.first) return x.first < y.first;
     return items[x.second].n > items[y.second].n;
   });
-  uint64_t pcol = 0;  // next point-major column
   for (size_t i = 0; i < order.size();) {
     const uint32_t m = order[i].first;
     size_t j = i;
@@ -363,19 +362,33 @@ int build_tables(const grid_gpu_plan* plan, grid_gpu_matrix* const* mats, size_t
     if (tile_instances) cap = std::min<size_t>(cap, tile_instances);
     while (j < order.size() && order[j].first == m && j - i < cap) {
       const grid_gpu_batch_item& it = items[order[j].second];
-      uint64_t s_off = it.s_offset;
-      if (tb.pm) {  // the instance's own 128-aligned columns; the rest of its last tile is 0
-        for (uint32_t r = 0; r < it.n; r += 128)
-          tb.xtiles.push_back(make_uint4((uint32_t)(it.s_offset + r), (uint32_t)(pcol + r),
-                                         std::min<uint32_t>(128, it.n - r), 0));
-        s_off = pcol;
-        pcol += round_up(it.n, 128);
-      }
-      tb.sorted.push_back(ItemDev{s_off, it.t_offset, it.n, 0});
+      tb.sorted.push_back(ItemDev{tb.pm ? 128ull * tb.xtiles.size() : it.s_offset, it.t_offset,
+                                  it.n, 0});
       tl.kmax = std::max(tl.kmax, it.n);
       ++j;
     }
     tl.count = (uint32_t)(j - i);
+    if (tb.pm) {
+      // The tile's evaluations, 128 columns (one transform tile) per block: every live
+      // instance's first block, then every live instance's second, ... (sorted longest
+      // first, so the live ones are a prefix; zeros past an instance's end). A block's
+      // columns are 128 times its index in the list. The c-th entry's fourth word
+      // describes the tile's c-th blocks: first of them (from the tile's first) << 8 | count.
+      const size_t x0 = tb.xtiles.size();
+      std::vector<uint32_t> dir;
+      uint32_t live = tl.count;
+      for (uint32_t k = 0; k < tl.kmax; k += 128) {
+        while (items[order[i + live - 1].second].n <= k) --live;
+        dir.push_back((uint32_t)(tb.xtiles.size() - x0) << 8 | live);
+        for (uint32_t r = 0; r < live; ++r) {
+          const grid_gpu_batch_item& it = items[order[i + r].second];
+          tb.xtiles.push_back(make_uint4((uint32_t)(it.s_offset + k),
+                                         (uint32_t)(128 * tb.xtiles.size()),
+                                         std::min<uint32_t>(128, it.n - k), 0));
+        }
+      }
+      for (size_t c = 0; c < dir.size(); ++c) tb.xtiles[x0 + c].w = dir[c];
+    }
     tb.tiles.push_back(tl);
     i = j;
   }
@@ -444,8 +457,8 @@ size_t ws_bytes(const grid_gpu_batch* b) { return core_bytes(b->s_region, b->t_p
 // point-major with rows of ps polys (the point-major engine's tables).
 int run_product(const grid_gpu_plan* p, bool tc, bool pm, const unsigned* class_begin,
                 const MatDev* d_mats, const ItemDev* d_items, const TileDev* d_tiles,
-                const WorkDev* d_work, unsigned nwork, const uint32_t* s_hat, uint64_t ps,
-                unsigned long long* acc, unsigned* counters, uint64_t t_polys, uint32_t* t,
+                const WorkDev* d_work, unsigned nwork, const uint4* xtiles,
+                const uint32_t* s_hat, uint64_t ps, unsigned long long* acc, unsigned* counters, uint64_t t_polys, uint32_t* t,
                 cudaStream_t st) {
   const size_t d = p->d;
   cudaError_t e = cudaMemsetAsync(acc, 0, t_polys * d * 8, st);
@@ -456,8 +469,8 @@ int run_product(const grid_gpu_plan* p, bool tc, bool pm, const unsigned* class_
     for (int c = 0; c < TC_CLASSES && !rc; ++c) {
       const unsigned n = class_begin[c + 1] - class_begin[c];
       if (n)
-        rc = launch_batch_pm(p, c, d_work + class_begin[c], n, d_tiles, d_items, d_mats, s_hat,
-                             ps, acc, st);
+        rc = launch_batch_pm(p, c, d_work + class_begin[c], n, d_tiles, d_items, d_mats, xtiles,
+                             s_hat, ps, acc, st);
     }
     if (rc) return rc;
   } else if (tc) {
@@ -499,12 +512,12 @@ int run_core(const grid_gpu_plan* p, bool tc, bool pm, const unsigned* class_beg
       reinterpret_cast<unsigned long long*>(base + round_up(ps * d * 4, 256));
   unsigned* counters =
       reinterpret_cast<unsigned*>(base + round_up(ps * d * 4, 256) + round_up(t_polys * d * 8, 256));
-  // point-major: [point][ps], every instance at its own 128-aligned columns
+  // point-major: [point][ps], in blocks of 128 columns (build_tables)
   const int rc = pm ? launch_ntt_tc_pm_tiles(p, s, s_polys, s_hat, ps, xtiles, nxtiles, st)
                     : launch_ntt(p, MODE_FWD, s, nullptr, s_hat, s_polys, st);
   if (rc) return rc;
-  return run_product(p, tc, pm, class_begin, d_mats, d_items, d_tiles, d_work, nwork, s_hat, ps,
-                     acc, counters, t_polys, t, st);
+  return run_product(p, tc, pm, class_begin, d_mats, d_items, d_tiles, d_work, nwork, xtiles,
+                     s_hat, ps, acc, counters, t_polys, t, st);
 }
 
 int run_sequence(grid_gpu_batch* b, const uint32_t* s, uint32_t* t, void* ws, cudaStream_t st) {
@@ -815,7 +828,7 @@ int grid_gpu_batch_gram_dev(const grid_gpu_plan* plan, const uint32_t* S,
   rc = send_tables(tb, base + core, &dm, &di, &dt, &dw, &dx, st);
   if (rc) return rc;
   return run_product(plan, true, false, tb.class_begin, dm, di, dt, dw, (unsigned)tb.work.size(),
-                     s_hat, 0, acc, counters, g_polys, G, st);
+                     nullptr, s_hat, 0, acc, counters, g_polys, G, st);
 }
 
 }  // extern "C"

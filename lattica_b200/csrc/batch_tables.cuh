@@ -53,10 +53,11 @@ int launch_batch_tc(const grid_gpu_plan* p, int cls, const WorkDev* work, unsign
                     cudaStream_t s);
 
 // grouped_pm.cu: the dense classes (TC_D16, TC_D32) over point-major
-// evaluations s_pm [point][ps] (ps >= the packed witness polys, a multiple of 4),
-// one evaluation point per work item (WorkDev::eg = the point).
+// evaluations s_pm [point][ps] (ps >= the packed witness polys, a multiple of 4) in the
+// blocks of the transform's tile list xtiles, one evaluation point per work item
+// (WorkDev::eg = the point).
 int launch_batch_pm(const grid_gpu_plan* p, int cls, const WorkDev* work, unsigned nwork,
                     const TileDev* tiles, const ItemDev* items, const MatDev* mats,
-                    const uint32_t* s_pm, uint64_t ps, unsigned long long* acc, cudaStream_t s);
+                    const uint4* xtiles, const uint32_t* s_pm, uint64_t ps, unsigned long long* acc, cudaStream_t s);
 
 }  // namespace grid

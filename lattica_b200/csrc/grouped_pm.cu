@@ -4,31 +4,38 @@
 //     out_e[i][r] = sum_{k < n_i} s_i,e[k] * A_e[r][k] * 2^-32 (mod q),
 // the point-major counterpart of grouped_tc.cu. The witnesses' forward
 // transform stored [point][poly] (ntt_tc.cu, point-major mode over a tile
-// list), so instance i's words at point e are n_i consecutive words at
-// s_pm + e ps + s_off_i, and matrices keep point-major evaluations
-// [point][row][ld].
+// list); matrices keep point-major evaluations [point][row][ld].
 //
 // A work item is (tile, K range, one evaluation point); a tile holds up to 128
-// instances of one matrix (the MMA's M), sorted longest first. The transform
-// gives every instance its own columns from a multiple of 128, zero past its
-// n_i, so that an instance row's 32-word chunk is 128 aligned bytes. Per chunk:
-//  * warps 4-7 (32 instance rows each) copy the chunk of every instance row
-//    still inside its length (8 lanes per row, 16-byte cp.async), zero-fill
-//    the slot's rows that ran out since the slot was last filled for this
-//    item, and copy the matrix rows into the slot's Y box; their lanes' copy
-//    completions arrive on the slot's mbarrier (cp.async.mbarrier.arrive.noinc);
-//  * warps 0-3 build the four byte planes of the matrix rows, B row l NP + r,
-//    K byte 4k + i = byte l of 2^(8i) A_e[r][k] mod q (emm_tc.cu's method);
-//  * one lane of warp 8 issues four MMAs (M 128, N 4 NP, K 32) into one of two
-//    tensor-memory accumulators (alternating per item) and commits them to the
-//    slots' barriers and, after the item's last chunk, to the accumulator's;
-//  * warps 9-12 combine the planes of a finished item, reduce once and add
+// instances of one matrix (the MMA's M), sorted longest first. A tile's words at a point
+// lie in blocks of 128: the first block of every instance, then the second of every
+// instance that has one, ... (batch.cu), zero past an instance's end. So the K words
+// 128 c .. + 127 of all J live instances are J consecutive rows of 512 bytes, and a chunk,
+// 32 words of each, is at most four TMA boxes of 8 to 64 rows. Per chunk:
+//  * one lane of warp 4 loads it (up to seven rows more, of other instances);
+//  * warps 6 and 7 zero the slot's rows from J on as far as they are not zero yet;
+//  * warps 0-3 build the byte planes of the matrix rows, from words loaded one chunk
+//    ahead: B row c NP + r, K byte 4k + i = byte c - i of A_e[r][k], so that column
+//    c NP + r of the product is the sum of its bytes' products of weight 2^(8c), c < 7
+//    (emm_pm.cu's method);
+//  * one lane of warp 5 issues four MMAs (M 128, N 7 NP, K 32) into a tensor-memory
+//    accumulator (two, alternating per item, up to 16 rows; one beyond, where two would
+//    leave the SM to one CTA) and commits them to the slots' barriers and, after the
+//    item's last chunk, to the accumulator's;
+//  * warps 8-11 combine the classes of a finished item, reduce once and add
 //    each canonical word into the 64-bit accumulator of its output poly and
 //    point, so K ranges of one instance may run in different items.
 // CTAs take the work list's items with a grid stride (longest first), every
 // role walking the same sequence. Instance rows past a tile's count and B rows
 // past the matrix's reach only results that are not stored, so they are never
 // cleared. Every wait is bounded.
+//
+// Bound: reading the evaluations (4.4 TB/s with 8 and 16 rows), then, with 32 rows, the
+// construction of the classes. Both launches of 4096 instances of 64 to 8192 polys, by a
+// profiler: 480 and 422 us with four warps copying every row's 128 bytes from rows an
+// instance apart (cp.async, eight lanes a row: as many issue slots as everything else) and
+// one CTA per SM; 271 and 252 with blocks and TMA; 268 and 203 with unscaled classes
+// instead of four planes of 2^(8i) A (three modular products a word).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -46,71 +53,67 @@ namespace {
 using namespace tcx;
 
 constexpr int kGpBuildWarps = 4;
-constexpr int kGpLoadWarp0 = 4, kGpLoadWarps = 4;  // 32 instance rows each
-constexpr int kGpMmaWarp = 8;
-constexpr int kGpEpiWarp0 = 9, kGpEpiWarps = 4;
+constexpr int kGpLoadWarp = 4, kGpMmaWarp = 5;
+constexpr int kGpZeroWarp0 = 6, kGpZeroWarps = 2;
+constexpr int kGpEpiWarp0 = 8, kGpEpiWarps = 4;
 constexpr int kGpThreads = (kGpEpiWarp0 + kGpEpiWarps) * 32;
-constexpr int kGpLoaders = kGpLoadWarps * 32;
-constexpr int KCH = 32;  // K words per chunk: one 128-byte swizzled row
+constexpr int KCH = 32;     // K words per chunk: one 128-byte swizzled row
+constexpr int KBLK = 128;   // K words per block of the evaluations
 
 template <int NP>
 struct GpShape {
-  static constexpr int NMMA = 4 * NP;            // B rows: four byte planes
-  static constexpr uint32_t XSLOT = 128u * 128;  // 128 instance rows x 128 bytes
-  static constexpr uint32_t YSLOT = NP * 128u;   // matrix rows
-  static constexpr uint32_t ASLOT = XSLOT + YSLOT;
+  static constexpr int NMMA = 7 * NP;            // B rows: seven classes
+  static constexpr uint32_t ASLOT = 128u * 128;  // 128 instance rows x 128 bytes
   static constexpr uint32_t BSLOT = NMMA * 128u;
-  static constexpr int NSB = BSLOT >= 16384 ? 2 : 3;
-  static constexpr uint32_t kBudget = 106496;  // two CTAs per SM
-  static constexpr int NSA_FIT = (int)((kBudget - NSB * BSLOT) / ASLOT);
-  static constexpr int NSA = NSA_FIT < 2 ? 2 : NSA_FIT > 6 ? 6 : NSA_FIT;
+  static constexpr int NSB = 2;
+  static constexpr int NACC = NP > 16 ? 1 : 2;   // accumulators
+  static constexpr uint32_t kBudget = 112640;  // two CTAs per SM
+  static constexpr int NSA = (int)((kBudget - NSB * BSLOT) / ASLOT);
   static constexpr uint32_t OFF_B = NSA * ASLOT;
   static constexpr uint32_t OFF_BAR = OFF_B + NSB * BSLOT;
-  static constexpr int NBARS = 2 * NSA + 2 * NSB + 5;
+  static constexpr int NBARS = 3 * NSA + 2 * NSB + 5;
   static constexpr uint32_t SMEM = OFF_BAR + NBARS * 8 + 16 + 1024;  // + alignment slack
-  static constexpr uint32_t TCOLS = 2 * NMMA;  // two accumulators
-  static_assert(TCOLS == 128 || TCOLS == 256, "tensor-memory allocation");
+  static constexpr uint32_t TCOLS = 256;
+  static_assert(NACC * NMMA <= TCOLS && NMMA % 16 == 0, "tensor-memory allocation");
+  static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 };
 
-__device__ __forceinline__ void cp_async16s(uint32_t dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
-               "r"(src_bytes)
-               : "memory");
-}
-
-// The barrier's phase completes (for this thread's arrival) once every
-// cp.async this thread issued before has landed; the arrival is one of the
-// barrier's expected count.
-__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
+// Boxes of 32 words of 64, 32, 16 and 8 rows of the evaluations.
+struct GpMaps {
+  CUtensorMap box[4];
+};
 
 __device__ __forceinline__ uint32_t item_chunks(const WorkDev& w) {
   return (w.k1 - w.k0 + KCH - 1) / KCH;
 }
 
-// 64 registers: two CTAs of 13 warps put up to 8 warps on one SM sub-partition,
-// whose 16384 registers hold 8 warps of 64 (not of 72).
+// What the roles know of the K words kc .. + 31 of a tile: J live instances, in the rows
+// from `row` on (of 512 bytes) of the point's evaluations, words kc % 128 .. + 31 of each.
+struct Chunk {
+  uint32_t row, live;
+};
+__device__ __forceinline__ Chunk chunk_at(const uint4* __restrict__ xtiles, uint32_t x0,
+                                          uint32_t kc) {
+  const uint32_t w = xtiles[x0 + kc / KBLK].w;
+  return Chunk{x0 + (w >> 8), w & 0xFFu};
+}
+
 template <int NP>
-__global__ void __maxnreg__(64)
-    batch_pm_kernel(const WorkDev* __restrict__ work, unsigned nwork,
-                    const TileDev* __restrict__ tiles, const ItemDev* __restrict__ rows,
-                    const MatDev* __restrict__ mats, const uint32_t* __restrict__ s_pm,
-                    unsigned long long ps, unsigned long long* __restrict__ acc, int d,
-                    uint4 scale, uint4 scale_q, const TcConsts k, int* __restrict__ err) {
+__global__ void __launch_bounds__(kGpThreads, 2)
+    batch_pm_kernel(const __grid_constant__ GpMaps maps, const WorkDev* __restrict__ work,
+                    unsigned nwork, const TileDev* __restrict__ tiles,
+                    const ItemDev* __restrict__ rows, const MatDev* __restrict__ mats,
+                    const uint4* __restrict__ xtiles, unsigned long long* __restrict__ acc, int d,
+                    const FieldParams f, int* __restrict__ err) {
   using S = GpShape<NP>;
-  constexpr int NSA = S::NSA, NSB = S::NSB, NMMA = S::NMMA;
+  constexpr int NSA = S::NSA, NSB = S::NSB, NMMA = S::NMMA, NACC = S::NACC;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   const uint32_t raw = smem_addr(sm_raw);
   unsigned char* sm = sm_raw + (((raw + 1023u) & ~1023u) - raw);
   const uint32_t s0 = smem_addr(sm);
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + S::OFF_BAR);  // slot's copies landed
-  uint64_t* a_free = full + NSA;                                  // slot's MMAs done
+  uint64_t* zeroed = full + NSA;                                  // its dead rows are zero
+  uint64_t* a_free = zeroed + NSA;                                // slot's MMAs done
   uint64_t* built = a_free + NSA;                                 // B slot written
   uint64_t* b_free = built + NSB;                                 // B slot's MMAs done
   uint64_t* acc_full = b_free + NSB;                              // [2] item's MMAs done
@@ -125,7 +128,8 @@ __global__ void __maxnreg__(64)
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < NSA; ++i) {
-      mbar_init(&full[i], kGpLoaders);
+      mbar_init(&full[i], 1);
+      mbar_init(&zeroed[i], kGpZeroWarps);
       mbar_init(&a_free[i], 1);
     }
     for (int i = 0; i < NSB; ++i) {
@@ -145,89 +149,94 @@ __global__ void __maxnreg__(64)
   const uint32_t tbase = *taddr_slot;
   bool ok = true;
 
-  if (warp >= kGpLoadWarp0 && warp < kGpLoadWarp0 + kGpLoadWarps) {
-    // ------------------------------------------------------------ copies
-    // Loader warp lw owns instance rows 32 lw .. + 31 of the tile. Rows are
-    // sorted longest first, so the rows still inside their length at chunk k
-    // form a prefix; each slot remembers from which row on it already holds
-    // zeros for the current item.
-    const int lw = warp - kGpLoadWarp0;
-    uint32_t gc = 0;  // chunks of this CTA so far
-    uint32_t zeroed[NSA];
+  if (warp == kGpLoadWarp) {
+    // ------------------------------------------------------------ loads
+    if (lane == 0) {
+      uint32_t gc = 0;  // chunks of this CTA so far
+      for (unsigned wi = blockIdx.x; ok && wi < nwork; wi += gridDim.x) {
+        const WorkDev w = work[wi];
+        const uint32_t x0 = (uint32_t)(rows[tiles[w.tile].first].s_off / KBLK);
+        const uint32_t nch = item_chunks(w);
+        Chunk ch = chunk_at(xtiles, x0, w.k0);
+        for (uint32_t c = 0; c < nch; ++c, ++gc) {
+          const uint32_t sl = gc % NSA, kc = w.k0 + c * KCH;
+          if (c && kc % KBLK == 0) ch = chunk_at(xtiles, x0, kc);
+          if (gc >= (uint32_t)NSA && !(ok = mbar_wait(&a_free[sl], ((gc / NSA) - 1) & 1, err)))
+            break;
+          const uint32_t bar = smem_addr(&full[sl]);
+          const uint32_t nrows = (ch.live + 7) & ~7u;
+          mbar_arrive_expect_tx(&full[sl], nrows * 128);
+          uint32_t r = 0;
+          for (int b = 0; b < 4; ++b) {  // 64 rows (twice for more than 120), 32, 16, 8
+            const uint32_t box = 64u >> b;
+            while (nrows - r >= box) {
+              tma_load_3d(s0 + sl * S::ASLOT + r * 128, &maps.box[b], (int)(kc % KBLK),
+                          (int)(ch.row + r), (int)w.eg, bar);
+              r += box;
+            }
+          }
+        }
+      }
+      // nothing may still be writing shared memory at exit
+      for (uint32_t i = 0; i < (uint32_t)NSA; ++i) {
+        const uint32_t uses = gc > i ? (gc - i + NSA - 1) / NSA : 0;
+        if (uses) mbar_wait_sleep(&full[i], (uses - 1) & 1, err);
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kGpZeroWarp0 && warp < kGpZeroWarp0 + kGpZeroWarps) {
+    // ------------------------------------------------------------ dead rows
+    // A slot remembers from which row on it holds zeros for the current item; the
+    // rows up to there that a chunk does not fill with live instances are cleared.
+    const uint32_t half = warp - kGpZeroWarp0;
+    uint32_t gc = 0, from[NSA];
     for (unsigned wi = blockIdx.x; ok && wi < nwork; wi += gridDim.x) {
       const WorkDev w = work[wi];
       const TileDev tl = tiles[w.tile];
-      const MatDev mt = mats[tl.matrix];
-      const uint32_t* se = s_pm + (unsigned long long)w.eg * ps;
-      const uint32_t* ye = mt.evals_pm + (unsigned long long)w.eg * mt.rows * mt.ld_pm;
-      const uint32_t row0 = 32u * lw;
-      const uint32_t cw = tl.count > row0 ? min(tl.count - row0, 32u) : 0u;  // this warp's rows
-      // this lane's row: point-major column (a multiple of 128) and length
-      unsigned long long off = 0;
-      uint32_t len = 0;
-      if ((uint32_t)lane < cw) {
-        const ItemDev it = rows[tl.first + row0 + lane];
-        off = it.s_off;
-        len = it.n;
-      }
-#pragma unroll
-      for (int i = 0; i < NSA; ++i) zeroed[i] = 32;  // the slots' rows hold older data
+      const uint32_t x0 = (uint32_t)(rows[tl.first].s_off / KBLK);
       const uint32_t nch = item_chunks(w);
+#pragma unroll
+      for (int i = 0; i < NSA; ++i) from[i] = tl.count;  // the slots' rows hold older data
+      Chunk ch = chunk_at(xtiles, x0, w.k0);
       for (uint32_t c = 0; c < nch; ++c, ++gc) {
-        const uint32_t sl = gc % NSA;
-        if (gc >= (uint32_t)NSA && !(ok = lane0_wait(&a_free[sl], ((gc / NSA) - 1) & 1, lane, err)))
-          break;
-        const uint32_t kc = w.k0 + c * KCH;
-        const uint32_t sa = s0 + sl * S::ASLOT;
-        const uint32_t J = __popc(__ballot_sync(0xffffffffu, len > kc));  // live rows of this warp
-        uint32_t zeroed_sl = 0;
+        const uint32_t sl = gc % NSA, kc = w.k0 + c * KCH;
+        if (c && kc % KBLK == 0) ch = chunk_at(xtiles, x0, kc);
+        if (!(ok = lane0_wait(&full[sl], (gc / NSA) & 1, lane, err))) break;
+        uint32_t end = 0;
 #pragma unroll
-        for (int i = 0; i < NSA; ++i) zeroed_sl = i == (int)sl ? zeroed[i] : zeroed_sl;
-        const uint32_t zend = min(max(zeroed_sl, J), cw);
-        // eight lanes per row, 16 bytes each: rows [0, J) from the witness,
-        // [J, zend) as zero fill (four rows per instruction)
-        const uint32_t r = lane >> 3, q4 = lane & 7;
-#pragma unroll
-        for (int s8 = 0; s8 < 8; ++s8) {
-          const uint32_t jr = 4 * s8 + r;  // row within this warp's 32
-          const unsigned long long o = __shfl_sync(0xffffffffu, off, jr);
-          if (jr < zend) {
-            const bool live = jr < J;
-            cp_async16s(sa + sw128(row0 + jr, 0, q4, 0), live ? se + o + kc + 4 * q4 : se,
-                        live ? 16u : 0u);
+        for (int i = 0; i < NSA; ++i) {
+          if (i == (int)sl) {
+            end = from[i];
+            from[i] = ch.live;
           }
         }
-#pragma unroll
-        for (int i = 0; i < NSA; ++i)
-          if (i == (int)sl) zeroed[i] = min(J, cw);
-        // Y: rows x eight 16-byte pieces, spread over the loader warps
-        for (uint32_t u = lw * 32 + lane; u < mt.rows * 8; u += kGpLoaders) {
-          const uint32_t yr = u >> 3, yq = u & 7;
-          const uint32_t kw = kc + 4 * yq;
-          const bool valid = kw < mt.ld_pm;
-          cp_async16s(sa + S::XSLOT + sw128(yr, 0, yq, 0),
-                      valid ? ye + (unsigned long long)yr * mt.ld_pm + kw : ye, valid ? 16u : 0u);
+        end = min(max(end, (ch.live + 7) & ~7u), tl.count);  // the load's last box included
+        if (ch.live < end) {
+          unsigned char* slot = sm + sl * S::ASLOT;
+          for (uint32_t u = ch.live * 8 + half * 32 + lane; u < end * 8; u += 32 * kGpZeroWarps)
+            *reinterpret_cast<uint4*>(slot + u * 16) = make_uint4(0, 0, 0, 0);
+          fence_proxy_async_smem();
         }
-        cp_async_arrive_noinc(&full[sl]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&zeroed[sl]);
       }
     }
-    cp_async_wait_all();  // nothing may still be writing shared memory at exit
   } else if (warp == kGpMmaWarp) {
     // ------------------------------------------------------------ MMA issue
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_u8(128, NMMA);
       uint32_t gc = 0, it = 0;
       for (unsigned wi = blockIdx.x; ok && wi < nwork; wi += gridDim.x, ++it) {
-        const uint32_t buf = it & 1;
-        if (it >= 2 && !(ok = mbar_wait_sleep(&acc_empty[buf], ((it >> 1) - 1) & 1, err))) break;
+        const uint32_t buf = it % NACC;
+        if (it >= NACC && !(ok = mbar_wait_sleep(&acc_empty[buf], (it / NACC - 1) & 1, err))) break;
         tc::fence_after_sync();
         const uint32_t nch = item_chunks(work[wi]);
         for (uint32_t c = 0; c < nch; ++c, ++gc) {
           const uint32_t sl = gc % NSA, bs = gc % NSB;
           if (!(ok = mbar_wait(&full[sl], (gc / NSA) & 1, err)) ||
+              !(ok = mbar_wait(&zeroed[sl], (gc / NSA) & 1, err)) ||
               !(ok = mbar_wait(&built[bs], (gc / NSB) & 1, err)))
             break;
-          fence_proxy_async_smem();  // the copied rows, read by the tensor cores
           tc::fence_after_sync();
           const uint32_t sa = s0 + sl * S::ASLOT, sb = s0 + S::OFF_B + bs * S::BSLOT;
 #pragma unroll
@@ -252,38 +261,45 @@ __global__ void __maxnreg__(64)
     uint32_t gc = 0;
     for (unsigned wi = blockIdx.x; ok && wi < nwork; wi += gridDim.x) {
       const WorkDev w = work[wi];
-      const uint32_t mrows = mats[tiles[w.tile].matrix].rows;
+      const MatDev mt = mats[tiles[w.tile].matrix];
+      const uint32_t mrows = mt.rows;
+      const uint32_t* ye = mt.evals_pm +
+                           ((unsigned long long)w.eg * mrows + n_base) * mt.ld_pm;
       const uint32_t nch = item_chunks(w);
-      for (uint32_t c = 0; c < nch; ++c, ++gc) {
-        const uint32_t sl = gc % NSA, bs = gc % NSB;
-        ok = lane0_wait(&full[sl], (gc / NSA) & 1, lane, err);
-        if (ok && gc >= (uint32_t)NSB) ok = lane0_wait(&b_free[bs], ((gc / NSB) - 1) & 1, lane, err);
-        if (!ok) break;
-        const unsigned char* src = sm + sl * S::ASLOT + S::XSLOT;
-        unsigned char* bt = sm + S::OFF_B + bs * S::BSLOT;
-        uint32_t y[kWords];
+      uint32_t next[kWords];
+      auto load = [&](uint32_t c) {
+        const uint32_t kw = w.k0 + c * KCH + kk;
 #pragma unroll
         for (int i = 0; i < kWords; ++i) {
-          const int n = n_base + kGpBuildWarps * i;
-          y[i] = n < (int)mrows ? *reinterpret_cast<const uint32_t*>(
-                                      src + sw128(n, 0, kk >> 2, 0) + 4 * (kk & 3))
-                                : 0u;
+          const uint32_t n = n_base + kGpBuildWarps * i;
+          next[i] = c < nch && n < mrows && kw < mt.ld_pm
+                        ? __ldg(ye + (unsigned long long)(kGpBuildWarps * i) * mt.ld_pm + kw)
+                        : 0u;
         }
+      };
+      load(0);
+      for (uint32_t c = 0; c < nch; ++c, ++gc) {
+        const uint32_t bs = gc % NSB;
+        uint32_t y[kWords];
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) y[i] = next[i];
+        load(c + 1);
+        if (gc >= (uint32_t)NSB && !(ok = lane0_wait(&b_free[bs], ((gc / NSB) - 1) & 1, lane, err)))
+          break;
+        unsigned char* bt = sm + S::OFF_B + bs * S::BSLOT;
 #pragma unroll
         for (int i = 0; i < kWords; ++i) {
           const int n = n_base + kGpBuildWarps * i;
           if (n >= (int)mrows) continue;
-          const uint32_t v = y[i];
-          const uint32_t y1 = mont_c(v, scale.x, scale_q.x, k.q);  // 2^8 y
-          const uint32_t y2 = mont_c(v, scale.y, scale_q.y, k.q);  // 2^16 y
-          const uint32_t y3 = mont_c(v, scale.z, scale_q.z, k.q);  // 2^24 y
-          const uint32_t lo = __byte_perm(v, y1, 0x5140), hi = __byte_perm(y2, y3, 0x5140);
-          const uint32_t lo2 = __byte_perm(v, y1, 0x7362), hi2 = __byte_perm(y2, y3, 0x7362);
+          const uint32_t v = __byte_perm(y[i], 0, 0x0123);  // bytes 3, 2, 1, 0
           unsigned char* dst = bt + sw128(n, 0, kk >> 2, 0) + 4 * (kk & 3);
-          *reinterpret_cast<uint32_t*>(dst) = __byte_perm(lo, hi, 0x5410);
-          *reinterpret_cast<uint32_t*>(dst + NP * 128) = __byte_perm(lo, hi, 0x7632);
-          *reinterpret_cast<uint32_t*>(dst + 2 * NP * 128) = __byte_perm(lo2, hi2, 0x5410);
-          *reinterpret_cast<uint32_t*>(dst + 3 * NP * 128) = __byte_perm(lo2, hi2, 0x7632);
+          *reinterpret_cast<uint32_t*>(dst) = v >> 24;
+          *reinterpret_cast<uint32_t*>(dst + NP * 128) = v >> 16;
+          *reinterpret_cast<uint32_t*>(dst + 2 * NP * 128) = v >> 8;
+          *reinterpret_cast<uint32_t*>(dst + 3 * NP * 128) = v;
+          *reinterpret_cast<uint32_t*>(dst + 4 * NP * 128) = v << 8;
+          *reinterpret_cast<uint32_t*>(dst + 5 * NP * 128) = v << 16;
+          *reinterpret_cast<uint32_t*>(dst + 6 * NP * 128) = v << 24;
         }
         fence_proxy_async_smem();  // the planes are read by the tensor cores
         __syncwarp();
@@ -296,34 +312,32 @@ __global__ void __maxnreg__(64)
     const uint32_t j = 32 * quarter + lane;
     uint32_t it = 0;
     for (unsigned wi = blockIdx.x; ok && wi < nwork; wi += gridDim.x, ++it) {
-      const uint32_t buf = it & 1;
+      const uint32_t buf = it % NACC;
       const WorkDev w = work[wi];
       const TileDev tl = tiles[w.tile];
       const uint32_t mrows = mats[tl.matrix].rows;
       const unsigned long long toff = j < tl.count ? rows[tl.first + j].t_off : 0ull;
       // the item's whole K loop: sleep in the barrier rather than poll
       bool got = true;
-      if (lane == 0) got = mbar_wait_sleep(&acc_full[buf], (it >> 1) & 1, err);
+      if (lane == 0) got = mbar_wait_sleep(&acc_full[buf], (it / NACC) & 1, err);
       __syncwarp();
       if (!(ok = __shfl_sync(0xffffffffu, got, 0))) break;
       tc::fence_after_sync();
       const uint32_t taddr = tc::tmem_addr(tbase, 32 * quarter, buf * NMMA);
 #pragma unroll 1
-      for (int n0 = 0; n0 < NP; n0 += 8) {
-        uint32_t eb[4][8];
+      for (int n0 = 0; n0 < (int)mrows; n0 += 8) {
+        uint32_t ds[7][8];
 #pragma unroll
-        for (int l = 0; l < 4; ++l) tc::tmem_ld8(taddr + l * NP + n0, eb[l]);
-        tc::tmem_ld_wait32(eb);
+        for (int c = 0; c < 7; ++c) tc::tmem_ld8(taddr + c * NP + n0, ds[c]);
+        tc::tmem_ld_wait7(ds);
         if (j >= tl.count) continue;
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) {
           const uint32_t n = n0 + jj;
           if (n >= mrows) continue;
-          uint64_t v = mad_wide(eb[1][jj], 256u, (uint64_t)eb[0][jj]);
-          v = mad_wide(eb[2][jj], 65536u, v);
-          v = mad_wide(eb[3][jj], 16777216u, v);
           atomicAdd(&acc[(toff + n) * (unsigned long long)d + w.eg],
-                    (unsigned long long)redc64(v, k.q, k.qinv));
+                    (unsigned long long)reduce_classes(ds[0][jj], ds[1][jj], ds[2][jj], ds[3][jj],
+                                                       ds[4][jj], ds[5][jj], ds[6][jj], f));
         }
       }
       tc::fence_before_sync();
@@ -341,30 +355,34 @@ __global__ void __maxnreg__(64)
 
 template <int NP>
 int launch_np(const grid_gpu_plan* p, const WorkDev* work, unsigned nwork, const TileDev* tiles,
-              const ItemDev* items, const MatDev* mats, const uint32_t* s_pm, uint64_t ps,
-              unsigned long long* acc, cudaStream_t s) {
+              const ItemDev* items, const MatDev* mats, const uint4* xtiles,
+              const uint32_t* s_pm, uint64_t ps, unsigned long long* acc, cudaStream_t s) {
   using S = GpShape<NP>;
   static int bps_cache[kMaxDevices] = {};
   int bps = 0;
   const int rc = prepare_kernel(batch_pm_kernel<NP>, S::SMEM, kGpThreads, p->device, bps_cache,
                                 &bps, true);
   if (rc) return rc;
-  // 2^(8i) R mod q (a Montgomery product with it is 2^(8i) y mod q) and the
-  // Shoup companions c qinv mod 2^32
-  uint32_t c[3], cq[3];
-  for (int i = 1; i <= 3; ++i) {
-    c[i - 1] = (uint32_t)(((unsigned __int128)1 << (32 + 8 * i)) % p->f.q);
-    cq[i - 1] = c[i - 1] * p->f.qinv;
+  // the evaluations as [point][ps / 128 rows][128 words]
+  EncodeTiled enc = encoder();
+  if (!enc) return GRID_ERR_CUDA;
+  GpMaps maps;
+  for (int b = 0; b < 4; ++b) {
+    const cuuint64_t dims[3] = {KBLK, ps / KBLK, p->d};
+    const cuuint64_t strides[2] = {KBLK * 4, ps * 4};
+    const cuuint32_t box[3] = {KCH, 64u >> b, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    if (enc(&maps.box[b], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint32_t*>(s_pm), dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return GRID_ERR_CUDA;
   }
-  TcConsts k;
-  k.q = p->f.q;
-  k.qinv = p->f.qinv;
-  // Two CTAs per SM (GpShape, 64 registers). The occupancy query answers 1 for any kernel
+  // Two CTAs per SM (GpShape, at most 80 registers). The occupancy query answers 1 for any kernel
   // that allocates tensor memory, whatever its registers and shared memory.
   const unsigned grid = std::min<unsigned>(nwork, 2u * (unsigned)p->num_sms);
   batch_pm_kernel<NP><<<grid, kGpThreads, S::SMEM, s>>>(
-      work, nwork, tiles, items, mats, s_pm, (unsigned long long)ps, acc, (int)p->d,
-      make_uint4(c[0], c[1], c[2], 0), make_uint4(cq[0], cq[1], cq[2], 0), k, p->d_err);
+      maps, work, nwork, tiles, items, mats, xtiles, acc, (int)p->d,
+      p->f, p->d_err);
   return cuda_status(cudaGetLastError());
 }
 
@@ -372,11 +390,11 @@ int launch_np(const grid_gpu_plan* p, const WorkDev* work, unsigned nwork, const
 
 int launch_batch_pm(const grid_gpu_plan* p, int cls, const WorkDev* work, unsigned nwork,
                     const TileDev* tiles, const ItemDev* items, const MatDev* mats,
-                    const uint32_t* s_pm, uint64_t ps, unsigned long long* acc, cudaStream_t s) {
+                    const uint4* xtiles, const uint32_t* s_pm, uint64_t ps, unsigned long long* acc, cudaStream_t s) {
   if (nwork == 0) return GRID_OK;
   switch (cls) {
-    case TC_D16: return launch_np<16>(p, work, nwork, tiles, items, mats, s_pm, ps, acc, s);
-    case TC_D32: return launch_np<32>(p, work, nwork, tiles, items, mats, s_pm, ps, acc, s);
+    case TC_D16: return launch_np<16>(p, work, nwork, tiles, items, mats, xtiles, s_pm, ps, acc, s);
+    case TC_D32: return launch_np<32>(p, work, nwork, tiles, items, mats, xtiles, s_pm, ps, acc, s);
     default: return GRID_ERR_INVALID_PARAMETERS;  // point-major tiles are dense commitments
   }
 }

@@ -192,6 +192,59 @@ def planes_roles(n, nsx, nsp):
     return counts, [loader(), mma()] + [builder() for _ in range(3)]
 
 
+def grouped_roles(items, nsa, nsb, nacc):
+    """batch_pm_kernel over one CTA's items (chunks each): loader, dead rows, builders, MMA,
+    epilogue. A slot's rows are the loaded ones (a) and the cleared ones (z)."""
+    chunks = [(it, c) for it, n in enumerate(items) for c in range(n)]
+
+    def loader():
+        for g in range(len(chunks)):
+            s = g % nsa
+            if g >= nsa:
+                yield ("wait", f"AFREE{s}", g // nsa - 1)
+            yield ("async", f"FULL{s}", (f"a{s}", "w", g))
+
+    def zero(h):
+        for g in range(len(chunks)):
+            s = g % nsa
+            yield ("wait", f"FULL{s}", g // nsa)
+            yield ("touch", f"a{s}", "r", g)
+            yield ("touch", f"z{h}{s}", "w", g)
+            yield ("arrive", f"ZEROED{s}")
+
+    def builder(h):
+        for g in range(len(chunks)):
+            p = g % nsb
+            if g >= nsb:
+                yield ("wait", f"BFREE{p}", g // nsb - 1)
+            yield ("touch", f"b{h}{p}", "w", g)
+            yield ("arrive", f"BUILT{p}")
+
+    def mma():
+        for g, (it, c) in enumerate(chunks):
+            s, p, acc = g % nsa, g % nsb, it % nacc
+            if c == 0 and it >= nacc:
+                yield ("wait", f"AEMPTY{acc}", it // nacc - 1)
+            yield ("wait", f"FULL{s}", g // nsa)
+            yield ("wait", f"ZEROED{s}", g // nsa)
+            yield ("wait", f"BUILT{p}", g // nsb)
+            yield ("async", f"AFREE{s}", (f"a{s}", "r", g), (f"z0{s}", "r", g), (f"z1{s}", "r", g))
+            yield ("async", f"BFREE{p}", (f"b0{p}", "r", g), (f"b1{p}", "r", g))
+            if c == items[it] - 1:
+                yield ("async", f"ACC{acc}", (f"acc{acc}", "w", it))
+
+    def epilogue():
+        for it in range(len(items)):
+            acc = it % nacc
+            yield ("wait", f"ACC{acc}", it // nacc)
+            yield ("touch", f"acc{acc}", "r", it)
+            yield ("arrive", f"AEMPTY{acc}")
+
+    counts = {f"{b}{i}": 2 for b in ("ZEROED", "BUILT", "AEMPTY") for i in range(nsa)}
+    return counts, ([loader(), mma()] + [zero(h) for h in (0, 1)] + [builder(h) for h in (0, 1)]
+                    + [epilogue() for _ in (0, 1)])
+
+
 def unit_roles(n, warps=4, group=2):
     """The JL kernels' hand-over: groups of warps share a barrier pair; n units go round
     the warps, a warp without a last unit arrives for its group."""
@@ -237,6 +290,15 @@ def test_protocol(n, kind):
             counts, roles = unit_roles(n)
         else:
             counts, roles = planes_roles(n, int(kind[-2]), int(kind[-1]))
+        Model(counts, rng).run(roles)
+
+
+@pytest.mark.parametrize("nsa,nsb,nacc", [(5, 2, 2), (3, 2, 1)])
+def test_grouped_protocol(nsa, nsb, nacc):
+    rng = random.Random(nsa)
+    for _ in range(300):
+        items = [rng.randint(1, 7) for _ in range(rng.randint(1, 5))]
+        counts, roles = grouped_roles(items, nsa, nsb, nacc)
         Model(counts, rng).run(roles)
 
 
