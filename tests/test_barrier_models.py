@@ -64,15 +64,15 @@ WARPS = 2  # per group: enough for the arrival counts to matter
 def transform_roles(n, nbuf=4):
     """ntt_tc_kernel: four tile buffers, two column sets."""
     def loader():
-        for t in range(n + nbuf):
-            b = t % nbuf
-            if t >= nbuf:
-                if t - nbuf >= n:
-                    return
-                yield ("wait", f"STAGED{b}", t // nbuf - 1)
-                yield ("touch", f"buf{b}", "r", ("result", t - nbuf))
-            if t < n:
-                yield ("async", f"AFULL{b}", (f"buf{b}", "w", ("input", t)))
+        for j in range(min(n, nbuf)):
+            yield ("async", f"AFULL{j}", (f"buf{j}", "w", ("input", j)))
+        for j in range(n):
+            yield ("wait", f"STAGED{j % nbuf}", j // nbuf)
+            if j >= 1:  # the store before this one has read its buffer
+                yield ("touch", f"buf{(j - 1) % nbuf}", "r", ("result", j - 1))
+                if j - 1 + nbuf < n:
+                    b = (j - 1) % nbuf
+                    yield ("async", f"AFULL{b}", (f"buf{b}", "w", ("input", j - 1 + nbuf)))
 
     def mma():
         for j in range(n):
