@@ -680,6 +680,7 @@ int grid_gpu_amortize_dev(const grid_gpu_plan* p, const uint32_t* S, const uint3
   uint32_t* c_hat = cv.take<uint32_t>(r * p->d);
   if (!is_crt(p)) {
     if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+    if (amortize_tc_fits(p, r, n)) return launch_amortize_tc(p, S, c, r, n, z, s_hat, st);
     int rc = launch_ntt(p, MODE_FWD, S, nullptr, s_hat, r * n, st);
     if (!rc) rc = launch_ntt(p, MODE_FWD, c, nullptr, c_hat, r, st);
     if (!rc) rc = launch_amortize(p, c_hat, s_hat, (int)r, n, z, st);
@@ -694,6 +695,10 @@ int grid_gpu_amortize_dev(const grid_gpu_plan* p, const uint32_t* S, const uint3
   int rc = GRID_OK;
   for (int j = 0; j < 3 && !rc; ++j) {
     const grid_gpu_plan* q = p->crt[j];
+    if (amortize_tc_fits(q, r, n)) {
+      rc = launch_amortize_tc(q, S, c, r, n, zj[j], s_hat, st);
+      continue;
+    }
     rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, st);
     if (!rc) rc = launch_ntt(q, MODE_FWD, c, nullptr, c_hat, r, st);
     if (!rc) rc = launch_amortize(q, c_hat, s_hat, (int)r, n, zj[j], st);

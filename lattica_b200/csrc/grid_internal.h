@@ -215,6 +215,10 @@ int launch_symmetrize_half(const grid_gpu_plan* p, const uint32_t* C, int r, uin
                            cudaStream_t s);
 int launch_amortize(const grid_gpu_plan* p, const uint32_t* c_hat, const uint32_t* s_hat, int r,
                     size_t n, uint32_t* z_hat, cudaStream_t s);
+// amortize_tc.cu: z = sum_i c_i s_i from coefficients, no transform (d = 64).
+bool amortize_tc_fits(const grid_gpu_plan* p, size_t r, size_t n);
+int launch_amortize_tc(const grid_gpu_plan* p, const uint32_t* S, const uint32_t* c, size_t r,
+                       size_t n, uint32_t* z, uint32_t* part, cudaStream_t s);
 int launch_add(const grid_gpu_plan* p, uint32_t* dst, const uint32_t* rhs, size_t words,
                cudaStream_t s);
 
