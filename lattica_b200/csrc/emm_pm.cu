@@ -8,12 +8,18 @@
 //
 // Byte planes, without scaling. With x = sum_i 2^(8i) x_i and y = sum_l 2^(8l) y_l in
 // bytes, sum_k x_k y_k = sum_s 2^(8s) D_s, D_s = sum_{i+l=s} sum_k x_i y_l, s = 0 .. 6.
-// A_i (128 rows x 128 K bytes per chunk) holds byte i of the X words, the four B_l
+// A_i (rows x 128 K bytes per chunk) holds byte i of the X words, the four B_l
 // stand one above the other (row l NP + n), so that the product of A_i with all of B is
-// added to tensor-memory columns i NP .. (i + 4) NP: class s at columns s NP, four
-// MMAs (N = 4 NP) per 32 K words, the same multiply-adds as with four planes of
-// 2^(8i) y mod q. D_s < 4 K 255^2 < 2^31 for K <= 8192 per CTA. V = sum_s 2^(8s) D_s <
-// 2^80 is reduced once.
+// added to tensor-memory columns i NP .. (i + 4) NP: class s at columns s NP.
+// The planes A_i stand one above the other too: of 33 to 64 rows, P = 2 of them fit the
+// 128 rows of one MMA (N = 4 NP), 4 / P MMAs per 32 K words. Rows g ROWS_A + m of
+// the product with planes i .. i + P - 1 hold byte i + g, so class s of those rows is at
+// columns (s - g) NP, and the row blocks' reduced sums, block g's times 2^(8g), are added
+// at the end. D_s < 4 K 255^2 < 2^31 for K <= 8192 per CTA. V = sum_s 2^(8s) D_s <
+// 2^80 is reduced once per block. (64 x 64 rows, n = 2048, garbage h and z together:
+// 87.4 us with one plane per MMA, 83.7 with two. Of up to 32 rows four would fit, but the
+// MMAs are short there and four blocks to reduce cost more: the Gram of r = 30, n = 1021
+// 20.9 us with one, 22.8 with four.)
 // Planes of 2^(8i) y cost three Montgomery products a word of Y, on eight warps that
 // bounded the kernel (about 1500 cycles per 32 K words of a 64-row Gram, MMAs 504); the
 // planes are now a 4 x 4 byte transpose of four consecutive words (two byte permutes and
@@ -29,7 +35,7 @@
 //    a ring of raw slots (zero fill past K), refilling a slot once it is transposed;
 //  * warps 0-7 write the chunk's planes into a ring of plane slots, once the rows
 //    landed and the slot's previous MMAs are done;
-//  * warp 9 (one lane) issues 16 MMAs (M 128, N 4 NP, K 32) per chunk into tensor
+//  * warp 9 (one lane) issues 16 / P MMAs (M 128, N 4 NP, K 32) per chunk into tensor
 //    memory, cleared beforehand, and commits them to the plane slot's mbarrier;
 //  * after the last chunk warps 0-7 combine the classes, reduce, stage the
 //    point's results in shared memory and store them contiguously, [split][e]
@@ -63,6 +69,8 @@ template <int NP, int MX, bool UPPER>
 struct PmShape {
   static constexpr int NMMA = 4 * NP;                         // B rows: four byte planes
   static constexpr int ROWS_A = UPPER ? NP : MX;
+  static constexpr int P = ROWS_A > 64 || ROWS_A <= 32 ? 1 : 2;  // planes per MMA
+  static constexpr int NC = 8 - P;                            // blocks of NP columns
   static constexpr uint32_t XRAW = ROWS_A * KCH * 4u;
   static constexpr uint32_t RAW = XRAW + (UPPER ? 0u : NP * KCH * 4u);  // X rows, Y rows
   static constexpr uint32_t PLANES_A = 4u * ROWS_A * KCH;
@@ -81,13 +89,14 @@ struct PmShape {
   static constexpr uint32_t OFF_RAW = NSP * PLANES;           // planes first, then raw rows
   static constexpr uint32_t OFF_BAR = OFF_RAW + NSX * RAW;
   static constexpr int NBARS = 2 * NSX + 2 * NSP + 1;
-  // the MMA reads 128 rows from every A plane: the last plane's run past its slot
+  // the MMA reads 128 rows from its first A plane: the last one's run past its slot
   static constexpr uint32_t END = OFF_BAR + NBARS * 8 + 16;
-  static constexpr uint32_t A_END = OFF_RAW - PLANES + (3u * ROWS_A + 128u) * 128u;
+  static constexpr uint32_t A_END = OFF_RAW - PLANES + ((4u - P) * ROWS_A + 128u) * 128u;
   static constexpr uint32_t SMEM = (END > A_END ? END : A_END) + 1024;  // + alignment slack
   static_assert(SMEM <= 232448, "shared memory budget");
   // the point's results are staged in the first plane slot
-  static_assert(PLANES >= (UPPER ? (uint32_t)NP * (NP + 1) / 2 : (uint32_t)MX * NP) * 4, "staging");
+  static_assert(PLANES >= P * (UPPER ? (uint32_t)NP * (NP + 1) / 2 : (uint32_t)MX * NP) * 4,
+                "staging");
 };
 
 // The builder warps' own barrier (named barrier 1; the CTA's is 0).
@@ -116,7 +125,7 @@ __global__ void __launch_bounds__(kPmThreads)
                   int N, int K, int k_per_split, uint32_t box_bytes, const FieldParams f,
                   int* __restrict__ err) {
   using S = PmShape<NP, MX, UPPER>;
-  constexpr int NSX = S::NSX, NSP = S::NSP, NMMA = S::NMMA;
+  constexpr int NSX = S::NSX, NSP = S::NSP, NMMA = S::NMMA, P = S::P;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   const uint32_t raw = smem_addr(sm_raw);
   unsigned char* sm = sm_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -155,7 +164,7 @@ __global__ void __launch_bounds__(kPmThreads)
   const uint32_t tbase = *taddr_slot;
   if (warp < 4) {  // the classes start at zero: MMAs of different A_i share them
 #pragma unroll
-    for (int c = 0; c < 7 * NP; c += 16) tc::tmem_zero16(tc::tmem_addr(tbase, 32 * warp, c));
+    for (int c = 0; c < S::NC * NP; c += 16) tc::tmem_zero16(tc::tmem_addr(tbase, 32 * warp, c));
     tc::tmem_st_wait();
   }
   tc::fence_before_sync();
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(kPmThreads)
         for (int ks = 0; ks < 4; ++ks) {
           if (ks >= steps) break;
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < 4; i += P)
             tc::mma_u8(tbase + i * NP, tc::desc_plus(da, i * S::ROWS_A * 128 + 32 * ks),
                        tc::desc_plus(db, 32 * ks), idesc, 1u);
         }
@@ -241,32 +250,38 @@ __global__ void __launch_bounds__(kPmThreads)
     // every builder reaches the barrier below (a failed wait skips only work)
     const int outputs = UPPER ? M * (M + 1) / 2 : M * N;
     uint32_t* stage = reinterpret_cast<uint32_t*>(sm);  // the planes: MMAs are done
-    const int m = 32 * (warp & 3) + lane;
-    if (ok && 32 * (warp & 3) < M) {
-      // warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (rows m) and
+    const int block = (32 * (warp & 3) + lane) / S::ROWS_A;
+    const int m = (32 * (warp & 3) + lane) % S::ROWS_A;
+    if (ok && 32 * (warp & 3) < P * S::ROWS_A) {
+      // warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (rows m of a block) and
       // column groups of 8 starting at 8 (w / 4)
       const uint32_t taddr = tc::tmem_addr(tbase, 32 * (warp & 3), 0);
 #pragma unroll 1
       for (int n0 = 8 * (warp >> 2); n0 < N; n0 += 8 * (kPmBuildWarps / 4)) {
-        uint32_t ds[7][8];
+        uint32_t ds[7][8] = {};
 #pragma unroll
-        for (int l = 0; l < 7; ++l) tc::tmem_ld8(taddr + l * NP + n0, ds[l]);
+        for (int c = 0; c < S::NC; ++c) tc::tmem_ld8(taddr + c * NP + n0, ds[c]);
         tc::tmem_ld_wait7(ds);
-        if (m >= M) continue;
+        if (m >= M || block >= P) continue;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int n = n0 + j;
           if (n >= N || (UPPER && n < m)) continue;
           const int idx = UPPER ? m * M - (m * (m - 1)) / 2 + (n - m) : m * N + n;
-          stage[idx] = reduce_classes(ds[0][j], ds[1][j], ds[2][j], ds[3][j], ds[4][j], ds[5][j],
-                                      ds[6][j], f);
+          stage[block * outputs + idx] = reduce_classes(ds[0][j], ds[1][j], ds[2][j], ds[3][j],
+                                                        ds[4][j], ds[5][j], ds[6][j], f, block);
         }
       }
     }
     builders_sync();
     if (ok) {
       uint32_t* o = part + ((size_t)blockIdx.y * gridDim.x + e) * outputs;
-      for (int i = threadIdx.x; i < outputs; i += kPmBuilders) o[i] = stage[i];
+      for (int i = threadIdx.x; i < outputs; i += kPmBuilders) {
+        uint32_t v = stage[i];
+#pragma unroll
+        for (int g = 1; g < P; ++g) v = add_mod(v, stage[g * outputs + i], f.q);
+        o[i] = v;
+      }
     }
   }
   tc::fence_before_sync();

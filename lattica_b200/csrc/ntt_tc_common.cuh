@@ -134,16 +134,19 @@ __device__ __forceinline__ void reduce16(uint32_t taddr, const TcConsts& k, uint
   reduce16(taddr, k, out, [] {});
 }
 
-// (sum_s 2^(8s) d_s) * 2^-32 mod q for the seven byte classes of a sum of word
-// products (each below 2^32, the sum below 2^80), canonical.
+// (sum_s 2^(8s) d_s) 2^(8 shift) 2^-32 mod q for the seven byte classes of a sum of word
+// products (each below 2^32, the shifted sum below 2^80), canonical; shift < 4.
 __device__ __forceinline__ uint32_t reduce_classes(uint32_t d0, uint32_t d1, uint32_t d2,
                                                    uint32_t d3, uint32_t d4, uint32_t d5,
-                                                   uint32_t d6, const FieldParams& f) {
+                                                   uint32_t d6, const FieldParams& f,
+                                                   int shift = 0) {
   const uint64_t lo = mad_wide(d3, 16777216u, mad_wide(d2, 65536u, mad_wide(d1, 256u, d0)));
   const uint64_t hi = mad_wide(d6, 65536u, mad_wide(d5, 256u, d4));
   const uint64_t mid = (lo >> 32) + (uint32_t)hi;
-  return acc96_reduce(Acc96{(uint32_t)lo, (uint32_t)mid, (uint32_t)(hi >> 32) + (uint32_t)(mid >> 32)},
-                      f);
+  const uint32_t w0 = (uint32_t)lo, w1 = (uint32_t)mid;
+  const uint32_t w2 = (uint32_t)(hi >> 32) + (uint32_t)(mid >> 32);
+  return acc96_reduce(Acc96{w0 << (8 * shift), __funnelshift_l(w0, w1, 8 * shift),
+                            __funnelshift_l(w1, w2, 8 * shift)}, f);
 }
 
 // One transform of a 128-row tile (A at `a`, B at `w`) into 256 columns.
