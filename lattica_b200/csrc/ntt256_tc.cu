@@ -6,34 +6,41 @@
 // negacyclic product over TwistedNttPlan (algebra/src/poly/ntt.rs:75-126,
 // forward slot j = x(psi^(2j+1)), inverse with d^-1), bit-exact.
 //
-// Split 256 = 4 x 64. With coefficient n = 64 a + b and slot j = 4 j2 + j1
-// (a, j1 < 4; b, j2 < 64), psi a primitive 512th root, zeta = psi^64 and
-// omega = psi^8:
-//   X_{4 j2 + j1} = sum_b omega^(j2 b) Y_{j1}[b],
-//   Y_{j1}[b]     = psi^((2 j1 + 1) b) sum_a zeta^(a (2 j1 + 1)) x_{64 a + b}.
-// The 4-point step and the twist run on CUDA cores; the four 64-point cyclic
-// transforms of a polynomial are four rows of one tensor-core product against
-// the single matrix omega^(j2 b), by the byte-plane method of the d = 64
-// kernel (ntt_tc_common.cuh). The inverse mirrors it:
-//   V_{j1}[b] = sum_j2 omega^(-j2 b) Z_{4 j2 + j1}
-// is the same matrix read at output column j' = -b mod 64, and
-//   out_{64 a + b} = sum_j1 zeta^(-a (2 j1 + 1)) 256^-1 psi^(-(2 j1 + 1) b) V_{j1}[b].
-// One matrix in shared memory serves both directions, which leaves room for
-// two input buffers and a staged tile of b.
+// Split 256 = 64 x 4. With coefficient n = 4 b + a and slot j = j2 + 64 j1 (b, j2 < 64;
+// a, j1 < 4), psi a primitive 512th root, w = psi^(2 j2 + 1) and i = psi^128, i^2 = -1:
+//   X_{j2 + 64 j1} = sum_a i^(j1 a) w^(a - 2) N_a[j2],
+//   N_a[j2]        = sum_b psi^(2 (2 j2 + 1)(2 b + 1)) x_{4 b + a}.
+// N_a is a 64-point transform of every fourth coefficient as it stands, so the four of a
+// polynomial are four rows of one tensor-core product by the byte-plane method of the
+// d = 64 kernel (ntt_tc_common.cuh), and everything of four points and the twists is
+// done between the two products, by one thread for the four slots of a j2, with the
+// product by b: 8 modular products and 16 additions for 4 words (14 and 19 with 4-point
+// steps and twists before the forward and after the inverse product, and another pass
+// through shared memory). The inverse mirrors it:
+//   out_{4 b + a} = sum_j2 psi^(-2 (2 j2 + 1)(2 b + 1)) 256^-1 w^(2 - a) u_a[j2],
+//   u_a[j2]       = sum_j1 i^(-j1 a) Z_{j2 + 64 j1}.
+// The matrix psi^(2 (2 j + 1)(2 k + 1)) is symmetric and changes its sign under inversion
+// with j reversed (psi^256 = -1), so one matrix in shared memory serves both directions,
+// the inverse's operand in reverse order of j2; it holds i / 16 times that, whose square
+// is the factor -1 / 256.
 //
-// A tile is 32 polynomials = 128 rows (row 32 j1 + p), so epilogue warp w
-// (tensor-memory lanes 32 (w % 4) ..) holds block j1 = w % 4 of every
-// polynomial. Per tile j of a CTA (one persistent CTA per SM):
-//   loader (warp 17): bulk-loads input tile j into buffer j % 2 once output
-//     tile j - 2 has been stored from it, and b's tile j into padded rows once
-//     F(j-1) has read the previous one; L2 prefetch of a and b 3 tiles ahead
-//   epilogue (warps 0-15): P(j) 4-point + twist -> forward A operand;
-//     E(j-1) inverse results -> 4-point inverse in buffer (j-1) % 2 -> staged;
-//     F(j) forward results (x) b -> inverse A operand
-//   MMA (warp 16): fwd(j) after P(j) and F(j-1) read columns 0-255;
-//     inv(j) after F(j) and E(j-1) read columns 256-511.
-// The epilogue warps agree on every wait's outcome through a named barrier,
-// so a timed-out wait ends all of them together; every wait is bounded.
+// A tile is 32 polynomials = 128 rows (row 32 a + p, tensor-memory lane the same). One
+// persistent CTA per SM; its tiles go to two groups of eight warps in turn, each with an A
+// operand, a buffer X and 256 tensor-memory columns of its own, so that one computes while
+// the other waits for its MMAs, its exchanges or its loads:
+//   loader (warp 18): bulk-loads tile j into X[j % 2] once F(j-2) has read its exchange
+//     there, and b's tile j once F(j-1) has read the previous one; L2 prefetch of a and b
+//   group (warps 8 (j % 2) .. + 7): P(j) every fourth word -> A; F(j) forward results,
+//     exchanged through X, 4-point steps, twists and (x) b -> A; E(j) inverse
+//     results, exchanged through A, to global memory
+//   MMA (warp 16 + j % 2): fwd(j) after P(j), inv(j) after F(j), into the same columns.
+// A wait that timed out ends a role's waits, not its steps, so the others still meet it at
+// their barriers; every wait is bounded.
+// Bound: instruction issue and the integer pipes (0.62 and 0.5 of their cycles), then the
+// waits of two groups that overlap only each other. 2^20 polynomials: 1.20 ms with sixteen
+// warps in step (0.47 of the issue slots), with the 4-point steps outside the products or,
+// a fifth fewer instructions, between them; 1.10 with two groups; 1.08 with the MMA and
+// loader lanes asleep in their waits rather than polling.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -52,62 +59,51 @@ using namespace tcx;
 
 constexpr int D = 256;
 constexpr int PT = ROWS / 4;                // polys per tile
-constexpr int EPI_THREADS = EPI_WARPS * 32;
-constexpr int NX = 2;                       // natural-order tile buffers
+constexpr int GROUP_WARPS = 8, GROUP = GROUP_WARPS * 32;
+constexpr int MMA0 = 2 * GROUP_WARPS, LOADER = MMA0 + 2;
+constexpr int THREADS256 = (LOADER + 1) * 32;
 constexpr uint32_t XT = PT * D * 4;         // 32 KB
-// b rows padded to 260 words: the 32 rows of one gather start 4 banks apart
-constexpr uint32_t BROW = (D + 4) * 4;
+static_assert(XT == TILE, "a tile of words and its operand have the same size");
 
 // Offsets from the 1 KB-aligned base of dynamic shared memory.
 constexpr uint32_t OFF_W = 0;               // the 64-point matrix (B of both transforms)
-constexpr uint32_t OFF_AF = OFF_W + WMAT;   // forward A operand
-constexpr uint32_t OFF_AI = OFF_AF + TILE;  // inverse A operand (pointwise products)
-constexpr uint32_t OFF_X = OFF_AI + TILE;   // input tiles, then inverse results
-constexpr uint32_t OFF_B = OFF_X + NX * XT;  // b's tile, padded rows
-constexpr uint32_t OFF_BAR = OFF_B + PT * BROW;
+constexpr uint32_t OFF_A = OFF_W + WMAT;    // [2] A operand, then E's exchange
+constexpr uint32_t OFF_X = OFF_A + 2 * TILE;  // [2] input tile, then F's exchange
+constexpr uint32_t OFF_B = OFF_X + 2 * XT;  // b's tile
+constexpr uint32_t OFF_BAR = OFF_B + XT;
 constexpr uint32_t OFF_TADDR = OFF_BAR + 16 * 8;
 constexpr uint32_t SMEM_BYTES = OFF_TADDR + 16 + 1024;  // + alignment slack
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
 // Device table: the matrix image (WMAT bytes), then {w, w q^-1 mod 2^32}
-// Montgomery constants: forward twists psi^((2 j1 + 1) b) [4][64], inverse
-// twists 256^-1 psi^(-(2 j1 + 1) b) [4][64], and zeta^2, zeta, zeta^3,
-// zeta^-1, zeta^-2, zeta^-3.
-constexpr uint32_t TW_F = WMAT / 8;  // in uint2 units
-constexpr uint32_t TW_I = TW_F + 256;
-constexpr uint32_t TW_C = TW_I + 256;
-constexpr size_t TABLE_BYTES = WMAT + (256 + 256 + 8) * 8;
+// Montgomery constants: w^-2, w^-1, w, w^2 of every j2 [4][64], and i.
+constexpr uint32_t TW_W = WMAT / 8;  // in uint2 units
+constexpr uint32_t TW_I = TW_W + 256;
+constexpr size_t TABLE_BYTES = WMAT + (256 + 1) * 8 + 8;
 
+// Barriers, one of each per group.
 enum Bar : int {
-  AFULL0 = 0,               // input tile landed in buffer i
-  STAGED0 = AFULL0 + NX,    // output tile written into buffer i
-  BFULL = STAGED0 + NX,     // b's tile landed
-  BFREE,                    // F has read b's tile
-  PREP, FDONE, FREAD, PREADY, IDONE, EREAD, NBARS
+  AFULL = 0,          // input tile landed
+  XFREE = 2,          // X read for the last time
+  BFULL = 4,          // b's tile landed
+  BFREE = 6,          // F has read b's tile
+  PREP = 8,           // forward operand written
+  FDONE = 10,
+  PREADY = 12,        // inverse operand written
+  IDONE = 14,
+  NBARS = 16
 };
-static_assert(NBARS <= 16, "barrier slots");
 
-// All epilogue warps: true iff every one of them passes ok (named barrier 1).
-__device__ __forceinline__ bool epi_all(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.and.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)ok), "n"(EPI_THREADS)
-      : "memory");
-  return r != 0;
-}
-
-__device__ __forceinline__ void epi_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
+// The warps of a group (named barrier 1 or 2).
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GROUP) : "memory");
 }
 
 __device__ __forceinline__ uint32_t mulc(uint32_t x, uint2 w, uint32_t q) {
   return mont_c(x, w.x, w.y, q);
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS256, 1)
     ntt256_tc_mulinv_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
                             uint32_t* out, unsigned long long npolys,
                             const unsigned char* __restrict__ table, const TcConsts k,
@@ -124,24 +120,17 @@ __global__ void __launch_bounds__(THREADS, 1)
   {
     const uint4* src = reinterpret_cast<const uint4*>(table);
     uint4* w = reinterpret_cast<uint4*>(sm + OFF_W);
-    for (int i = threadIdx.x; i < (int)(WMAT / 16); i += THREADS) w[i] = src[i];
+    for (int i = threadIdx.x; i < (int)(WMAT / 16); i += THREADS256) w[i] = src[i];
   }
-  if (warp == MMA_WARP) {
+  if (warp == MMA0) {
     tc::tmem_alloc(taddr_slot, 512);
     tc::tmem_relinquish();
     if (lane == 0) {
-      for (int i = 0; i < NX; ++i) {
-        mbar_init(&bars[AFULL0 + i], 1);
-        mbar_init(&bars[STAGED0 + i], EPI_WARPS);
-      }
-      mbar_init(&bars[BFULL], 1);
-      mbar_init(&bars[BFREE], EPI_WARPS);
-      mbar_init(&bars[PREP], EPI_WARPS);
-      mbar_init(&bars[FDONE], 1);
-      mbar_init(&bars[FREAD], EPI_WARPS);
-      mbar_init(&bars[PREADY], EPI_WARPS);
-      mbar_init(&bars[IDONE], 1);
-      mbar_init(&bars[EREAD], EPI_WARPS);
+      for (int i = 0; i < NBARS; ++i)
+        mbar_init(&bars[i], (i & ~1) == XFREE || (i & ~1) == BFREE || (i & ~1) == PREP ||
+                                    (i & ~1) == PREADY
+                                ? GROUP_WARPS
+                                : 1);
       fence_mbar_init();
     }
   }
@@ -150,7 +139,6 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *taddr_slot;
-  const uint32_t R0 = tbase, R1 = tbase + 256;
 
   const unsigned long long ntiles = (npolys + PT - 1) / PT;
   const uint32_t n = blockIdx.x < ntiles
@@ -164,227 +152,173 @@ __global__ void __launch_bounds__(THREADS, 1)
     return (uint32_t)(left < PT ? left : PT) * D * 4;
   };
 
-  if (warp == LOAD_WARP) {
+  if (warp == LOADER) {
     // ------------------------------------------------------------ loader
-    uint32_t armed[NX] = {}, barmed = 0;
-    bool ok = true;
-    auto prefetch = [&](uint32_t j) {
-      if (lane == 0 && j < n) {
+    if (lane == 0) {
+      bool ok = true;
+      uint32_t xs = 0, bs = 0;  // tiles requested
+      auto prefetch = [&](uint32_t j) {
+        if (j >= n) return;
         prefetch_l2(a + poly0(j) * D, tile_bytes(j));
         prefetch_l2(b + poly0(j) * D, tile_bytes(j));
+      };
+      for (uint32_t j = 0; j < 3; ++j) prefetch(j);
+      for (uint32_t j = 0; ok && j < n; ++j) {
+        const uint32_t g = j & 1, u = j >> 1;
+        if (u && !(ok = mbar_wait_sleep(&bars[XFREE + g], (u - 1) & 1, err))) break;
+        mbar_arrive_expect_tx(&bars[AFULL + g], tile_bytes(j));
+        bulk_load(sm + OFF_X + g * XT, a + poly0(j) * D, tile_bytes(j), &bars[AFULL + g]);
+        ++xs;
+        if (j && !(ok = mbar_wait_sleep(&bars[BFREE + (g ^ 1)], ((j - 1) >> 1) & 1, err))) break;
+        mbar_arrive_expect_tx(&bars[BFULL + g], tile_bytes(j));
+        bulk_load(sm + OFF_B, b + poly0(j) * D, tile_bytes(j), &bars[BFULL + g]);
+        ++bs;
+        prefetch(j + 3);
       }
-    };
-    for (uint32_t j = 0; j < 3; ++j) prefetch(j);
-    for (uint32_t t = 0; ok && t < n + NX; ++t) {
-      const uint32_t buf = t % NX;
-      unsigned char* xb = sm + OFF_X + buf * XT;
-      if (t >= (uint32_t)NX) {  // store output tile t - 2, which frees the buffer
-        const uint32_t js = t - NX;
-        ok = warp_wait_fast(&bars[STAGED0 + buf], (js / NX) & 1, err);
-        if (ok && lane == 0) {
-          bulk_store(out + poly0(js) * D, xb, tile_bytes(js));
-          bulk_commit();
-          bulk_wait_read_all();
-        }
-        __syncwarp();
+      // nothing may still be writing shared memory at exit
+      for (uint32_t g = 0; g < 2; ++g) {
+        if (xs > g) mbar_wait_sleep(&bars[AFULL + g], ((xs - g - 1) >> 1) & 1, err);
+        if (bs > g) mbar_wait_sleep(&bars[BFULL + g], ((bs - g - 1) >> 1) & 1, err);
       }
-      if (ok && t < n) {
-        ++armed[buf];
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&bars[AFULL0 + buf], tile_bytes(t));
-          bulk_load(xb, a + poly0(t) * D, tile_bytes(t), &bars[AFULL0 + buf]);
-        }
-        __syncwarp();
-        // b's tile t, one row per lane, once F(t-1) has read tile t-1
-        if (t >= 1) ok = warp_wait_fast(&bars[BFREE], (t - 1) & 1, err);
-        if (ok) {
-          ++barmed;
-          if (lane == 0) mbar_arrive_expect_tx(&bars[BFULL], tile_bytes(t));
-          __syncwarp();
-          if ((uint32_t)lane * D * 4 < tile_bytes(t))
-            bulk_load(sm + OFF_B + lane * BROW, b + (poly0(t) + lane) * D, D * 4, &bars[BFULL]);
-          __syncwarp();
-        }
-      }
-      prefetch(t + 3);
     }
-    if (lane == 0) bulk_wait_all();
-    if (!ok) {
-      for (int i = 0; i < NX; ++i)
-        if (armed[i]) mbar_wait_sleep(&bars[AFULL0 + i], (armed[i] - 1) & 1, err);
-      if (barmed) mbar_wait_sleep(&bars[BFULL], (barmed - 1) & 1, err);
-    }
-  } else if (warp == MMA_WARP) {
+    __syncwarp();
+  } else if (warp >= MMA0) {
     // ------------------------------------------------------------ MMA issue
-    uint32_t armed[NBARS] = {};
-    auto issue = [&](uint32_t dcol, uint32_t abase, int bar) {
-      tc::fence_after_sync();
-      if (lane == 0) {
-        issue_transform(dcol, abase, s0 + OFF_W);
-        tc::mma_commit(&bars[bar]);
+    const uint32_t g = warp - MMA0;
+    if (lane == 0) {
+      uint32_t fwd = 0, inv = 0;
+      for (uint32_t j = g, u = 0; j < n; j += 2, ++u) {
+        if (!mbar_wait_sleep(&bars[PREP + g], u & 1, err)) break;
+        tc::fence_after_sync();
+        issue_transform(tbase + 256 * g, s0 + OFF_A + g * TILE, s0 + OFF_W);
+        tc::mma_commit(&bars[FDONE + g]);
+        ++fwd;
+        if (!mbar_wait_sleep(&bars[PREADY + g], u & 1, err)) break;
+        tc::fence_after_sync();
+        issue_transform(tbase + 256 * g, s0 + OFF_A + g * TILE, s0 + OFF_W);
+        tc::mma_commit(&bars[IDONE + g]);
+        ++inv;
       }
-      ++armed[bar];
-      __syncwarp();
-    };
-    bool ok = true;
-    for (uint32_t j = 0; ok && j < n; ++j) {
-      ok = warp_wait_fast(&bars[PREP], j & 1, err);
-      if (ok && j >= 1) ok = warp_wait_fast(&bars[FREAD], (j - 1) & 1, err);
-      if (!ok) break;
-      issue(R0, s0 + OFF_AF, FDONE);
-      ok = warp_wait_fast(&bars[PREADY], j & 1, err);
-      if (ok && j >= 1) ok = warp_wait_fast(&bars[EREAD], (j - 1) & 1, err);
-      if (!ok) break;
-      issue(R1, s0 + OFF_AI, IDONE);
+      // every MMA issued is done before shared and tensor memory are released
+      if (fwd) mbar_wait_sleep(&bars[FDONE + g], (fwd - 1) & 1, err);
+      if (inv) mbar_wait_sleep(&bars[IDONE + g], (inv - 1) & 1, err);
     }
-    // the last results must be read before the columns are freed
-    if (ok && n > 0) warp_wait(&bars[EREAD], (n - 1) & 1, err);
-    if (!ok) {
-      const int started[2] = {FDONE, IDONE};
-      for (int bar : started)
-        if (armed[bar]) mbar_wait_sleep(&bars[bar], (armed[bar] - 1) & 1, err);
-    }
+    __syncwarp();
   } else {
-    // ------------------------------------------------------------ epilogue
-    const uint32_t wl = warp & 3, cq = warp >> 2;  // block j1 = wl, columns 16 cq .. + 15
-    const uint32_t p = lane;                       // polynomial of this thread's row
-    const uint32_t row = 32 * wl + lane;
-    const uint32_t lane_off = ((32 * wl) << 16) + 16 * cq;
-    const int tid = threadIdx.x;  // 0 .. 511
+    // ------------------------------------------------------------ groups
+    const uint32_t g = warp / GROUP_WARPS;
+    const uint32_t aa = warp & 3, half = (warp >> 2) & 1;  // row block, columns 32 half .. + 31
+    const uint32_t p = lane;                               // polynomial of this thread's row
+    const uint32_t taddr = tc::tmem_addr(tbase, 32 * aa, 256 * g + 32 * half);
     const uint32_t q = k.q;
     bool ok = true;
-    // The 4-point steps give this thread coefficient / slot index bb = tid % 64
-    // of polynomials tid / 64 + 8 it: its twists are fixed. Montgomery words
-    // only; the Shoup companions are recomputed at use.
-    const uint32_t bb = tid & 63;
-    uint32_t twf[4], twi[4];
-#pragma unroll
-    for (int j1 = 0; j1 < 4; ++j1) {
-      twf[j1] = tw[TW_F + 64 * j1 + bb].x;
-      twi[j1] = tw[TW_I + 64 * j1 + bb].x;
-    }
-    const uint2 ci = tw[TW_C + 0], cz = tw[TW_C + 1], cz3 = tw[TW_C + 2];
-    const uint2 czi1 = tw[TW_C + 3], czi2 = tw[TW_C + 4], czi3 = tw[TW_C + 5];
-    auto mulw = [&](uint32_t x, uint32_t w) { return mont_c(x, w, w * k.qinv, q); };
-
-    // P(j): Y_{j1}[bb] for 4 polynomials per thread, into the forward A operand
-    auto prep = [&](uint32_t j) {
-      const uint32_t* x = reinterpret_cast<const uint32_t*>(sm + OFF_X + (j % NX) * XT);
-      unsigned char* af = sm + OFF_AF;
-#pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const uint32_t pp = (it * EPI_THREADS + tid) >> 6;
-        const uint32_t* xr = x + pp * D + bb;
-        const uint32_t x0 = xr[0], x1 = xr[64], x2 = xr[128], x3 = xr[192];
-        const uint32_t t2 = mulc(x2, ci, q), t3 = mulc(x3, ci, q);  // zeta^2 x2, zeta^2 x3
-        const uint32_t e0 = add_lazy(x0, t2, r1), e1 = sub_lazy(x0, t2, q);
-        const uint32_t o0 = add_lazy(x1, t3, r1), o1 = sub_lazy(x1, t3, q);
-        const uint32_t s = mulc(o0, cz, q), s1 = mulc(o1, cz3, q);
-        uint32_t z[4];
-        z[0] = add_lazy(e0, s, r1);   // j1 = 0: zeta^(a)
-        z[2] = sub_lazy(e0, s, q);    // j1 = 2: zeta^(5a)
-        z[1] = add_lazy(e1, s1, r1);  // j1 = 1: zeta^(3a)
-        z[3] = sub_lazy(e1, s1, q);   // j1 = 3: zeta^(7a)
-#pragma unroll
-        for (int j1 = 0; j1 < 4; ++j1) {
-          const uint32_t y = mulw(z[j1], twf[j1]);
-          *reinterpret_cast<uint32_t*>(af + sw128(32 * j1 + pp, bb >> 5, (bb & 31) >> 2, BOX) +
-                                       4 * (bb & 3)) = y;
-        }
-      }
+    // Outside the reductions a thread has word / slot index bb of the polynomials
+    // pp0 + 4 it: its twists are fixed.
+    const uint32_t bb = threadIdx.x & 63, pp0 = (threadIdx.x & (GROUP - 1)) >> 6;
+    const uint2 wm2 = tw[TW_W + bb], wm1 = tw[TW_W + 64 + bb], w1 = tw[TW_W + 128 + bb],
+                w2 = tw[TW_W + 192 + bb], im = tw[TW_I];
+    unsigned char* const opnd = sm + OFF_A + g * TILE;
+    uint32_t* const x = reinterpret_cast<uint32_t*>(sm + OFF_X + g * XT);
+    const uint32_t* const bt = reinterpret_cast<const uint32_t*>(sm + OFF_B);
+    // word of K index kk of row 32 a + pp of the A operand
+    auto operand = [&](uint32_t a_, uint32_t pp, uint32_t kk) -> uint32_t* {
+      return reinterpret_cast<uint32_t*>(
+          opnd + sw128(32 * a_ + pp, kk >> 5, (kk & 31) >> 2, BOX) + 4 * (kk & 3));
     };
-    // F(j): forward results (x) b -> inverse A operand
-    auto forward_out = [&](uint32_t j) -> bool {
-      bool got = warp_wait_fast(&bars[FDONE], j & 1, err);
-      got = got && warp_wait_fast(&bars[BFULL], j & 1, err);
-      if (!epi_all(got)) return false;
-      tc::fence_after_sync();
-      uint32_t res[16];
-      reduce16(R0 + lane_off, k, res);
+    // Reduced results from the layout of the rows to buffer `to`: word 64 a + c of
+    // polynomial p at that index with its low 5 bits XORed with p (the 32 lanes hit 32
+    // banks, here and where a warp reads 32 consecutive c of one polynomial)
+    auto exchange = [&](uint32_t* to) {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        uint32_t res[16];
+        reduce16(taddr + 16 * h, k, res);
+#pragma unroll
+        for (int t = 0; t < 16; ++t)
+          to[p * D + ((64 * aa + 32 * half + 16 * h + t) ^ p)] = res[t];
+      }
       tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[FREAD]);  // columns 0-255 free for fwd(j+1)
-      // b at slots 4 (16 cq + t) + wl of polynomial p
-      const uint32_t* brow = reinterpret_cast<const uint32_t*>(sm + OFF_B + p * BROW) + 64 * cq + wl;
-      uint32_t bv[16];
-#pragma unroll
-      for (int t = 0; t < 16; ++t) bv[t] = brow[4 * t];
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[BFREE]);
-#pragma unroll
-      for (int t = 0; t < 16; ++t) res[t] = redc64(mad_wide(res[t], bv[t], 0ull), q, k.qinv);
-      unsigned char* ai = sm + OFF_AI;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(ai + sw128(row, cq >> 1, (cq & 1) * 4 + c, BOX)) =
-            make_uint4(res[4 * c], res[4 * c + 1], res[4 * c + 2], res[4 * c + 3]);
-      tc::fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[PREADY]);
-      return true;
+      group_sync(g);
     };
-    // E(j): inverse results -> 4-point inverse -> output tile in buffer j % 3
-    auto inverse_out = [&](uint32_t j) -> bool {
-      if (!epi_all(warp_wait_fast(&bars[IDONE], j & 1, err))) return false;
-      tc::fence_after_sync();
-      uint32_t res[16];
-      reduce16(R1 + lane_off, k, res);
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[EREAD]);  // columns 256-511 free for inv(j+1)
-      uint32_t* x = reinterpret_cast<uint32_t*>(sm + OFF_X + (j % NX) * XT);
-      // column 16 cq + t is V_{wl}[c] with c = -(16 cq + t) mod 64; word 64 wl + c of
-      // polynomial p, its low 5 bits XORed with p (the 32 lanes hit 32 banks)
-#pragma unroll
-      for (int t = 0; t < 16; ++t) {
-        const uint32_t c = (64u - (16u * cq + t)) & 63u;
-        x[p * D + ((64 * wl + c) ^ p)] = res[t];
-      }
-      epi_sync();
-      uint32_t o[4][4];
-#pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const uint32_t pp = (it * EPI_THREADS + tid) >> 6;
-        const uint32_t* xr = x + pp * D;
-        uint32_t v[4];
-#pragma unroll
-        for (int j1 = 0; j1 < 4; ++j1) v[j1] = mulw(xr[(64 * j1 + bb) ^ pp], twi[j1]);
-        const uint32_t p0 = add_canon(v[0], v[2], q), q0 = sub_lazy(v[0], v[2], q);
-        const uint32_t p1 = add_canon(v[1], v[3], q), q1 = sub_lazy(v[1], v[3], q);
-        const uint32_t tq = mulc(q1, czi2, q);
-        o[it][0] = add_canon(p0, p1, q);
-        o[it][1] = mulc(add_canon(q0, tq, q), czi1, q);
-        o[it][2] = mulc(sub_lazy(p0, p1, q), czi2, q);
-        o[it][3] = mulc(sub_lazy(q0, tq, q), czi3, q);
-      }
-      epi_sync();  // every swizzled word read before the tile is rewritten in order
-#pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const uint32_t pp = (it * EPI_THREADS + tid) >> 6;
-#pragma unroll
-        for (int aa = 0; aa < 4; ++aa) x[pp * D + 64 * aa + bb] = o[it][aa];
-      }
-      tc::fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[STAGED0 + j % NX]);
-      return true;
+    auto arrive = [&](int bar) {
+      if (lane == 0) mbar_arrive(&bars[bar + g]);
     };
 
-    for (uint32_t j = 0; ok && j < n; ++j) {
-      ok = epi_all(warp_wait_fast(&bars[AFULL0 + j % NX], (j / NX) & 1, err));
-      if (!ok) break;
-      prep(j);  // the forward A operand is free: F(j-1) saw fwd(j-1) complete
+    for (uint32_t j = g, u = 0; j < n; j += 2, ++u) {
+      // P(j)
+      ok = ok && lane0_wait(&bars[AFULL + g], u & 1, lane, err);
+#pragma unroll 4
+      for (int it = 0; it < 8; ++it) {
+        const uint32_t pp = pp0 + 4 * it;
+        const uint4 v = reinterpret_cast<const uint4*>(x)[pp * (D / 4) + bb];
+        *operand(0, pp, bb) = v.x;
+        *operand(1, pp, bb) = v.y;
+        *operand(2, pp, bb) = v.z;
+        *operand(3, pp, bb) = v.w;
+      }
       tc::fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[PREP]);
-      if (j >= 1 && !(ok = inverse_out(j - 1))) break;  // also frees the inverse A operand
-      if (!(ok = forward_out(j))) break;
+      arrive(PREP);
+      // F(j)
+      ok = ok && lane0_wait(&bars[FDONE + g], u & 1, lane, err);
+      tc::fence_after_sync();
+      exchange(x);
+      ok = ok && lane0_wait(&bars[BFULL + g], u & 1, lane, err);
+#pragma unroll 2
+      for (int it = 0; it < 8; ++it) {
+        const uint32_t pp = pp0 + 4 * it;
+        uint32_t v[4], z[4];
+#pragma unroll
+        for (int a_ = 0; a_ < 4; ++a_) v[a_] = x[pp * D + ((64 * a_ + bb) ^ pp)];
+        v[0] = mulc(v[0], wm2, q);
+        v[1] = mulc(v[1], wm1, q);
+        v[3] = mulc(v[3], w1, q);
+        // all canonical: b is any word
+        const uint32_t c0 = add_canon(v[0], v[2], q), c1 = sub_lazy(v[0], v[2], q);
+        const uint32_t e0 = add_canon(v[1], v[3], q);
+        const uint32_t e1 = mulc(sub_lazy(v[1], v[3], q), im, q);
+        z[0] = add_canon(c0, e0, q);
+        z[2] = sub_lazy(c0, e0, q);
+        z[1] = add_canon(c1, e1, q);
+        z[3] = sub_lazy(c1, e1, q);
+#pragma unroll
+        for (int j1 = 0; j1 < 4; ++j1)
+          z[j1] = redc64(mad_wide(z[j1], bt[pp * D + 64 * j1 + bb], 0ull), q, k.qinv);
+        const uint32_t t0 = add_canon(z[0], z[2], q), d0 = sub_lazy(z[0], z[2], q);
+        const uint32_t t1 = add_canon(z[1], z[3], q);
+        const uint32_t d1 = mulc(sub_lazy(z[1], z[3], q), im, q);
+        *operand(0, pp, 63 - bb) = mulc(add_lazy(t0, t1, r1), w2, q);
+        *operand(1, pp, 63 - bb) = mulc(sub_lazy(d0, d1, q), w1, q);
+        *operand(2, pp, 63 - bb) = sub_lazy(t0, t1, q);
+        *operand(3, pp, 63 - bb) = mulc(add_lazy(d0, d1, r1), wm1, q);
+      }
+      tc::fence_async_smem();  // the operand, and X before its refill by a bulk copy
+      __syncwarp();
+      arrive(BFREE);
+      arrive(XFREE);
+      arrive(PREADY);
+      // E(j)
+      ok = ok && lane0_wait(&bars[IDONE + g], u & 1, lane, err);
+      tc::fence_after_sync();
+      uint32_t* ex = reinterpret_cast<uint32_t*>(opnd);
+      exchange(ex);
+      const unsigned long long first = poly0(j);
+      const uint32_t valid = tile_bytes(j) / (D * 4);
+      uint4* o = reinterpret_cast<uint4*>(out + first * D) + bb;
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const uint32_t pp = pp0 + 4 * it;
+        const uint32_t* xr = ex + pp * D;
+        if (ok && pp < valid)
+          o[pp * (D / 4)] = make_uint4(xr[bb ^ pp], xr[(64 + bb) ^ pp], xr[(128 + bb) ^ pp],
+                                       xr[(192 + bb) ^ pp]);
+      }
+      group_sync(g);  // the exchange is read before P(j + 2) writes the operand there
     }
-    if (ok && n > 0) inverse_out(n - 1);
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == MMA_WARP) {
+  if (warp == MMA0) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tbase, 512);
   }
@@ -400,7 +334,7 @@ int launch_ntt256_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* 
   static int bps_cache[kMaxDevices] = {};
   int bps = 0;
   const int st =
-      prepare_kernel(ntt256_tc_mulinv_kernel, SMEM_BYTES, THREADS, p->device, bps_cache, &bps);
+      prepare_kernel(ntt256_tc_mulinv_kernel, SMEM_BYTES, THREADS256, p->device, bps_cache, &bps);
   if (st) return st;
   const unsigned long long tiles = (npolys + PT - 1) / PT;
   const unsigned long long grid =
@@ -408,15 +342,15 @@ int launch_ntt256_tc(const grid_gpu_plan* p, const uint32_t* a, const uint32_t* 
   TcConsts k;
   k.q = p->f.q;
   k.qinv = p->f.qinv;
-  ntt256_tc_mulinv_kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(
+  ntt256_tc_mulinv_kernel<<<(unsigned)grid, THREADS256, SMEM_BYTES, s>>>(
       a, b, out, (unsigned long long)npolys, static_cast<const unsigned char*>(p->d_tcw), k,
       p->f.r1, p->d_err);
   return cuda_status(cudaGetLastError());
 }
 
 // The 64-point matrix image (row 64 l + j, K byte 4k + i = byte l of
-// 2^(8i) omega^(jk) 2^32 mod q, 128-byte-swizzled K-major), then the twist and
-// 4-point constants as {Montgomery word, word * q^-1 mod 2^32}.
+// 2^(8i) (psi^128 / 16) psi^(2 (2 j + 1)(2 k + 1)) 2^32 mod q, 128-byte-swizzled K-major),
+// then the twists as {Montgomery word, word * q^-1 mod 2^32}.
 void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& out) {
   out.assign(TABLE_BYTES, 0);
   auto mulm = [q](uint64_t x, uint64_t y) { return (uint64_t)((unsigned __int128)x * y % q); };
@@ -433,10 +367,11 @@ void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& ou
   uint32_t qinv = 1;
   for (int i = 0; i < 5; ++i) qinv *= 2u - q * qinv;
   const uint64_t R = ((uint64_t)1 << 32) % q;
-  const uint64_t omega = powm(psi, 8);
+  const uint64_t im = powm(psi, 128);
+  const uint64_t scale = mulm(mulm(im, powm(16, q - 2)), R);
   for (uint32_t j = 0; j < 64; ++j)
     for (uint32_t kk = 0; kk < 64; ++kk) {
-      uint64_t w = mulm(powm(omega, (j * kk) % 64), R);
+      uint64_t w = mulm(powm(psi, (2 * (2 * j + 1) * (2 * kk + 1)) % (2 * D)), scale);
       for (uint32_t i = 0; i < 4; ++i) {
         const uint32_t kb = 4 * kk + i, h = kb / 128, kc = kb % 128;
         for (uint32_t l = 0; l < 4; ++l)
@@ -449,21 +384,14 @@ void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& ou
     const uint32_t pair[2] = {wm, wm * qinv};
     std::memcpy(out.data() + (size_t)idx * 8, pair, 8);
   };
-  const uint64_t psi_inv = powm(psi, 2 * D - 1);
-  const uint64_t dinv = powm(D, q - 2);
-  for (uint32_t j1 = 0; j1 < 4; ++j1)
-    for (uint32_t bb = 0; bb < 64; ++bb) {
-      const uint64_t e = ((2 * j1 + 1) * bb) % (2 * D);
-      put(TW_F + 64 * j1 + bb, powm(psi, e));
-      put(TW_I + 64 * j1 + bb, mulm(dinv, powm(psi_inv, e)));
-    }
-  const uint64_t zeta = powm(psi, 64), zeta_inv = powm(psi_inv, 64);
-  put(TW_C + 0, powm(zeta, 2));
-  put(TW_C + 1, zeta);
-  put(TW_C + 2, powm(zeta, 3));
-  put(TW_C + 3, zeta_inv);
-  put(TW_C + 4, powm(zeta_inv, 2));
-  put(TW_C + 5, powm(zeta_inv, 3));
+  for (uint32_t j2 = 0; j2 < 64; ++j2) {
+    const uint32_t e = 2 * j2 + 1, order = 2 * D;
+    put(TW_W + j2, powm(psi, order - 2 * e % order));
+    put(TW_W + 64 + j2, powm(psi, order - e));
+    put(TW_W + 128 + j2, powm(psi, e));
+    put(TW_W + 192 + j2, powm(psi, 2 * e % order));
+  }
+  put(TW_I, im);
 }
 
 }  // namespace grid

@@ -245,6 +245,62 @@ def grouped_roles(items, nsa, nsb, nacc):
                     + [epilogue() for _ in (0, 1)])
 
 
+def product256_roles(n):
+    """ntt256_tc_mulinv_kernel: two groups, each with an operand and a buffer of its own, one
+    tile of b between them."""
+    def loader():
+        for j in range(n):
+            g, u = j & 1, j >> 1
+            if u:
+                yield ("wait", f"XFREE{g}", u - 1)
+            yield ("async", f"AFULL{g}", (f"x{g}", "w", ("in", j)))
+            if j:
+                yield ("wait", f"BFREE{g ^ 1}", (j - 1) >> 1)
+            yield ("async", f"BFULL{g}", ("b", "w", j))
+
+    def mma(g):
+        for u, j in enumerate(range(g, n, 2)):
+            yield ("wait", f"PREP{g}", u)
+            yield ("async", f"FDONE{g}", *((f"a{g}{h}", "r", ("fwd", j)) for h in range(WARPS)),
+                   (f"col{g}", "w", ("fwd", j)))
+            yield ("wait", f"PREADY{g}", u)
+            yield ("async", f"IDONE{g}", *((f"a{g}{h}", "r", ("inv", j)) for h in range(WARPS)),
+                   (f"col{g}", "w", ("inv", j)))
+
+    def warp(g, h):
+        syncs = 0
+        for u, j in enumerate(range(g, n, 2)):
+            yield ("wait", f"AFULL{g}", u)
+            yield ("touch", f"x{g}", "r", ("in", j))
+            yield ("touch", f"a{g}{h}", "w", ("fwd", j))
+            yield ("arrive", f"PREP{g}")
+            yield ("wait", f"FDONE{g}", u)
+            yield ("touch", f"col{g}", "r", ("fwd", j))
+            yield ("touch", f"x{g}", "w", ("ex", j))
+            for phase in ("F", "E", "done"):
+                if phase == "E":
+                    yield ("wait", f"IDONE{g}", u)
+                    yield ("touch", f"col{g}", "r", ("inv", j))
+                    yield ("touch", f"a{g}{h}", "w", ("ex", j))
+                yield ("arrive", f"SYNC{g}")
+                yield ("wait", f"SYNC{g}", syncs)
+                syncs += 1
+                if phase == "F":
+                    yield ("wait", f"BFULL{g}", u)
+                    yield ("touch", "b", "r", j)
+                    yield ("touch", f"x{g}", "r", ("ex", j))
+                    yield ("touch", f"a{g}{h}", "w", ("inv", j))
+                    for bar in ("BFREE", "XFREE", "PREADY"):
+                        yield ("arrive", f"{bar}{g}")
+                elif phase == "E":
+                    for o in range(WARPS):
+                        yield ("touch", f"a{g}{o}", "r", ("ex", j))
+
+    counts = {f"{b}{g}": WARPS for b in ("XFREE", "BFREE", "PREP", "PREADY", "SYNC") for g in (0, 1)}
+    return counts, ([loader(), mma(0), mma(1)]
+                    + [warp(g, h) for g in (0, 1) for h in range(WARPS)])
+
+
 def unit_roles(n, warps=4, group=2):
     """The JL kernels' hand-over: groups of warps share a barrier pair; n units go round
     the warps, a warp without a last unit arrives for its group."""
@@ -278,7 +334,7 @@ def unit_roles(n, warps=4, group=2):
 
 @pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 9, 13])
 @pytest.mark.parametrize("kind", ["transform", "product", "planes11", "planes12", "planes22",
-                                  "units"])
+                                  "units", "product256"])
 def test_protocol(n, kind):
     rng = random.Random(100 * n + len(kind))
     for _ in range(150):
@@ -286,6 +342,8 @@ def test_protocol(n, kind):
             counts, roles = transform_roles(n)
         elif kind == "product":
             counts, roles = product_roles(n)
+        elif kind == "product256":
+            counts, roles = product256_roles(n)
         elif kind == "units":
             counts, roles = unit_roles(n)
         else:
