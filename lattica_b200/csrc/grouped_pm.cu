@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kGpThreads, 2)
         for (uint32_t c = 0; c < nch; ++c, ++gc) {
           const uint32_t sl = gc % NSA, kc = w.k0 + c * KCH;
           if (c && kc % KBLK == 0) ch = chunk_at(xtiles, x0, kc);
-          if (gc >= (uint32_t)NSA && !(ok = mbar_wait(&a_free[sl], ((gc / NSA) - 1) & 1, err)))
+          if (gc >= (uint32_t)NSA && !(ok = mbar_wait_sleep(&a_free[sl], ((gc / NSA) - 1) & 1, err)))
             break;
           const uint32_t bar = smem_addr(&full[sl]);
           const uint32_t nrows = (ch.live + 7) & ~7u;
@@ -233,9 +233,9 @@ __global__ void __launch_bounds__(kGpThreads, 2)
         const uint32_t nch = item_chunks(work[wi]);
         for (uint32_t c = 0; c < nch; ++c, ++gc) {
           const uint32_t sl = gc % NSA, bs = gc % NSB;
-          if (!(ok = mbar_wait(&full[sl], (gc / NSA) & 1, err)) ||
-              !(ok = mbar_wait(&zeroed[sl], (gc / NSA) & 1, err)) ||
-              !(ok = mbar_wait(&built[bs], (gc / NSB) & 1, err)))
+          if (!(ok = mbar_wait_sleep(&full[sl], (gc / NSA) & 1, err)) ||
+              !(ok = mbar_wait_sleep(&zeroed[sl], (gc / NSA) & 1, err)) ||
+              !(ok = mbar_wait_sleep(&built[bs], (gc / NSB) & 1, err)))
             break;
           tc::fence_after_sync();
           const uint32_t sa = s0 + sl * S::ASLOT, sb = s0 + S::OFF_B + bs * S::BSLOT;
