@@ -156,8 +156,12 @@ __device__ __forceinline__ void tmem_ld_wait7(uint32_t (&r)[7][8]) {
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld_wait() {
+// Wait for this thread's tensor-memory loads; no use of r can be scheduled above it.
+template <int N>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[N]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
 }
 
 // Wait for this thread's tensor-memory loads, naming the 16 registers they

@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
     uint32_t dv[2][4];
     tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 0), dv[0]);
     tc::tmem_ld4(tc::tmem_addr(tbase, 32 * warp, 16), dv[1]);
-    tc::tmem_ld_wait();
+    tc::tmem_ld_wait(dv[0]);
+    tc::tmem_ld_wait(dv[1]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int row = tile_row_to_row(128 * h + 32 * warp + lane);
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(kEvThreads, 1) jl_eval_tc_kernel(
     for (int t0 = tbeg; t0 < tbeg + 32; t0 += 2) {
       uint32_t dv[8];
       tc::tmem_ld8(base + 4 * t0, dv);
-      tc::tmem_ld_wait();
+      tc::tmem_ld_wait(dv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) dv[i] = unscale(dv[i], lane);
 #pragma unroll

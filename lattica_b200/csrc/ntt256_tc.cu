@@ -367,11 +367,13 @@ void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& ou
   uint32_t qinv = 1;
   for (int i = 0; i < 5; ++i) qinv *= 2u - q * qinv;
   const uint64_t R = ((uint64_t)1 << 32) % q;
-  const uint64_t im = powm(psi, 128);
+  std::vector<uint64_t> power(2 * D, 1);  // of psi
+  for (uint32_t e = 1; e < 2 * D; ++e) power[e] = mulm(power[e - 1], psi);
+  const uint64_t im = power[128];
   const uint64_t scale = mulm(mulm(im, powm(16, q - 2)), R);
   for (uint32_t j = 0; j < 64; ++j)
     for (uint32_t kk = 0; kk < 64; ++kk) {
-      uint64_t w = mulm(powm(psi, (2 * (2 * j + 1) * (2 * kk + 1)) % (2 * D)), scale);
+      uint64_t w = mulm(power[(2 * (2 * j + 1) * (2 * kk + 1)) % (2 * D)], scale);
       for (uint32_t i = 0; i < 4; ++i) {
         const uint32_t kb = 4 * kk + i, h = kb / 128, kc = kb % 128;
         for (uint32_t l = 0; l < 4; ++l)
@@ -386,10 +388,10 @@ void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& ou
   };
   for (uint32_t j2 = 0; j2 < 64; ++j2) {
     const uint32_t e = 2 * j2 + 1, order = 2 * D;
-    put(TW_W + j2, powm(psi, order - 2 * e % order));
-    put(TW_W + 64 + j2, powm(psi, order - e));
-    put(TW_W + 128 + j2, powm(psi, e));
-    put(TW_W + 192 + j2, powm(psi, 2 * e % order));
+    put(TW_W + j2, power[order - 2 * e % order]);
+    put(TW_W + 64 + j2, power[order - e]);
+    put(TW_W + 128 + j2, power[e]);
+    put(TW_W + 192 + j2, power[2 * e % order]);
   }
   put(TW_I, im);
 }
