@@ -71,7 +71,7 @@ constexpr uint32_t OFF_A = OFF_W + WMAT;    // [2] A operand, then E's exchange
 constexpr uint32_t OFF_X = OFF_A + 2 * TILE;  // [2] input tile, then F's exchange
 constexpr uint32_t OFF_B = OFF_X + 2 * XT;  // b's tile
 constexpr uint32_t OFF_BAR = OFF_B + XT;
-constexpr uint32_t OFF_TADDR = OFF_BAR + 16 * 8;
+constexpr uint32_t OFF_TADDR = OFF_BAR + 18 * 8;
 constexpr uint32_t SMEM_BYTES = OFF_TADDR + 16 + 1024;  // + alignment slack
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
@@ -91,7 +91,8 @@ enum Bar : int {
   FDONE = 10,
   PREADY = 12,        // inverse operand written
   IDONE = 14,
-  NBARS = 16
+  WFULL = 16,         // the matrix landed (one barrier)
+  NBARS
 };
 
 // The warps of a group (named barrier 1 or 2).
@@ -117,14 +118,7 @@ __global__ void __launch_bounds__(THREADS256, 1)
   uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(sm + OFF_TADDR);
   const uint2* tw = reinterpret_cast<const uint2*>(table);
 
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(table);
-    uint4* w = reinterpret_cast<uint4*>(sm + OFF_W);
-    for (int i = threadIdx.x; i < (int)(WMAT / 16); i += THREADS256) w[i] = src[i];
-  }
   if (warp == MMA0) {
-    tc::tmem_alloc(taddr_slot, 512);
-    tc::tmem_relinquish();
     if (lane == 0) {
       for (int i = 0; i < NBARS; ++i)
         mbar_init(&bars[i], (i & ~1) == XFREE || (i & ~1) == BFREE || (i & ~1) == PREP ||
@@ -132,9 +126,14 @@ __global__ void __launch_bounds__(THREADS256, 1)
                                 ? GROUP_WARPS
                                 : 1);
       fence_mbar_init();
+      tc::fence_async_smem();
+      mbar_arrive_expect_tx(&bars[WFULL], WMAT);
+      bulk_load(sm + OFF_W, table, WMAT, &bars[WFULL]);
     }
+    __syncwarp();
+    tc::tmem_alloc(taddr_slot, 512);
+    tc::tmem_relinquish();
   }
-  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -187,7 +186,8 @@ __global__ void __launch_bounds__(THREADS256, 1)
     const uint32_t g = warp - MMA0;
     if (lane == 0) {
       uint32_t fwd = 0, inv = 0;
-      for (uint32_t j = g, u = 0; j < n; j += 2, ++u) {
+      const bool ready = mbar_wait_sleep(&bars[WFULL], 0, err);
+      for (uint32_t j = g, u = 0; ready && j < n; j += 2, ++u) {
         if (!mbar_wait_sleep(&bars[PREP + g], u & 1, err)) break;
         tc::fence_after_sync();
         issue_transform(tbase + 256 * g, s0 + OFF_A + g * TILE, s0 + OFF_W);

@@ -70,6 +70,7 @@ enum Bar : int {
   IDONE,                // inverse done (S and D read)
   EREAD,                // its columns read
   DRAIN,                // every MMA done
+  WFULL,                // the matrices landed
   NBARS
 };
 static_assert(NBARS <= 32, "barrier slots");
@@ -106,15 +107,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
   uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(bars + 32);
 
-  {
-    uint4* w = reinterpret_cast<uint4*>(sm + OFF_W);
-    for (int i = threadIdx.x; i < (int)(WMAT / 16); i += THREADS) w[i] = wtab[i];
-    uint4* g = reinterpret_cast<uint4*>(sm + OFF_G);
-    for (int i = threadIdx.x; i < (int)(2 * BOX / 16); i += THREADS) g[i] = gtab[i];
-  }
   if (warp == MMA_WARP) {
-    tc::tmem_alloc(taddr_slot, 512);
-    tc::tmem_relinquish();
     if (lane == 0) {
       for (int i = 0; i < NXA; ++i) {
         mbar_init(&bars[AFULL + i], 1);
@@ -130,10 +123,17 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&bars[IDONE], 1);
       mbar_init(&bars[EREAD], 2 * GROUP_WARPS);
       mbar_init(&bars[DRAIN], 1);
+      mbar_init(&bars[WFULL], 1);
       fence_mbar_init();
+      tc::fence_async_smem();
+      mbar_arrive_expect_tx(&bars[WFULL], WMAT + 2 * BOX);
+      bulk_load(sm + OFF_W, wtab, WMAT, &bars[WFULL]);
+      bulk_load(sm + OFF_G, gtab, 2 * BOX, &bars[WFULL]);
     }
+    __syncwarp();
+    tc::tmem_alloc(taddr_slot, 512);
+    tc::tmem_relinquish();
   }
-  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         tc::mma_commit(&bars[IDONE]);
         return true;
       };
-      bool ok = true;
+      bool ok = mbar_wait(&bars[WFULL], 0, err);
       uint32_t boxes = 0;
       for (uint32_t j = 0; ok && j < n; ++j) {
         if (j) ok = mbar_wait(&bars[FREAD], (j - 1) & 1, err);

@@ -25,7 +25,8 @@
 // L2 prefetch), warp 16 issues the MMAs into two sets of tensor-memory columns in
 // turn, warps 0-15 reduce one tile while the next is multiplied. Epilogue warp w owns
 // tensor-memory lanes 32 (w % 4) .. + 31 (its rows) and columns 16 (w / 4) .. + 15 of
-// each E_l block. Bound by HBM: 512 bytes a polynomial. At 2^22
+// each E_l block. The B matrix comes by one bulk copy beside the first tiles' loads.
+// Bound by HBM: 512 bytes a polynomial. At 2^22
 // polynomials in place 0.36 ms forward and 0.34 inverse (0.91 and 0.97 of the measured
 // rate); with two buffers and one set of columns 0.39 and 0.44. A buffer is refilled once
 // the store issued before the newest one has read it: a point-major store (64 rows of 512
@@ -55,7 +56,7 @@ constexpr int NBUF = 4;
 constexpr uint32_t OFF_XA = 0;                     // input tiles, then their results
 constexpr uint32_t OFF_W = OFF_XA + NBUF * TILE;   // B matrix
 constexpr uint32_t OFF_BAR = OFF_W + WMAT;
-constexpr uint32_t SMEM_BYTES = OFF_BAR + (2 * NBUF + 4) * 8 + 16 + 1024;  // + alignment slack
+constexpr uint32_t SMEM_BYTES = OFF_BAR + (2 * NBUF + 5) * 8 + 16 + 1024;  // + alignment slack
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
 enum Bar : int {
@@ -63,7 +64,8 @@ enum Bar : int {
   STAGED = AFULL + NBUF, // [4] result tile written into buffer i
   FDONE = STAGED + NBUF, // [2] transform done into column set i
   FREAD = FDONE + 2,     // [2] column set read
-  NBARS = FREAD + 2
+  WFULL = FREAD + 2,     // B matrix landed
+  NBARS
 };
 
 // MODE_FWD / MODE_INV / MODE_FWD_PM. Tile j of this CTA uses buffer j % 4 and column set
@@ -87,14 +89,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
   uint32_t* taddr_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
 
-  {
-    const uint4* w1 = wtab + (MODE == MODE_INV ? WMAT / 16 : 0);
-    uint4* w = reinterpret_cast<uint4*>(sm + OFF_W);
-    for (int i = threadIdx.x; i < (int)(WMAT / 16); i += THREADS) w[i] = w1[i];
-  }
   if (warp == MMA_WARP) {
-    tc::tmem_alloc(taddr_slot, 512);
-    tc::tmem_relinquish();
     if (lane == 0) {
       for (int i = 0; i < NBUF; ++i) {
         mbar_init(&bars[AFULL + i], 1);
@@ -104,10 +99,16 @@ __global__ void __launch_bounds__(THREADS, 1)
         mbar_init(&bars[FDONE + i], 1);
         mbar_init(&bars[FREAD + i], EPI_WARPS);
       }
+      mbar_init(&bars[WFULL], 1);
       fence_mbar_init();
+      tc::fence_async_smem();
+      mbar_arrive_expect_tx(&bars[WFULL], WMAT);
+      bulk_load(sm + OFF_W, wtab + (MODE == MODE_INV ? WMAT / 16 : 0), WMAT, &bars[WFULL]);
     }
+    __syncwarp();
+    tc::tmem_alloc(taddr_slot, 512);
+    tc::tmem_relinquish();
   }
-  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -194,9 +195,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------ MMA issue
     uint32_t issued = 0;
-    bool ok = true;
     if (lane == 0) {
-      for (uint32_t j = 0; j < n; ++j) {
+      bool ok = mbar_wait(&bars[WFULL], 0, err);
+      for (uint32_t j = 0; ok && j < n; ++j) {
         ok = mbar_wait(&bars[AFULL + j % NBUF], (j / NBUF) & 1, err);
         if (ok && j >= 2) ok = mbar_wait(&bars[FREAD + (j & 1)], ((j >> 1) - 1) & 1, err);
         if (!ok) break;
