@@ -124,6 +124,12 @@ __device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem,
                : "memory");
 }
 
+// Contiguous global bytes -> L2 (a multiple of 16, 16-byte aligned; no shared memory, no
+// completion tracking).
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ void bulk_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }

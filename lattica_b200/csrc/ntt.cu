@@ -617,12 +617,14 @@ __global__ void __launch_bounds__(D * kSmallSlots) commit_small_kernel(
 // spend 44 cycles on every MMA for one useful row of 128.
 //  * vec_partial_kernel: a CTA takes up to 64 columns at a time of one product: eight
 //    threads transform each polynomial (as in commit_small_kernel), thread (e, slot)
-//    accumulates evaluation point e of rows slot, slot + 8, ... over the columns; the
-//    canonical sums go to part [cta][row][e].
+//    accumulates evaluation point e of rows slot, slot + 8, ... over the columns, which
+//    are on their way to L2 since the kernel's first instruction; the canonical sums go
+//    to part [cta][row][e].
 //  * vec_finish_kernel: a CTA per output polynomial sums the partials and inverts.
 // Two launches for the sum of two products, where each took a transform, a product and
 // an inverse of its own and an addition. u1 = B t + C g and u2 = D h of the LaBRADOR level
-// at r = 64, kappa = 16: 119 us before, 45 us now.
+// at r = 64, kappa = 16: 119 us before, 45 us, and 43 with the matrix's rows sent for
+// before the transforms and the sum over 296 partials on 512 threads (on 256 46, on 1024 43).
 // ---------------------------------------------------------------------------
 constexpr int kVecMaxRows = 64, kVecMaxBatch = 4, kVecCols = 64;
 constexpr int kVecThreads = 512;
@@ -642,14 +644,19 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
   __shared__ uint2 tws[TWN];
   __shared__ __align__(16) uint32_t sh[kVecCols * PS];
   const int tid = threadIdx.x;
-  for (int i = tid; i < TWN; i += kVecThreads) tws[i] = gtw[i];
-  __syncthreads();
-  grid_dep_wait();
-  grid_dep_launch();
   const bool second = (int)blockIdx.x >= p0.ctas;
   const VecProduct& p = second ? p1 : p0;
   const int c0 = ((int)blockIdx.x - (second ? p0.ctas : 0)) * p.span;
   const int c1 = min(p.cols, c0 + p.span);
+  auto prefetch = [&](int k) {  // the matrix's block of columns from k on, a thread per row
+    if (tid < rows && k < c1)
+      prefetch_l2(p.A + ((size_t)tid * p.ld + k) * D, (uint32_t)(min(kVecCols, c1 - k) * D * 4));
+  };
+  prefetch(c0);
+  for (int i = tid; i < TWN; i += kVecThreads) tws[i] = gtw[i];
+  __syncthreads();
+  grid_dep_wait();
+  grid_dep_launch();
   const uint32_t* s = p.s + (size_t)blockIdx.y * p.cols * D;
   const int pl = tid / T, t = tid % T;
   const int bt_t = brv(4 * t, LOGD);
@@ -660,6 +667,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
   for (int i = 0; i < RPT; ++i) acc96_zero(acc[i]);
   for (int k0 = c0; k0 < c1; k0 += kVecCols) {  // uniform over the CTA
     const int n = min(kVecCols, c1 - k0);
+    prefetch(k0 + kVecCols);
     {  // groups past the last polynomial transform zeros
       uint32_t x[E];
 #pragma unroll
@@ -708,7 +716,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
   }
 }
 
-constexpr int kVfThreads = 256;
+constexpr int kVfThreads = 512;
 
 __global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
     const uint32_t* __restrict__ part, int count, int rows, uint32_t* __restrict__ t_out,
@@ -730,7 +738,8 @@ __global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
   if (g == 0) {
 #pragma unroll
     for (int i = 1; i < G; ++i) v += sums[i][e];
-    sh[e] = (uint32_t)(v % f.q);
+    sh[e] = add_mod(reduce_word((uint32_t)v, f),  // 2^32 v_1 + v_0 mod q
+                    mont_mul((uint32_t)(v >> 32), f.r2, f.q, f.qinv), f.q);
   }
   __syncthreads();
   // eight threads invert; the others repeat them (the stages hold CTA barriers)

@@ -192,11 +192,6 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
       : "memory");
 }
 
-// Contiguous global bytes -> L2 (no shared memory, no completion tracking).
-__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-
 // Bounded wait by lane 0 alone (mbarrier operations of a whole warp on one
 // barrier serialise over its lanes); __syncwarp then orders what lane 0
 // acquired before every lane's later accesses.
