@@ -986,10 +986,11 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
       int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, cs);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, Aq->d_evals_pm, (int)r, (int)kappa, (int)n, (int)ldx,
-                           (int)Aq->ld_pm, EMM_DENSE, false, tl.out ? nullptr : tt, tl, work, cs);
+                           (int)Aq->ld_pm, EMM_DENSE, false, tl.out ? nullptr : tt, tl, work, cs,
+                           true);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
-                           false, gg, gl, work, cs);
+                           false, gg, gl, work, cs, true);
       return rc;
     }
     int rc = launch_ntt(q, MODE_FWD, S, nullptr, s_hat, r * n, cs);

@@ -380,7 +380,7 @@ size_t emm_pm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int m
 
 int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N,
                   int K, int ldx, int ldy, int mode, bool symmetrize, uint32_t* out,
-                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s) {
+                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s, bool in_round) {
   EmmPmGeometry g;
   if (!emm_pm_geometry(p, M, N, K, mode, &g) || ldx < K || ldx % 4) return GRID_ERR_INVALID_PARAMETERS;
   if (mode != EMM_UPPER && (ldy < K || ldy % 4)) return GRID_ERR_INVALID_PARAMETERS;
@@ -398,7 +398,8 @@ int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, 
   if (rc) return rc;
   // point-major partials [split][e][output] -> coefficients [output][64]
   const int outputs = mode == EMM_UPPER ? M * (M + 1) / 2 : M * N;
-  return launch_sum_inverse(p, work, outputs, g.splits, symmetrize ? M : 0, out, limbs, s);
+  return launch_sum_inverse(p, work, outputs, g.splits, symmetrize ? M : 0, out, limbs, s,
+                            in_round);
 }
 
 }  // namespace grid

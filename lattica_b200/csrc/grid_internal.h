@@ -196,7 +196,7 @@ size_t emm_pm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int m
 // limbs: the outputs' balanced limbs as well (out may then be null).
 int launch_emm_pm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N,
                   int K, int ldx, int ldy, int mode, bool symmetrize, uint32_t* out,
-                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s);
+                  const LimbSpec& limbs, uint32_t* work, cudaStream_t s, bool in_round = false);
 // Row stride of point-major evaluations of rows of n polys: whole 16-byte units.
 inline size_t pm_stride(size_t n) { return (n + 3) / 4 * 4; }
 // in [rows][cols][d] -> out [d][rows][ld], words past cols zero
@@ -206,7 +206,8 @@ int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t rows, size_t
 // transformed, out [output][64]. sym_r > 0: part holds the dense sym_r x sym_r product C
 // and the outputs are the packed upper triangle of (C_ij + C_ji) / 2.
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
-                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s);
+                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s,
+                       bool in_round = false);
 // The least workspace grid_gpu_gram_dev runs in (grid_gpu_gram_workspace: what it runs
 // best in).
 int gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes);

@@ -759,31 +759,35 @@ __global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
 
 // ---------------------------------------------------------------------------
 // The end of a point-major contraction (emm_pm.cu): a CTA sums the K-range partials of
-// 32 outputs point by point (reads along the outputs, 128 bytes per point and
-// split), and eight threads per output run its inverse transform from shared memory.
+// kPolys outputs point by point (reads along the outputs), and eight threads per output
+// run its inverse transform from shared memory. 32 outputs, or 16 where those are few
+// CTAs (up to 1024 outputs: the Gram of r = 30, n = 1021 20.7 us a call with 32, 17.4 with 16;
+// garbage h of r = 64 83.1 and 84.6) and no projection of the prover round competes for
+// the SMs: there more of these CTAs hold up its own (r = 64, n = 2048 490 us with 32, 530 with 16).
 // One launch instead of a transposing sum and a transform of its own, whose 64 KB
 // matrix copy a few hundred polynomials do not pay for; the prover round's balanced
 // limbs come out of the same registers (the Gram of r = 30, n = 1021 went
-// from 41 to 27 us a call with this and the products' byte planes, u1 and u2 of the outer
+// from 41 to 27 us a call with 32 outputs and the products' byte planes, u1 and u2 of the outer
 // commitment at r = 64 from 204 to 130).
 // kSym: output (i, j) is (C_ij + C_ji) / 2 of a dense r x r product (garbage h).
 // ---------------------------------------------------------------------------
-constexpr int kSiPolys = 32;
-constexpr int kSiThreads = kSiPolys * kSmallT;
+constexpr int kSiThreads = 256;
+constexpr int kSiFew = 1024;
 
-template <bool kSym>
+template <bool kSym, int kPolys>
 __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
     const uint32_t* __restrict__ part, int outputs, int splits, int r, uint32_t two_inv,
     uint32_t* __restrict__ out, LimbSpec limbs, const uint2* __restrict__ gtw, FieldParams f) {
   constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2;
-  constexpr int PS = D + 1;  // the 32 outputs of a point fall in distinct banks
+  constexpr int PS = D + 1;  // the outputs of a point fall in distinct banks
   __shared__ uint2 tws[TWN];
-  __shared__ uint32_t sh[kSiPolys * PS];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t sh[kPolys * PS];
+  constexpr int GROUPS = kSiThreads / kPolys;
+  const int tid = threadIdx.x, lane = tid % kPolys, group = tid / kPolys;
   for (int i = tid; i < TWN; i += kSiThreads) tws[i] = gtw[i];
   grid_dep_wait();
   grid_dep_launch();
-  const int o = blockIdx.x * kSiPolys + lane;
+  const int o = blockIdx.x * kPolys + lane;
   const bool valid = o < outputs;
   int at = o, mirror = 0;
   const int width = kSym ? r * r : outputs;  // words per (split, point) of part
@@ -797,16 +801,16 @@ __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
     mirror = j * r + i;
   }
   const size_t stride = (size_t)D * width;
-  // this warp's points warp, warp + 8, ...: the loads of one split are independent
-  constexpr int PTS = D / (kSiThreads / 32);
+  // this group's points group, group + GROUPS, ...: the loads of one split are independent
+  constexpr int PTS = D / GROUPS;
   uint32_t v[PTS] = {};
   if (valid) {
-    const uint32_t* src = part + (size_t)warp * width;
-#pragma unroll 2
+    const uint32_t* src = part + (size_t)group * width;
+#pragma unroll 16 / PTS
     for (int s = 0; s < splits; ++s, src += stride) {
 #pragma unroll
       for (int k = 0; k < PTS; ++k) {
-        const uint32_t* row = src + (size_t)(k * (kSiThreads / 32)) * width;
+        const uint32_t* row = src + (size_t)(k * GROUPS) * width;
         uint32_t w = row[at];
         if (kSym) w = add_mod(w, row[mirror], f.q);
         v[k] = add_mod(v[k], w, f.q);
@@ -815,10 +819,10 @@ __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
   }
 #pragma unroll
   for (int k = 0; k < PTS; ++k)
-    sh[lane * PS + warp + k * (kSiThreads / 32)] =
+    sh[lane * PS + group + k * GROUPS] =
         kSym ? mont_mul(v[k], two_inv, f.q, f.qinv) : v[k];
   __syncthreads();
-  const int pl = tid / T, t = tid % T;
+  const int pl = tid / T % kPolys, t = tid % T;  // of 16 the second half repeats the first
   const int bt_t = brv(4 * t, LOGD);
   const Consts c = consts_of(f);
   uint32_t x[E];
@@ -828,8 +832,8 @@ __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
     x[e] = sh[pl * PS + (brv(i, LOGD) | bt_t)];
   }
   invT_stages<D, T, 1>(x, tws, t, c);
-  const int po = blockIdx.x * kSiPolys + pl;
-  if (po < outputs) {
+  const int po = blockIdx.x * kPolys + pl;
+  if (tid < kPolys * T && po < outputs) {
 #pragma unroll
     for (int m = 0; m < E / 4; ++m) {
       const uint4 v = make_uint4(x[4 * m + 0], x[4 * m + 1], x[4 * m + 2], x[4 * m + 3]);
@@ -988,18 +992,23 @@ int launch_commit_vec(const grid_gpu_plan* p, const VecOperand& o0, const VecOpe
 }
 
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
-                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s) {
+                       int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s,
+                       bool in_round) {
   if (p->d != 64) return GRID_ERR_UNSUPPORTED_DEGREE;
   if (sym_r) outputs = sym_r * (sym_r + 1) / 2;
   if (outputs <= 0) return GRID_OK;
   // (q + 1) / 2 in Montgomery form
   const uint32_t two_inv =
       (uint32_t)(((unsigned __int128)((p->f.q + 1ull) / 2) << 32) % p->f.q);
-  const unsigned grid = (unsigned)((outputs + kSiPolys - 1) / kSiPolys);
-  return sym_r ? launch_chained(sum_inverse_kernel<true>, dim3(grid), kSiThreads, 0, s, part, outputs,
-                                splits, sym_r, two_inv, out, limbs, p->d_tw, p->f)
-               : launch_chained(sum_inverse_kernel<false>, dim3(grid), kSiThreads, 0, s, part,
-                                outputs, splits, 0, two_inv, out, limbs, p->d_tw, p->f);
+  const int polys = outputs <= kSiFew && !in_round ? 16 : 32;
+  const unsigned grid = (unsigned)((outputs + polys - 1) / polys);
+  auto run = [&](auto kernel) {
+    return launch_chained(kernel, dim3(grid), kSiThreads, 0, s, part, outputs, splits, sym_r, two_inv,
+                          out, limbs, p->d_tw, p->f);
+  };
+  if (polys == 16)
+    return sym_r ? run(sum_inverse_kernel<true, 16>) : run(sum_inverse_kernel<false, 16>);
+  return sym_r ? run(sum_inverse_kernel<true, 32>) : run(sum_inverse_kernel<false, 32>);
 }
 
 bool commit_small_fits(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
