@@ -63,6 +63,12 @@ struct Consts {
   uint4 w, wq;  // 2^(8b) 2^32 mod q and companions
 };
 
+// The builder warps' own barrier (named barrier 1; the CTA's is 0).
+__device__ __forceinline__ void builders_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(kBuilders) : "memory");
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
     amortize_tc_kernel(const __grid_constant__ CUtensorMap map_s, const uint32_t* __restrict__ c,
                        uint32_t* __restrict__ out, uint32_t r, uint32_t n, const Consts w,
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       const uint32_t bs = t % NB;
       if (ok && t >= (uint32_t)NB) ok = lane0_wait(&bfree[bs], (t / NB - 1) & 1, lane, err);
-      asm volatile("bar.sync 1, %0;" ::"n"(kBuilders) : "memory");
+      builders_sync();
       if (!ok) continue;  // the other warps still meet at the barrier
       unsigned char* mat = sm + OFF_B + bs * kMat;
       for (int u = tid; u < 4 * kCores * 8; u += kBuilders) {
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           at[0] = make_uint4(z[0], z[1], z[2], z[3]);
           at[1] = make_uint4(z[4], z[5], z[6], z[7]);
         }
+        __syncwarp();  // the whole warp issues the next loads
       }
     }
   }

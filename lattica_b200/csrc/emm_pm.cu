@@ -101,6 +101,7 @@ struct PmShape {
 
 // The builder warps' own barrier (named barrier 1; the CTA's is 0).
 __device__ __forceinline__ void builders_sync() {
+  __syncwarp();
   asm volatile("bar.sync 1, %0;" ::"n"(kPmBuilders) : "memory");
 }
 
@@ -262,15 +263,17 @@ __global__ void __launch_bounds__(kPmThreads)
 #pragma unroll
         for (int c = 0; c < S::NC; ++c) tc::tmem_ld8(taddr + c * NP + n0, ds[c]);
         tc::tmem_ld_wait7(ds);
-        if (m >= M || block >= P) continue;
+        if (m < M && block < P) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int n = n0 + j;
-          if (n >= N || (UPPER && n < m)) continue;
-          const int idx = UPPER ? m * M - (m * (m - 1)) / 2 + (n - m) : m * N + n;
-          stage[block * outputs + idx] = reduce_classes(ds[0][j], ds[1][j], ds[2][j], ds[3][j],
-                                                        ds[4][j], ds[5][j], ds[6][j], f, block);
+          for (int j = 0; j < 8; ++j) {
+            const int n = n0 + j;
+            if (n >= N || (UPPER && n < m)) continue;
+            const int idx = UPPER ? m * M - (m * (m - 1)) / 2 + (n - m) : m * N + n;
+            stage[block * outputs + idx] = reduce_classes(ds[0][j], ds[1][j], ds[2][j], ds[3][j],
+                                                          ds[4][j], ds[5][j], ds[6][j], f, block);
+          }
         }
+        __syncwarp();  // the whole warp issues the next loads
       }
     }
     builders_sync();

@@ -330,15 +330,18 @@ __global__ void __launch_bounds__(kGpThreads, 2)
 #pragma unroll
         for (int c = 0; c < 7; ++c) tc::tmem_ld8(taddr + c * NP + n0, ds[c]);
         tc::tmem_ld_wait7(ds);
-        if (j >= tl.count) continue;
+        if (j < tl.count) {
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const uint32_t n = n0 + jj;
-          if (n >= mrows) continue;
-          atomicAdd(&acc[(toff + n) * (unsigned long long)d + w.eg],
-                    (unsigned long long)reduce_classes(ds[0][jj], ds[1][jj], ds[2][jj], ds[3][jj],
-                                                       ds[4][jj], ds[5][jj], ds[6][jj], f));
+          for (int jj = 0; jj < 8; ++jj) {
+            const uint32_t n = n0 + jj;
+            if (n >= mrows) continue;
+            atomicAdd(&acc[(toff + n) * (unsigned long long)d + w.eg],
+                      (unsigned long long)reduce_classes(ds[0][jj], ds[1][jj], ds[2][jj],
+                                                         ds[3][jj], ds[4][jj], ds[5][jj],
+                                                         ds[6][jj], f));
+          }
         }
+        __syncwarp();  // the whole warp issues the next loads
       }
       tc::fence_before_sync();
       __syncwarp();

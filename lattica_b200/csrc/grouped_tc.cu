@@ -213,20 +213,22 @@ __device__ bool gt_item(const WorkDev& wk, const TileDev& tile, const MatDev& ma
 #pragma unroll
         for (int l = 0; l < 4; ++l) tc::tmem_ld8(taddr + l * NP + n0, eb[l]);
         tc::tmem_ld_wait32(eb);
-        if (m >= M) continue;
+        if (m < M) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int n = n0 + j;
-          if (n >= N || (upper && n < m)) continue;
-          uint64_t v = mad_wide(eb[1][j], 256u, (uint64_t)eb[0][j]);
-          v = mad_wide(eb[2][j], 65536u, v);
-          v = mad_wide(eb[3][j], 16777216u, v);
-          const uint32_t r = redc64(v, k.q, k.qinv);
-          const unsigned long long poly =
-              upper ? rows[0].t_off + (unsigned long long)(m * M - (m * (m - 1)) / 2 + (n - m))
-                    : rows[m].t_off + (unsigned long long)n;
-          atomicAdd(&acc[poly * (unsigned long long)d + e], (unsigned long long)r);
+          for (int j = 0; j < 8; ++j) {
+            const int n = n0 + j;
+            if (n >= N || (upper && n < m)) continue;
+            uint64_t v = mad_wide(eb[1][j], 256u, (uint64_t)eb[0][j]);
+            v = mad_wide(eb[2][j], 65536u, v);
+            v = mad_wide(eb[3][j], 16777216u, v);
+            const uint32_t r = redc64(v, k.q, k.qinv);
+            const unsigned long long poly =
+                upper ? rows[0].t_off + (unsigned long long)(m * M - (m * (m - 1)) / 2 + (n - m))
+                      : rows[m].t_off + (unsigned long long)n;
+            atomicAdd(&acc[poly * (unsigned long long)d + e], (unsigned long long)r);
+          }
         }
+        __syncwarp();  // the whole warp issues the next loads
       }
     }
   }

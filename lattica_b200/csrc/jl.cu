@@ -669,6 +669,7 @@ __global__ void __launch_bounds__(kEvThreads, 1) jl_eval_tc_kernel(
         atomicAdd(&gsum[(size_t)row * kEvD + t0 + k],
                   (unsigned long long)(fold ? (long long)residue(v, q) : v));
       }
+      __syncwarp();
     }
   }
   tc::fence_before_sync();

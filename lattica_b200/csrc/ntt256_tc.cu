@@ -97,6 +97,7 @@ enum Bar : int {
 
 // The warps of a group (named barrier 1 or 2).
 __device__ __forceinline__ void group_sync(int g) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GROUP) : "memory");
 }
 
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(THREADS256, 1)
     // polynomial p at that index with its low 5 bits XORed with p (the 32 lanes hit 32
     // banks, here and where a warp reads 32 consecutive c of one polynomial)
     auto exchange = [&](uint32_t* to) {
+      __syncwarp();
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         uint32_t res[16];
@@ -236,6 +238,7 @@ __global__ void __launch_bounds__(THREADS256, 1)
 #pragma unroll
         for (int t = 0; t < 16; ++t)
           to[p * D + ((64 * aa + 32 * half + 16 * h + t) ^ p)] = res[t];
+        __syncwarp();
       }
       tc::fence_before_sync();
       group_sync(g);

@@ -83,6 +83,7 @@ __device__ __forceinline__ uint32_t sw64(uint32_t row, uint32_t c) {
 // True iff every warp of the group (named barrier id) passes ok.
 __device__ __forceinline__ bool group_all(int id, bool ok) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
       "bar.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -305,6 +306,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             *reinterpret_cast<uint4*>(pp + BOX + off) =
                 make_uint4(z1[4 * c], z1[4 * c + 1], z1[4 * c + 2], z1[4 * c + 3]);
           }
+          __syncwarp();
         }
         if (!ok) break;
         tc::fence_async_smem();
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             tma_store_2d(&tmap_out, (int)(32 * h + 16 * bt), (int)row0(j), smem_addr(st));
             bulk_commit();
           }
+          __syncwarp();
         }
       }
       if (elected) bulk_wait_all();
