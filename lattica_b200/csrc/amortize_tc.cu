@@ -70,7 +70,7 @@ __device__ __forceinline__ void builders_sync() {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    amortize_tc_kernel(const __grid_constant__ CUtensorMap map_s, const uint32_t* __restrict__ c,
+    amortize_tc_kernel(const __grid_constant__ CUtensorMap map_s, const uint32_t* c,
                        uint32_t* __restrict__ out, uint32_t r, uint32_t n, const Consts w,
                        const FieldParams f, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
@@ -162,8 +162,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t next = 0;
     // word e = k' + m of the matrix: c~_(63 - e)
     auto load = [&](uint32_t t) {
-      next = tid < 127 && t < cnt ? __ldg(c + (unsigned long long)(i0 + t) * D + ((127 - tid) & 63))
-                                  : 0u;
+      next = tid < 127 && t < cnt
+                 ? load_dep(c + (unsigned long long)(i0 + t) * D + ((127 - tid) & 63))
+                 : 0u;
     };
     load(0);
     for (uint32_t t = 0; t < cnt; ++t) {
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // z = the sum of the splits' words mod q, four words per thread.
-__global__ void __launch_bounds__(256) amortize_sum_kernel(const uint4* __restrict__ part,
+__global__ void __launch_bounds__(256) amortize_sum_kernel(const uint4* part,
                                                            uint4* __restrict__ z,
                                                            unsigned long long words4, int splits,
                                                            uint32_t q) {
@@ -247,10 +248,10 @@ __global__ void __launch_bounds__(256) amortize_sum_kernel(const uint4* __restri
   grid_dep_wait();
   const unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= words4) return;
-  uint4 a = part[i];
+  uint4 a = load_dep(part + i);
 #pragma unroll 8
   for (int s = 1; s < splits; ++s) {
-    const uint4 b = part[s * words4 + i];
+    const uint4 b = load_dep(part + s * words4 + i);
     a = make_uint4(add_canon(a.x, b.x, q), add_canon(a.y, b.y, q), add_canon(a.z, b.z, q),
                    add_canon(a.w, b.w, q));
   }

@@ -51,6 +51,24 @@ __device__ __forceinline__ void grid_dep_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Loads of what the predecessor in the stream may have written, in a kernel launched with
+// launch_chained: it is resident while that memory changes, so the read-only path (__ldg,
+// or a const __restrict__ parameter that the compiler takes it for) has no claim to it.
+// Volatile, so none is scheduled above grid_dep_wait().
+__device__ __forceinline__ uint32_t load_dep(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ uint4 load_dep(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
 // Plain arrive (release semantics, shared::cta).
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");

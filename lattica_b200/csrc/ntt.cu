@@ -673,7 +673,8 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
 #pragma unroll
       for (int m = 0; m < E / 4; ++m) {
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (pl < n) v = __ldg(reinterpret_cast<const uint4*>(s + (size_t)(k0 + pl) * D) + T * m + t);
+        if (pl < n)
+          v = load_dep(reinterpret_cast<const uint4*>(s + (size_t)(k0 + pl) * D) + T * m + t);
         x[4 * m + 0] = v.x;
         x[4 * m + 1] = v.y;
         x[4 * m + 2] = v.z;
@@ -697,7 +698,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
         for (int i = 0; i < RPT; ++i) {
           const int r = slot + kSmallSlots * i;
           av[i][j] = kk + j < n && r < rows
-                         ? __ldg(p.A + ((size_t)r * p.ld + k0 + kk + j) * D + e)
+                         ? load_dep(p.A + ((size_t)r * p.ld + k0 + kk + j) * D + e)
                          : 0u;
         }
       }
@@ -719,7 +720,7 @@ __global__ void __launch_bounds__(kVecThreads, 2) vec_partial_kernel(
 constexpr int kVfThreads = 512;
 
 __global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
-    const uint32_t* __restrict__ part, int count, int rows, uint32_t* __restrict__ t_out,
+    const uint32_t* part, int count, int rows, uint32_t* __restrict__ t_out,
     const uint2* __restrict__ gtw, FieldParams f) {
   constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2, G = kVfThreads / D;
   __shared__ uint2 tws[TWN];
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(kVfThreads) vec_finish_kernel(
   const uint32_t* src = part + ((size_t)blockIdx.y * count * rows + blockIdx.x) * D + e;
   unsigned long long v = 0;  // count canonical words stay below 2^64
 #pragma unroll 8
-  for (int i = g; i < count; i += G) v += __ldg(src + (size_t)i * rows * D);
+  for (int i = g; i < count; i += G) v += load_dep(src + (size_t)i * rows * D);
   sums[g][e] = v;
   __syncthreads();
   if (g == 0) {
@@ -776,7 +777,7 @@ constexpr int kSiFew = 1024;
 
 template <bool kSym, int kPolys>
 __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
-    const uint32_t* __restrict__ part, int outputs, int splits, int r, uint32_t two_inv,
+    const uint32_t* part, int outputs, int splits, int r, uint32_t two_inv,
     uint32_t* __restrict__ out, LimbSpec limbs, const uint2* __restrict__ gtw, FieldParams f) {
   constexpr int D = 64, LOGD = 6, T = kSmallT, E = D / T, TWN = 2 * D + 2;
   constexpr int PS = D + 1;  // the outputs of a point fall in distinct banks
@@ -811,8 +812,8 @@ __global__ void __launch_bounds__(kSiThreads) sum_inverse_kernel(
 #pragma unroll
       for (int k = 0; k < PTS; ++k) {
         const uint32_t* row = src + (size_t)(k * GROUPS) * width;
-        uint32_t w = row[at];
-        if (kSym) w = add_mod(w, row[mirror], f.q);
+        uint32_t w = load_dep(row + at);
+        if (kSym) w = add_mod(w, load_dep(row + mirror), f.q);
         v[k] = add_mod(v[k], w, f.q);
       }
     }

@@ -96,8 +96,8 @@ __device__ __forceinline__ bool group_all(int id, bool ok) {
 __global__ void __launch_bounds__(THREADS, 1)
     ntt_mul_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
                       const __grid_constant__ CUtensorMap tmap_b,
-                      const __grid_constant__ CUtensorMap tmap_out, const uint32_t* __restrict__ a,
-                      const uint32_t* __restrict__ b, unsigned long long npolys,
+                      const __grid_constant__ CUtensorMap tmap_out, const uint32_t* a,
+                      const uint32_t* b, unsigned long long npolys,
                       const uint4* __restrict__ wtab, const uint4* __restrict__ gtab, const TcConsts k,
                       int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];

@@ -76,9 +76,9 @@ enum Bar : int {
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
     ntt_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                  const __grid_constant__ CUtensorMap tmap_out, const uint32_t* __restrict__ a,
+                  const __grid_constant__ CUtensorMap tmap_out, const uint32_t* a,
                   unsigned long long npolys, const uint4* __restrict__ wtab, const TcConsts k,
-                  int* __restrict__ err, const uint4* __restrict__ ptiles,
+                  int* __restrict__ err, const uint4* ptiles,
                   unsigned long long nptiles, uint32_t row_polys) {
   constexpr bool kPm = MODE == MODE_FWD_PM;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
@@ -136,13 +136,13 @@ __global__ void __launch_bounds__(THREADS, 1)
       const uint32_t t = (uint32_t)tile_index(j);
       return (unsigned long long)(t / row_tiles) * row_polys + (t % row_tiles) * ROWS;
     }
-    return listed ? (unsigned long long)ptiles[tile_index(j)].x : tile_index(j) * ROWS;
+    return listed ? load_dep(&ptiles[tile_index(j)].x) : tile_index(j) * ROWS;
   };
   auto tile_out0 = [&](uint32_t j) -> unsigned long long {
-    return listed ? (unsigned long long)ptiles[tile_index(j)].y : tile_index(j) * ROWS;
+    return listed ? load_dep(&ptiles[tile_index(j)].y) : tile_index(j) * ROWS;
   };
   auto tile_valid = [&](uint32_t j) -> uint32_t {
-    return listed ? ptiles[tile_index(j)].z : (uint32_t)ROWS;
+    return listed ? load_dep(&ptiles[tile_index(j)].z) : (uint32_t)ROWS;
   };
 
   if (warp == LOAD_WARP) {
