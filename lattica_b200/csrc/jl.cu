@@ -22,6 +22,7 @@
 #include "grid_internal.h"
 #include "grid_chacha.cuh"
 #include "grid_tc.cuh"
+#include "jl_units.h"
 
 namespace grid {
 namespace {
@@ -86,7 +87,6 @@ __device__ __forceinline__ void keystream64(const ChachaKey& key, uint32_t nonce
 // Measured at 64 x 131072 columns: 0.51 ms before, 0.42 ms now; with the int8 entries
 // 1.21 ms before, 0.90 ms now.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kUnitCols = 32;                      // columns per unit (K of one MMA)
 constexpr uint32_t kUnitA = 256u * kUnitCols;           // A tile: 256 rows x 32 columns
 constexpr uint32_t kPjB = 16u * kUnitCols;              // B tile: 16 bytes x 32 columns
 constexpr int kGroup = 4;                               // warps per hand-over (mma_loop)
@@ -104,9 +104,6 @@ struct PjShape {
       OFF_BAR + (2 * WARPS / kGroup + 1) * 8 + 32 + 128;  // + alignment slack
   static_assert(SMEM <= 232448 && WARPS % kGroup == 0, "shape");
 };
-// A packed byte is at most 2 (1 + 4 + 16 + 64) = 170, a byte of x 255: 170 * 255 * 2^16
-// stays below 2^32, the accumulators' wrap.
-constexpr unsigned long long kMaxUnitsPerCta = (1ull << 16) / kUnitCols;
 
 // Row m, column k of a unit's A tile: 16-row x 8-column core matrices.
 __device__ __forceinline__ uint32_t unit_a_off(uint32_t m, uint32_t k) {
@@ -677,19 +674,6 @@ __global__ void __launch_bounds__(kEvThreads, 1) jl_eval_tc_kernel(
   if (warp == kEvWarps) tc::tmem_dealloc(tbase, 512);
 }
 
-// Grid of a unit kernel: every SM (or every unit, if fewer), and more CTAs (they
-// queue) where one would accumulate past its bound. False if the units do not fit
-// 32-bit indices.
-bool unit_grid(unsigned long long nunits, int warps, int num_sms, unsigned* grid) {
-  const unsigned long long per_cta = kMaxUnitsPerCta / warps * warps;
-  unsigned long long g =
-      std::max((unsigned long long)num_sms, (nunits + per_cta - 1) / per_cta);
-  g = std::min(g, nunits);
-  if (nunits + g * warps >= (1ull << 32)) return false;
-  *grid = (unsigned)g;
-  return true;
-}
-
 // Signed 64-bit sums over all columns stay exact without a reduction per CTA while
 // columns * 255 * (1 + 2^8 + 2^16 + 2^24) < 2^63.
 bool must_fold(unsigned long long columns) { return columns >= (1ull << 30); }
@@ -724,10 +708,10 @@ int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
     auto run = [&](auto kernel, auto shape, int* cache) -> int {
       using S = decltype(shape);
-      unsigned grid = 0;
-      if (per_part > (0xFFFFFFFFull / num_parts) ||
-          !unit_grid(per_part * num_parts, S::WARPS, num_sms, &grid))
-        return GRID_ERR_INVALID_PARAMETERS;
+      const unsigned grid = per_part <= 0xFFFFFFFFull / num_parts
+                                ? unit_grid(per_part * num_parts, S::WARPS, num_sms)
+                                : 0;
+      if (!grid) return GRID_ERR_INVALID_PARAMETERS;
       int bps = 0;
       const int rc = prepare_kernel(kernel, S::SMEM, S::THREADS, dev, cache, &bps);
       if (rc) return rc;
@@ -784,10 +768,10 @@ int launch_jl_evals(const FieldParams& f, const uint8_t seed[32], size_t rows,
   cudaError_t e = cudaMemsetAsync(gsum, 0, jl_evals_scratch_bytes(), s);
   if (e != cudaSuccess) return cuda_status(e);
   const unsigned long long per_part = cols / kUnitCols;  // d = 64: a whole, even number
-  unsigned grid = 0;
-  if (per_part > (0xFFFFFFFFull / num_parts) ||
-      !unit_grid(per_part * num_parts, kEvWarps, num_sms, &grid))
-    return GRID_ERR_INVALID_PARAMETERS;
+  const unsigned grid = per_part <= 0xFFFFFFFFull / num_parts
+                            ? unit_grid(per_part * num_parts, kEvWarps, num_sms)
+                            : 0;
+  if (!grid) return GRID_ERR_INVALID_PARAMETERS;
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
   static int bps_cache[kMaxDevices] = {};
