@@ -220,12 +220,14 @@ __device__ __forceinline__ bool tiles_free(uint64_t* bar, uint32_t it, int lane,
 // swap bytes (a 4 x 4 transpose: two shuffles, two byte permutes) so that lane
 // 4 g + r holds one row of polynomials 4 g .. 4 g + 3, and the warp's stores fill
 // whole 32-byte sectors of four rows.
-template <bool kWholeBlocks, bool kFlat = false>
+// kMany: parts from part0 on, one of several launches (an instance of its own: with the
+// offset in every projection 64 x 131072 columns took 418 us for 413).
+template <bool kWholeBlocks, bool kFlat = false, bool kMany = false>
 __global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
     const uint32_t* __restrict__ parts, unsigned long long cols, int rows, int packed_len,
     ChachaKey key, uint32_t nunits, uint32_t per_part, uint32_t d, unsigned long long plane,
     int8_t* __restrict__ flat, unsigned long long* __restrict__ gsum, uint32_t q, bool fold,
-    int* __restrict__ err) {
+    int* __restrict__ err, uint32_t part0) {
   using S = PjShape<kFlat>;
   constexpr int WARPS = S::WARPS;
   extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -290,6 +292,7 @@ __global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
     uint32_t bsum[4] = {0, 0, 0, 0};
     uint32_t unit = first(warp);
     uint32_t part = unit / per_part, ci = unit % per_part;
+    if constexpr (kMany) part += part0;
     const uint32_t step_part = stride / per_part, step_ci = stride % per_part;
     uint64_t* grp_full = &full[warp / kGroup];
     uint64_t* grp_empty = &empty[warp / kGroup];
@@ -706,27 +709,36 @@ int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
   if (cols > 0) {
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
+    const unsigned long long step = parts_per_launch(per_part, num_parts);
+    if (!step) return GRID_ERR_INVALID_PARAMETERS;
     auto run = [&](auto kernel, auto shape, int* cache) -> int {
       using S = decltype(shape);
-      const unsigned grid = per_part <= 0xFFFFFFFFull / num_parts
-                                ? unit_grid(per_part * num_parts, S::WARPS, num_sms)
-                                : 0;
-      if (!grid) return GRID_ERR_INVALID_PARAMETERS;
       int bps = 0;
-      const int rc = prepare_kernel(kernel, S::SMEM, S::THREADS, dev, cache, &bps);
-      if (rc) return rc;
-      kernel<<<grid, S::THREADS, S::SMEM, s>>>(
-          parts, cols, (int)rows, packed_len, key, (uint32_t)(per_part * num_parts),
-          (uint32_t)per_part, (uint32_t)d, plane, fused_flat ? flat_out : nullptr, gsum, f.q,
-          must_fold(plane), err);
-      return cuda_status(cudaGetLastError());
+      int rc = prepare_kernel(kernel, S::SMEM, S::THREADS, dev, cache, &bps);
+      for (unsigned long long at = 0; !rc && at < num_parts; at += step) {
+        const unsigned long long nunits =
+            per_part * std::min(step, (unsigned long long)num_parts - at);
+        kernel<<<unit_grid(nunits, S::WARPS, num_sms), S::THREADS, S::SMEM, s>>>(
+            parts, cols, (int)rows, packed_len, key, (uint32_t)nunits, (uint32_t)per_part,
+            (uint32_t)d, plane, fused_flat ? flat_out : nullptr, gsum, f.q, must_fold(plane), err,
+            (uint32_t)at);
+        rc = cuda_status(cudaGetLastError());
+      }
+      return rc;
     };
     static int cache_whole[kMaxDevices] = {}, cache_part[kMaxDevices] = {},
-               cache_flat[kMaxDevices] = {};
-    const int rc = fused_flat ? run(jl_tc_kernel<true, true>, PjShape<true>(), cache_flat)
-                   : packed_len == 64
-                       ? run(jl_tc_kernel<true>, PjShape<false>(), cache_whole)
-                       : run(jl_tc_kernel<false>, PjShape<false>(), cache_part);
+               cache_flat[kMaxDevices] = {}, cache_many[2][kMaxDevices] = {};
+    const PjShape<false> plain;
+    int rc;
+    if (fused_flat)  // 2^31 units' entries fit no memory
+      rc = step < num_parts ? GRID_ERR_INVALID_PARAMETERS
+                            : run(jl_tc_kernel<true, true>, PjShape<true>(), cache_flat);
+    else if (step < num_parts)
+      rc = packed_len == 64 ? run(jl_tc_kernel<true, false, true>, plain, cache_many[1])
+                            : run(jl_tc_kernel<false, false, true>, plain, cache_many[0]);
+    else
+      rc = packed_len == 64 ? run(jl_tc_kernel<true>, plain, cache_whole)
+                            : run(jl_tc_kernel<false>, plain, cache_part);
     if (rc) return rc;
   }
   jl_finish_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(gsum, p_out, (int)rows, f.q);
@@ -768,18 +780,17 @@ int launch_jl_evals(const FieldParams& f, const uint8_t seed[32], size_t rows,
   cudaError_t e = cudaMemsetAsync(gsum, 0, jl_evals_scratch_bytes(), s);
   if (e != cudaSuccess) return cuda_status(e);
   const unsigned long long per_part = cols / kUnitCols;  // d = 64: a whole, even number
-  const unsigned grid = per_part <= 0xFFFFFFFFull / num_parts
-                            ? unit_grid(per_part * num_parts, kEvWarps, num_sms)
-                            : 0;
-  if (!grid) return GRID_ERR_INVALID_PARAMETERS;
+  if (parts_per_launch(per_part, num_parts) < num_parts)  // 2^31 units fit no memory
+    return GRID_ERR_INVALID_PARAMETERS;
+  const unsigned long long nunits = per_part * num_parts;
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_status(e);
   static int bps_cache[kMaxDevices] = {};
   int bps = 0;
   int rc = prepare_kernel(jl_eval_tc_kernel, kEvSmem, kEvThreads, dev, bps_cache, &bps);
   if (rc) return rc;
-  jl_eval_tc_kernel<<<grid, kEvThreads, kEvSmem, s>>>(
-      parts, cols, key, (uint32_t)(per_part * num_parts), (uint32_t)per_part, gsum, f.q,
+  jl_eval_tc_kernel<<<unit_grid(nunits, kEvWarps, num_sms), kEvThreads, kEvSmem, s>>>(
+      parts, cols, key, (uint32_t)nunits, (uint32_t)per_part, gsum, f.q,
       must_fold((unsigned long long)num_parts * cols), err);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e);
   const int n = kEvRows * kEvD;

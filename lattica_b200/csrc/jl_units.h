@@ -14,14 +14,21 @@ constexpr unsigned long long kMaxUnitsPerCta = (1ull << 16) / kUnitCols;
 // accumulate past their bound as many more as fill every SM again. The units are shared
 // out evenly, so a few CTAs in a wave of their own would take as long as all of the first
 // (projection of r = 64, n = 2304, 148 CTAs: 0.46 ms; of n = 2400 0.93 on 151, 0.49 on 296).
-// 0 if the units do not fit 32-bit indices.
+// nunits at most 2^31 (parts_per_launch), so that unit indices fit 32 bits past the last turn.
 inline unsigned unit_grid(unsigned long long nunits, int warps, int num_sms) {
   const unsigned long long sms = (unsigned long long)num_sms;
   const unsigned long long per_cta = kMaxUnitsPerCta / warps * warps;
   const unsigned long long need = (nunits + per_cta - 1) / per_cta;
   const unsigned long long all = (need + sms - 1) / sms * sms;
-  const unsigned long long g = all < nunits ? all : nunits;
-  return nunits + g * warps < (1ull << 32) ? (unsigned)g : 0u;
+  return (unsigned)(all < nunits ? all : nunits);
+}
+
+// Parts of per_part units that one launch takes (billions of short parts take several);
+// 0 if a single part is too long.
+inline unsigned long long parts_per_launch(unsigned long long per_part,
+                                           unsigned long long num_parts) {
+  const unsigned long long fit = (1ull << 31) / per_part;
+  return fit < num_parts ? fit : num_parts;
 }
 
 }  // namespace grid
