@@ -59,6 +59,30 @@ __device__ __forceinline__ void keystream64(const ChachaKey& key, uint32_t nonce
   }
 }
 
+// Keystream bytes [off, off + len), len <= 64, in a loop over one or two blocks, the second
+// only where the bytes reach into it. With both written out, always, the projection of
+// 64 x 65536 columns took 524 us for 128 rows and 656 for 200, 228 and 382 so, and
+// 16 x 32768 columns of 4 rows 85 us (79 with more CTAs per SM), 40 so. In jl_flat_kernel
+// the stores lose more than the keystream gains (64 x 153600 columns of 200 rows 2.5 ms
+// there, 3.6 so): it keeps keystream64.
+__device__ __forceinline__ void keystream_bytes(const ChachaKey& key, uint32_t nonce0,
+                                                uint64_t off, int len, uint32_t (&w)[16]) {
+  const uint32_t blk = (uint32_t)(off >> 6);
+  const uint32_t sh = (uint32_t)(off & 63);
+  const int blocks = sh + (uint32_t)len > 64 ? 2 : 1;
+  uint32_t buf[32] = {};  // in local memory: shifted by a variable number of bytes
+#pragma unroll 1
+  for (int b = 0; b < blocks; ++b) {
+    uint32_t o[16];
+    chacha20_block(key, blk + b, nonce0, o);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) buf[16 * b + i] = o[i];
+  }
+  const uint32_t ws = sh >> 2, bs = (sh & 3) * 8;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i] = __funnelshift_r(buf[i + ws], buf[i + ws + 1], bs);
+}
+
 // ---------------------------------------------------------------------------
 // Tensor-core projection. A producer warp takes a unit of 32 columns of one
 // part: lane l computes the keystream of its column and writes the column's 256
@@ -320,7 +344,7 @@ __global__ void __launch_bounds__(PjShape<kFlat>::THREADS, 1) jl_tc_kernel(
         if constexpr (kWholeBlocks)
           chacha20_block(key, (uint32_t)c, part, w);
         else
-          keystream64(key, part, c * (unsigned long long)packed_len, w);
+          keystream_bytes(key, part, c * (unsigned long long)packed_len, packed_len, w);
       } else {
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = 0xFFFFFFFFu;  // padding column: x = 0
