@@ -25,8 +25,9 @@
 // the splits. Bound: the MMAs (1536 cycles a step of 0.8 us), at small sizes the chain of
 // launch, first load, steps and reduction. r = 64, n = 2048: 52 us a call with the
 // transforms of s and c, the products per point and the inverse, 20 now; n = 100000: 1372
-// and 470; r = 6, n = 100: 35 and 19; r = 3, n = 100000: 131 and 47. Plans without the
-// tensor-core transform, r > 4096 and more than 2^31 polys keep the chain of transforms.
+// and 470; r = 6, n = 100: 35 and 19; r = 3, n = 100000: 131 and 47. r = 5000, n = 10: 650 to 730
+// us with the chain, one thread a word over all i, 76 now. Plans without the tensor-core
+// transform and more than 2^31 polys keep the chain of transforms.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -52,6 +53,7 @@ constexpr int NA = 4, NB = 3;                // tiles of s, matrices
 constexpr int kCores = 30;                   // per plane
 constexpr uint32_t kPlane = kCores * 128, kMat = 4 * kPlane;
 constexpr int kMaxSum = 64;                  // i per CTA: 64 * 2^24 stays below 2^31
+constexpr size_t kMaxR = 65535u * kMaxSum;   // splits in the grid's second dimension
 constexpr uint32_t OFF_B = NA * TILE;
 constexpr uint32_t OFF_T = OFF_B + NB * kMat;          // [2][4 planes][128] words by k' + m
 constexpr uint32_t OFF_BAR = OFF_T + 2 * 4 * 128 * 4;
@@ -278,7 +280,7 @@ int amortize_tc_splits(size_t r, size_t n, int num_sms) {
 }
 
 bool amortize_tc_fits(const grid_gpu_plan* p, size_t r, size_t n) {
-  return ntt_tc_available(p) && r <= 4096 && r * n <= (size_t)INT32_MAX - ROWS;
+  return ntt_tc_available(p) && r <= kMaxR && r * n <= (size_t)INT32_MAX - ROWS;
 }
 
 // part: r x n polys of scratch.
