@@ -310,10 +310,15 @@ int launch_amortize_tc(const grid_gpu_plan* p, const uint32_t* S, const uint32_t
   w.w = make_uint4(x[0], x[1], x[2], x[3]);
   w.wq = make_uint4(xq[0], xq[1], xq[2], xq[3]);
   const int splits = amortize_tc_splits(r, n, p->num_sms);
+  // z may lie over s or c: CTAs still read those while the first ones store
+  auto over = [&](const uint32_t* x, size_t polys) {
+    return z < x + polys * D && x < z + n * D;
+  };
+  const bool direct = splits == 1 && !over(S, r * n) && !over(c, r);
   const unsigned tiles = (unsigned)((n + ROWS - 1) / ROWS);
   rc = launch_chained(amortize_tc_kernel, dim3(tiles, (unsigned)splits), kThreads, SMEM, s, map, c,
-                      splits > 1 ? part : z, (uint32_t)r, (uint32_t)n, w, p->f, p->d_err);
-  if (rc || splits == 1) return rc;
+                      direct ? z : part, (uint32_t)r, (uint32_t)n, w, p->f, p->d_err);
+  if (rc || direct) return rc;
   const unsigned long long words4 = (unsigned long long)n * (D / 4);
   return launch_chained(amortize_sum_kernel, dim3((unsigned)((words4 + 255) / 256)), 256, 0, s,
                         reinterpret_cast<const uint4*>(part), reinterpret_cast<uint4*>(z), words4,
