@@ -86,13 +86,20 @@ bool square_dims_ok(const grid_gpu_plan* p, size_t r, size_t n) {
 }
 
 // The evaluations of matrix m (plan, shape and ld set) from A, and, where products on
-// the TMA-fed tensor-core kernel apply, their point-major copy in the same allocation.
+// the TMA-fed tensor-core kernel apply, their point-major copy in the same allocation
+// (left out where memory holds the evaluations alone: products gather those then).
 int prepare_evals(grid_gpu_matrix* m, const uint32_t* A, bool a_is_evals, cudaStream_t st) {
   const grid_gpu_plan* p = m->plan;
   const size_t polys = m->rows * m->cols, words = polys * p->d;
-  const bool pm = pm_fits(p, 1, m->rows, m->cols, EMM_DENSE);
+  bool pm = pm_fits(p, 1, m->rows, m->cols, EMM_DENSE);
   const size_t part = words_bytes(words), ld = pm_stride(m->cols);
-  int rc = cuda_status(cudaMalloc(&m->d_evals, pm ? part + m->rows * ld * p->d * 4 : words * 4));
+  cudaError_t e = cudaMalloc(&m->d_evals, pm ? part + m->rows * ld * p->d * 4 : words * 4);
+  if (pm && e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();  // or the next launch's check would report it
+    pm = false;
+    e = cudaMalloc(&m->d_evals, words * 4);
+  }
+  int rc = cuda_status(e);
   if (rc) return rc;
   if (a_is_evals)
     rc = cuda_status(cudaMemcpyAsync(m->d_evals, A, words * 4, cudaMemcpyDeviceToDevice, st));
