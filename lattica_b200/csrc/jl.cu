@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kJlThreads) jl_flat_kernel(unsigned long long 
   const unsigned long long total = (unsigned long long)num_parts * d * jchunks;
   const unsigned long long plane = (unsigned long long)num_parts * cols;  // bytes per row
   const unsigned long long stride = (unsigned long long)gridDim.x * kJlWarps;
-  const bool vec_ok = (n % 4) == 0;
+  const bool vec_ok = (n % 4) == 0 && (reinterpret_cast<uintptr_t>(flat) & 3u) == 0;
   for (unsigned long long wk = (unsigned long long)blockIdx.x * kJlWarps + warp; wk < total;
        wk += stride) {
     const unsigned long long jc = wk % jchunks;
