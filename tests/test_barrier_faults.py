@@ -84,12 +84,17 @@ PROTOCOLS = {
 IMPLIED = {("grouped", "mma", "FULL"), ("product256", "loader", "XFREE")}
 
 
-class Late(random.Random):
-    """Copies and MMAs finish late more often than the roles take a step."""
+class Uneven(random.Random):
+    """Interleavings in which copies and MMAs finish late, or one role falls behind."""
+
+    def new_run(self, roles):
+        self.late, self.slow = self.random() < 0.5, self.randrange(2 * roles)
 
     def choice(self, seq):
-        steps = [c for c in seq if c[0] == "role"]
-        return super().choice(steps if steps and self.random() < 0.8 else seq)
+        if self.random() < 0.9:
+            few = [c for c in seq if (c[0] == "role" if self.late else c != ("role", self.slow))]
+            seq = few or seq
+        return super().choice(seq)
 
 
 def _waits(name):
@@ -102,20 +107,21 @@ def _waits(name):
 
 @pytest.mark.parametrize("name,role,bar", [(n, r, b) for n in PROTOCOLS for r, b in _waits(n)])
 def test_every_wait_is_needed(name, role, bar):
-    rngs = random.Random(len(bar)), Late(len(bar))
+    rng = Uneven(len(bar))
 
     def without(ops):
         return (op for op in ops if not (op[0] == "wait" and op[1].rstrip("0123456789") == bar))
     with pytest.raises(AssertionError):
-        for i in range(800):
+        for _ in range(800):
             counts, roles = PROTOCOLS[name]()
-            Model(counts, rngs[i % 2]).run([without(r) if r.__name__ == role else r
-                                            for r in roles])
+            rng.new_run(len(roles))
+            Model(counts, rng).run([without(r) if r.__name__ == role else r for r in roles])
 
 
 @pytest.mark.parametrize("name", PROTOCOLS)
-def test_whole_protocols_pass_with_late_completions(name):
-    rng = Late(1)
+def test_whole_protocols_pass_uneven_runs(name):
+    rng = Uneven(1)
     for _ in range(200):
         counts, roles = PROTOCOLS[name]()
+        rng.new_run(len(roles))
         Model(counts, rng).run(roles)
