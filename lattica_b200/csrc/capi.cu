@@ -63,7 +63,7 @@ size_t round_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa, 
   const size_t e2 = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
   const size_t base = words_bytes(r * pm_stride(n) * d) + words_bytes(e1 > e2 ? e1 : e2) +
                       words_bytes(r * kappa * d) +
-                      round_up(jl_scratch_bytes(jl_rows ? jl_rows : 1, 0, 0), 256);
+                      round_up(jl_scratch_bytes(jl_rows ? jl_rows : 1), 256);
   return is_crt(p) ? base + 3 * (words_bytes(r * kappa * d) + words_bytes(r * (r + 1) / 2 * d))
                    : base;
 }
@@ -745,7 +745,7 @@ int grid_gpu_amortize(grid_gpu_plan* p, const uint32_t* S, const uint32_t* c, si
 
 int grid_gpu_jl_workspace(size_t rows, size_t* bytes) {
   if (!bytes) return GRID_ERR_NULL_POINTER;
-  *bytes = round_up(jl_scratch_bytes(rows, 0, 0), 256);
+  *bytes = round_up(jl_scratch_bytes(rows), 256);
   return GRID_OK;
 }
 
@@ -766,7 +766,7 @@ int grid_gpu_jl_project(grid_gpu_plan* p, const uint8_t* seed, size_t rows,
   if (rows == 0 || rows > 256 || d == 0 || cols % d) return GRID_ERR_INVALID_PARAMETERS;
   std::lock_guard<std::mutex> lk(p->mu);
   const size_t in_bytes = num_parts * cols * 4, flat_bytes = flat_out ? rows * num_parts * cols : 0;
-  const size_t ws = round_up(jl_scratch_bytes(rows, 0, 0), 256);
+  const size_t ws = round_up(jl_scratch_bytes(rows), 256);
   int rc;
   if ((rc = ensure_scratch(p, 6, in_bytes ? in_bytes : 16)) ||
       (rc = ensure_scratch(p, 7, rows * 4)) || (rc = ensure_scratch(p, 8, ws)) ||
@@ -971,7 +971,7 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
   const size_t ew = e1 > e2 ? e1 : e2;
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   uint32_t* t = cv.take<uint32_t>(r * kappa * d);
-  void* jl_ws = cv.take<char>(jl_scratch_bytes(jl_rows ? jl_rows : 1, 0, 0));
+  void* jl_ws = cv.take<char>(jl_scratch_bytes(jl_rows ? jl_rows : 1));
   // ring plan without an NTT for q: t and g per auxiliary prime
   const size_t tw = r * kappa * d, gw = r * (r + 1) / 2 * d;
   uint32_t *tj[3] = {}, *gj[3] = {};
@@ -1028,7 +1028,7 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
     // 3. JL projection of the coefficient vectors (one part per witness vector)
     if (jl)
       rc_jl = launch_jl_project(p->f, jl_seed, jl_rows, S, r, n * d, d, p_out, jl_flat, jl_ws,
-                                jl_scratch_bytes(jl_rows, 0, 0), p->num_sms, p->d_err, lo);
+                                jl_scratch_bytes(jl_rows), p->num_sms, p->d_err, lo);
     // 1. inner commitments t_i = A s_i and 2. garbage g_ij = <s_i, s_j>, i <= j, with
     // the balanced limbs of both (inner_commit_decomposed, decompose_polys)
     auto spec = [](uint32_t* out, uint64_t base, size_t limbs) {

@@ -24,10 +24,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
                : "memory");
 }
 
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -165,15 +161,6 @@ __device__ __forceinline__ void bulk_wait_read_older() {
 // Wait until this thread's committed bulk stores are complete.
 __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-
-// Per-thread 16-byte global -> shared copy (L2 only); src_bytes < 16 zero-fills
-// the rest (0 reads nothing). Both addresses 16-byte aligned.
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem,
-                                           uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst_smem)),
-               "l"(src_gmem), "r"(src_bytes)
-               : "memory");
 }
 
 // Per-thread 8-byte global -> shared copy (through L1); src_bytes < 8 zero-fills

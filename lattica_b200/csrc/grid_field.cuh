@@ -28,16 +28,6 @@ __device__ __forceinline__ uint32_t mont_mul(uint32_t a, uint32_t b, uint32_t q,
   return hi < u ? r + q : r;
 }
 
-// Multiply by a fixed constant w < q with precomputed wq = w * q^-1 mod 2^32
-// (saves the low product: m = a*w*q^-1 = a*wq mod 2^32).
-__device__ __forceinline__ uint32_t mont_mul_c(uint32_t a, uint32_t w, uint32_t wq, uint32_t q) {
-  const uint32_t hi = __umulhi(a, w);
-  const uint32_t m = a * wq;
-  const uint32_t u = __umulhi(m, q);
-  const uint32_t r = hi - u;
-  return hi < u ? r + q : r;
-}
-
 // (a + b) mod q for canonical a, b (works for q up to 2^32 - 1: computes
 // a - (q - b) and adds q back on borrow).
 __device__ __forceinline__ uint32_t add_mod(uint32_t a, uint32_t b, uint32_t q) {

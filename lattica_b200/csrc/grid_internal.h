@@ -41,7 +41,6 @@ enum NttMode : int {
   MODE_FWD = 0,     // coefficients -> twisted evaluations (natural order)
   MODE_INV = 1,     // twisted evaluations -> coefficients
   MODE_MULINV = 2,  // out = INTT(NTT(a) (.) b_evals)
-  MODE_POLYMUL = 3, // out = INTT(NTT(a) (.) NTT(b))  (negacyclic product)
   MODE_FWD_PM = 4,  // MODE_FWD stored point-major (launch_ntt_tc_pm, d = 64 tensor cores)
 };
 
@@ -236,7 +235,7 @@ int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
                       const uint32_t* parts, size_t num_parts, size_t cols, size_t d,
                       uint32_t* p_out, int8_t* flat_out, void* scratch, size_t scratch_bytes,
                       int num_sms, int* d_err, cudaStream_t s);
-size_t jl_scratch_bytes(size_t rows, size_t num_parts, int num_sms);
+size_t jl_scratch_bytes(size_t rows);
 // crs.cu: `count` uniform Montgomery words from ChaCha20Rng(seed) (accept_max 0:
 // the reference's rejection threshold).
 size_t sample_uniform_workspace_bytes(uint32_t q, unsigned long long count,

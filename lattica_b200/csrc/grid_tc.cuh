@@ -16,12 +16,6 @@
 namespace grid {
 namespace tc {
 
-// Byte offset of (row, 16-byte chunk) in the K-major no-swizzle layout.
-__host__ __device__ constexpr uint32_t core_offset(uint32_t row, uint32_t chunk, uint32_t lbo,
-                                                   uint32_t sbo) {
-  return (row >> 3) * sbo + chunk * lbo + (row & 7u) * 16u;
-}
-
 // Shared-memory matrix descriptor: start address, leading (K) and stride
 // (8-row) byte offsets, all in 16-byte units; descriptor version 1 (bits
 // 46-47), no swizzle (bits 61-63 = 0), base offset 0.
@@ -162,18 +156,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[N]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
-}
-
-// Wait for this thread's tensor-memory loads, naming the 16 registers they
-// fill so that no use of them can be scheduled above the wait.
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[4][4]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[1][0]),
-                 "+r"(r[1][1]), "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[2][0]), "+r"(r[2][1]),
-                 "+r"(r[2][2]), "+r"(r[2][3]), "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]),
-                 "+r"(r[3][3])
-               :
-               : "memory");
 }
 
 }  // namespace tc

@@ -707,7 +707,7 @@ bool must_fold(unsigned long long columns) { return columns >= (1ull << 30); }
 
 }  // namespace
 
-size_t jl_scratch_bytes(size_t rows, size_t, int) { return 2 * rows * sizeof(unsigned long long); }
+size_t jl_scratch_bytes(size_t rows) { return rows * sizeof(unsigned long long); }
 
 int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
                       const uint32_t* parts, size_t num_parts, size_t cols, size_t d,
@@ -716,7 +716,7 @@ int launch_jl_project(const FieldParams& f, const uint8_t seed[32], size_t rows,
   if (rows == 0 || rows > 256 || d == 0 || cols % d != 0 || num_parts == 0 ||
       num_parts > 0xFFFFFFFFull)
     return GRID_ERR_INVALID_PARAMETERS;
-  if (scratch_bytes < jl_scratch_bytes(rows, num_parts, num_sms)) return GRID_ERR_INVALID_PARAMETERS;
+  if (scratch_bytes < jl_scratch_bytes(rows)) return GRID_ERR_INVALID_PARAMETERS;
   const ChachaKey key = chacha::make_key(seed);
   const int packed_len = (int)((rows + 3) / 4);
   unsigned long long* gsum = static_cast<unsigned long long*>(scratch);

@@ -202,17 +202,5 @@ __device__ __forceinline__ bool lane0_wait(uint64_t* bar, uint32_t parity, int l
   return __shfl_sync(0xffffffffu, ok, 0);
 }
 
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err) {
-  const bool ok = mbar_wait_sleep(bar, parity, err);
-  return __all_sync(0xffffffffu, ok);
-}
-
-// The epilogue's waits on MMA results are on the critical path: poll
-// without a suspend hint.
-__device__ __forceinline__ bool warp_wait_fast(uint64_t* bar, uint32_t parity, int* err) {
-  const bool ok = mbar_wait(bar, parity, err);
-  return __all_sync(0xffffffffu, ok);
-}
-
 }  // namespace tcx
 }  // namespace grid
