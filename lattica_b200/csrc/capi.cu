@@ -21,33 +21,61 @@ bool pm_fits(const grid_gpu_plan* p, size_t M, size_t N, size_t K, int mode) {
   return ntt_tc_available(p) && emm_pm_geometry(p, (int)M, (int)N, (int)K, mode, &g);
 }
 
+// The plan whose products a call runs: p, or the first auxiliary prime's (all alike).
+const grid_gpu_plan* residue_plan(const grid_gpu_plan* p) { return is_crt(p) ? p->crt[0] : p; }
+
+// Evaluations of rows of n polys and the products' partials on plan e: for the point-major
+// products (and the gathering ones, should a matrix lack its copy), or those alone.
+struct EvalsLayout {
+  const grid_gpu_plan* e;
+  bool pm;
+  size_t stride;  // polys per row
+  EvalsLayout(const grid_gpu_plan* plan, bool point_major, size_t n)
+      : e(plan), pm(point_major), stride(point_major ? pm_stride(n) : n) {}
+  size_t work(size_t M, size_t N, size_t K, int mode) const {
+    return pm ? emm_workspace_words(e, (int)M, (int)N, (int)K, mode)
+              : emm_gather_words(e, (int)M, (int)N, (int)K, mode);
+  }
+};
+
 // Workspace layouts. On a ring plan without an NTT for q (is_crt) a call runs the
 // prime's own call for each auxiliary prime in turn, on the inputs as they are (the
 // forward transforms reduce any 32-bit words, ring_crt.cu) and in the same workspace,
 // and keeps the three residue results; the reconstruction writes the output.
+//
+// The sizes are what a call runs best in. One that is given less runs by the gathering
+// products if those fit (point-major rows are padded to whole 16-byte units and have more
+// K ranges, the vector products a partial per CTA): a caller may size its workspace for the
+// largest of several shapes.
 size_t commit_ws_bytes(const grid_gpu_plan* p, size_t rows, size_t cols, size_t batch) {
   if (is_crt(p))
     return 3 * words_bytes(batch * rows * p->d) + commit_ws_bytes(p->crt[0], rows, cols, batch);
   if (commit_small_fits(p, rows, cols, batch)) return 0;  // one launch, no intermediate
   if (commit_vec_fits(p, rows, cols, batch))
     return words_bytes(commit_vec_words(p, rows, cols, 0, batch));
-  return words_bytes(batch * pm_stride(cols) * p->d) +
-         words_bytes(emm_workspace_words(p, (int)batch, (int)rows, (int)cols, EMM_DENSE));
+  const EvalsLayout l(p, true, cols);
+  return words_bytes(batch * l.stride * p->d) +
+         words_bytes(l.work(batch, rows, cols, EMM_DENSE));
 }
 
-// stride: polys per witness row of the evaluations (pm_stride(n), or n where only the
-// gathering products are to fit)
-size_t gram_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t stride) {
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
-  const size_t base = words_bytes(r * stride * p->d) +
-                      words_bytes(emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER));
+bool gram_pm(const grid_gpu_plan* p, size_t r, size_t n) {
+  return pm_fits(residue_plan(p), r, r, n, EMM_UPPER);
+}
+
+size_t gram_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, bool pm) {
+  const EvalsLayout l(residue_plan(p), pm, n);
+  const size_t base = words_bytes(r * l.stride * p->d) + words_bytes(l.work(r, r, n, EMM_UPPER));
   return is_crt(p) ? base + 3 * words_bytes(r * (r + 1) / 2 * p->d) : base;
 }
 
-size_t garbage_h_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n) {
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
-  const size_t base = 2 * words_bytes(r * pm_stride(n) * p->d) + words_bytes(r * r * p->d) +
-                      words_bytes(emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_DENSE));
+bool garbage_h_pm(const grid_gpu_plan* p, size_t r, size_t n) {
+  return pm_fits(residue_plan(p), r, r, n, EMM_DENSE);
+}
+
+size_t garbage_h_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, bool pm) {
+  const EvalsLayout l(residue_plan(p), pm, n);
+  const size_t base = 2 * words_bytes(r * l.stride * p->d) + words_bytes(r * r * p->d) +
+                      words_bytes(l.work(r, r, n, EMM_DENSE));
   return is_crt(p) ? base + 3 * words_bytes(r * r * p->d) : base;
 }
 
@@ -56,12 +84,22 @@ size_t amortize_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n) {
   return is_crt(p) ? base + 3 * words_bytes(n * p->d) : base;
 }
 
-size_t round_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa, size_t jl_rows) {
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
+bool round_pm(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa) {
+  const grid_gpu_plan* e = residue_plan(p);
+  return pm_fits(e, r, kappa, n, EMM_DENSE) && pm_fits(e, r, r, n, EMM_UPPER);
+}
+
+// Partials of the round's two products, one after the other.
+size_t round_work(const EvalsLayout& l, size_t r, size_t n, size_t kappa) {
+  const size_t t = l.work(r, kappa, n, EMM_DENSE), g = l.work(r, r, n, EMM_UPPER);
+  return t > g ? t : g;
+}
+
+size_t round_ws_bytes(const grid_gpu_plan* p, size_t r, size_t n, size_t kappa, size_t jl_rows,
+                      bool pm) {
   const size_t d = p->d;
-  const size_t e1 = emm_workspace_words(e, (int)r, (int)kappa, (int)n, EMM_DENSE);
-  const size_t e2 = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
-  const size_t base = words_bytes(r * pm_stride(n) * d) + words_bytes(e1 > e2 ? e1 : e2) +
+  const EvalsLayout l(residue_plan(p), pm, n);
+  const size_t base = words_bytes(r * l.stride * d) + words_bytes(round_work(l, r, n, kappa)) +
                       words_bytes(r * kappa * d) +
                       round_up(jl_scratch_bytes(jl_rows ? jl_rows : 1), 256);
   return is_crt(p) ? base + 3 * (words_bytes(r * kappa * d) + words_bytes(r * (r + 1) / 2 * d))
@@ -140,25 +178,32 @@ int commit_core(const grid_gpu_matrix* A, const uint32_t* s, size_t batch, uint3
   }
   if (commit_small_fits(p, A->rows, A->cols, batch))
     return launch_commit_small(p, A->d_evals, A->rows, A->cols, A->ld, s, batch, t, st);
+  const Carver given = cv;
   if (commit_vec_fits(p, A->rows, A->cols, batch)) {
     uint32_t* part = cv.take<uint32_t>(commit_vec_words(p, A->rows, A->cols, 0, batch));
-    if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-    return launch_commit_vec(p, VecOperand{A->d_evals, s, A->cols, A->ld}, nullptr, A->rows, batch,
-                             t, part, st);
+    if (cv.ok)
+      return launch_commit_vec(p, VecOperand{A->d_evals, s, A->cols, A->ld}, nullptr, A->rows,
+                               batch, t, part, st);
+    cv = given;
   }
-  const size_t ldx = pm_stride(A->cols);
-  uint32_t* s_hat = cv.take<uint32_t>(batch * ldx * p->d);
-  const size_t ew = emm_workspace_words(p, (int)batch, (int)A->rows, (int)A->cols, EMM_DENSE);
+  if (A->d_evals_pm && pm_fits(p, batch, A->rows, A->cols, EMM_DENSE)) {
+    const size_t ldx = pm_stride(A->cols);
+    uint32_t* s_hat = cv.take<uint32_t>(batch * ldx * p->d);
+    uint32_t* work = cv.take<uint32_t>(
+        emm_pm_workspace_words(p, (int)batch, (int)A->rows, (int)A->cols, EMM_DENSE));
+    if (cv.ok) {
+      const int rc = launch_ntt_tc_pm(p, s, batch, A->cols, s_hat, st);
+      if (rc) return rc;
+      return launch_emm_pm(p, s_hat, A->d_evals_pm, (int)batch, (int)A->rows, (int)A->cols,
+                           (int)ldx, (int)A->ld_pm, EMM_DENSE, false, t, LimbSpec(), work, st);
+    }
+    cv = given;
+  }
+  uint32_t* s_hat = cv.take<uint32_t>(batch * A->cols * p->d);
+  const size_t ew = emm_gather_words(p, (int)batch, (int)A->rows, (int)A->cols, EMM_DENSE);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-  int rc;
-  if (A->d_evals_pm && pm_fits(p, batch, A->rows, A->cols, EMM_DENSE)) {
-    rc = launch_ntt_tc_pm(p, s, batch, A->cols, s_hat, st);
-    if (rc) return rc;
-    return launch_emm_pm(p, s_hat, A->d_evals_pm, (int)batch, (int)A->rows, (int)A->cols, (int)ldx,
-                         (int)A->ld_pm, EMM_DENSE, false, t, LimbSpec(), work, st);
-  }
-  rc = launch_ntt(p, MODE_FWD, s, nullptr, s_hat, batch * A->cols, st);
+  int rc = launch_ntt(p, MODE_FWD, s, nullptr, s_hat, batch * A->cols, st);
   if (!rc)
     rc = launch_emm(p, s_hat, A->d_evals, (int)batch, (int)A->rows, (int)A->cols, (int)A->ld,
                     EMM_DENSE, t, work, st);
@@ -171,14 +216,17 @@ int linear_core(const grid_gpu_matrix* A, const grid_gpu_matrix* B, const uint32
                 const uint32_t* r, size_t batch, uint32_t* t, uint32_t* t2, Carver& cv,
                 cudaStream_t st) {
   const grid_gpu_plan* p = A->plan;
+  const Carver given = cv;
   if (linear_vec_fits(A, B, batch)) {
     uint32_t* part = cv.take<uint32_t>(commit_vec_words(p, A->rows, A->cols, B->cols, batch));
-    if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
     const VecOperand second{B->d_evals, r, B->cols, B->ld};
-    return launch_commit_vec(p, VecOperand{A->d_evals, m, A->cols, A->ld}, &second, A->rows, batch,
-                             t, part, st);
+    if (cv.ok)
+      return launch_commit_vec(p, VecOperand{A->d_evals, m, A->cols, A->ld}, &second, A->rows,
+                               batch, t, part, st);
+    cv = given;
   }
   int rc = commit_core(A, m, batch, t, cv, st);
+  cv = given;  // the second product reuses the first one's workspace
   if (!rc) rc = commit_core(B, r, batch, t2, cv, st);
   // A_msg*m + A_open*r: INTT is linear, so adding the coefficient forms is exact.
   if (!rc) rc = launch_add(p, t, t2, batch * B->rows * p->d, st);
@@ -197,7 +245,7 @@ size_t linear_ws_bytes(const grid_gpu_matrix* A, const grid_gpu_matrix* B, size_
 int grid::gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes) {
   if (!p || !bytes) return GRID_ERR_NULL_POINTER;
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
-  *bytes = gram_ws_bytes(p, r, n, n);
+  *bytes = gram_ws_bytes(p, r, n, false);
   return GRID_OK;
 }
 
@@ -453,7 +501,9 @@ int grid_gpu_bdlop_commit_dev(const grid_gpu_matrix* A_mask, const grid_gpu_matr
   Carver cv(workspace, workspace_bytes);
   uint32_t* t2 = cv.take<uint32_t>(batch * A_open->rows * p->d);
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
+  const Carver given = cv;
   int rc = commit_core(A_mask, r, batch, u, cv, st);
+  cv = given;
   if (!rc) rc = linear_core(A_msg, A_open, m, r, batch, v, t2, cv, st);
   return rc;
 }
@@ -503,7 +553,7 @@ int grid_gpu_bdlop_commit(grid_gpu_matrix* A_mask, grid_gpu_matrix* A_msg, grid_
 int grid_gpu_gram_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes) {
   if (!p || !bytes) return GRID_ERR_NULL_POINTER;
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
-  *bytes = gram_ws_bytes(p, r, n, pm_stride(n));
+  *bytes = gram_ws_bytes(p, r, n, true);
   return GRID_OK;
 }
 
@@ -514,15 +564,13 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
   if (!aligned16(S) || !aligned16(G) || !aligned16(workspace)) return GRID_ERR_MISALIGNED;
   cudaStream_t st = (cudaStream_t)stream;
   if (is_crt(p) && !crt_bound_ok(p, n)) return GRID_ERR_INVALID_PARAMETERS;
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
   const size_t gw = r * (r + 1) / 2 * p->d;
-  // rows of whole 16-byte units where they fit the workspace (a caller with a fixed
-  // buffer may have room for the gathering products' layout only)
-  const bool padded = workspace_bytes >= gram_ws_bytes(p, r, n, pm_stride(n));
-  const size_t ldx = padded ? pm_stride(n) : n;
+  const bool pm = gram_pm(p, r, n) && workspace_bytes >= gram_ws_bytes(p, r, n, true);
+  const EvalsLayout l(residue_plan(p), pm, n);
+  const size_t ldx = l.stride;
   Carver cv(workspace, workspace_bytes);
   uint32_t* s_hat = cv.take<uint32_t>(r * ldx * p->d);
-  const size_t ew = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
+  const size_t ew = l.work(r, r, n, EMM_UPPER);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   uint32_t* gj[3] = {};
   if (is_crt(p))
@@ -532,7 +580,7 @@ int grid_gpu_gram_dev(const grid_gpu_plan* p, const uint32_t* S, size_t r, size_
   for (int j = 0; j < (is_crt(p) ? 3 : 1) && !rc; ++j) {
     const grid_gpu_plan* q = is_crt(p) ? p->crt[j] : p;
     uint32_t* out = is_crt(p) ? gj[j] : G;
-    if (ldx % 4 == 0 && pm_fits(q, r, r, n, EMM_UPPER)) {
+    if (pm) {
       rc = launch_ntt_tc_pm(q, S, r, n, s_hat, st);
       if (!rc)
         rc = launch_emm_pm(q, s_hat, s_hat, (int)r, (int)r, (int)n, (int)ldx, (int)ldx, EMM_UPPER,
@@ -553,7 +601,7 @@ int grid_gpu_gram(grid_gpu_plan* p, const uint32_t* S, size_t r, size_t n, uint3
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
   std::lock_guard<std::mutex> lk(p->mu);
   const size_t s_bytes = r * n * p->d * 4, g_bytes = r * (r + 1) / 2 * p->d * 4;
-  const size_t ws = gram_ws_bytes(p, r, n, pm_stride(n));
+  const size_t ws = gram_ws_bytes(p, r, n, true);
   int rc;
   if ((rc = ensure_scratch(p, 6, s_bytes)) || (rc = ensure_scratch(p, 7, g_bytes)) ||
       (rc = ensure_scratch(p, 8, ws)))
@@ -574,7 +622,7 @@ int grid_gpu_gram(grid_gpu_plan* p, const uint32_t* S, size_t r, size_t n, uint3
 int grid_gpu_garbage_h_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes) {
   if (!p || !bytes) return GRID_ERR_NULL_POINTER;
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
-  *bytes = garbage_h_ws_bytes(p, r, n);
+  *bytes = garbage_h_ws_bytes(p, r, n, true);
   return GRID_OK;
 }
 
@@ -587,12 +635,13 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     return GRID_ERR_MISALIGNED;
   cudaStream_t st = (cudaStream_t)stream;
   Carver cv(workspace, workspace_bytes);
-  const size_t ldx = pm_stride(n);
+  const bool pm = garbage_h_pm(p, r, n) && workspace_bytes >= garbage_h_ws_bytes(p, r, n, true);
+  const EvalsLayout l(residue_plan(p), pm, n);
+  const size_t ldx = l.stride;
   uint32_t* s_hat = cv.take<uint32_t>(r * ldx * p->d);
   uint32_t* phi_hat = cv.take<uint32_t>(r * ldx * p->d);
   uint32_t* cross = cv.take<uint32_t>(r * r * p->d);
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
-  const size_t ew = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_DENSE);
+  const size_t ew = l.work(r, r, n, EMM_DENSE);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   uint32_t* cj[3] = {};
   if (is_crt(p)) {
@@ -600,7 +649,6 @@ int grid_gpu_garbage_h_dev(const grid_gpu_plan* p, const uint32_t* S, const uint
     for (auto& x : cj) x = cv.take<uint32_t>(r * r * p->d);
   }
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-  const bool pm = pm_fits(e, r, r, n, EMM_DENSE);
   // point-major: <phi_i, s_j> through to coefficients, symmetrised if sym
   auto cross_pm = [&](const grid_gpu_plan* q, bool sym, uint32_t* out) {
     int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, st);
@@ -647,7 +695,7 @@ int grid_gpu_garbage_h(grid_gpu_plan* p, const uint32_t* S, const uint32_t* Phi,
   if (!square_dims_ok(p, r, n)) return GRID_ERR_INVALID_PARAMETERS;
   std::lock_guard<std::mutex> lk(p->mu);
   const size_t s_bytes = r * n * p->d * 4, h_bytes = r * (r + 1) / 2 * p->d * 4;
-  const size_t ws = garbage_h_ws_bytes(p, r, n);
+  const size_t ws = garbage_h_ws_bytes(p, r, n, true);
   int rc;
   if ((rc = ensure_scratch(p, 6, s_bytes)) || (rc = ensure_scratch(p, 9, s_bytes)) ||
       (rc = ensure_scratch(p, 7, h_bytes)) || (rc = ensure_scratch(p, 8, ws)))
@@ -945,7 +993,7 @@ int grid_gpu_prover_round_workspace(const grid_gpu_matrix* A, size_t r, size_t j
   const size_t n = A->cols, kappa = A->rows, d = p->d;
   if (!dims_ok(r, n, kappa) || !square_dims_ok(p, r, n) || !words_fit(r, kappa, d))
     return GRID_ERR_INVALID_PARAMETERS;
-  *bytes = round_ws_bytes(p, r, n, kappa, jl_rows);
+  *bytes = round_ws_bytes(p, r, n, kappa, jl_rows, true);
   return GRID_OK;
 }
 
@@ -962,13 +1010,13 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
   if (!aligned16(S) || !aligned16(g) || !aligned16(workspace)) return GRID_ERR_MISALIGNED;
   if (is_crt(p) && !crt_bound_ok(p, n)) return GRID_ERR_INVALID_PARAMETERS;
   cudaStream_t st = (cudaStream_t)stream;
-  const grid_gpu_plan* e = is_crt(p) ? p->crt[0] : p;
+  const bool pm = round_pm(p, r, n, kappa) &&
+                  workspace_bytes >= round_ws_bytes(p, r, n, kappa, jl_rows, true);
+  const EvalsLayout l(residue_plan(p), pm, n);
   Carver cv(workspace, workspace_bytes);
-  const size_t ldx = pm_stride(n);
+  const size_t ldx = l.stride;
   uint32_t* s_hat = cv.take<uint32_t>(r * ldx * d);
-  const size_t e1 = emm_workspace_words(e, (int)r, (int)kappa, (int)n, EMM_DENSE);
-  const size_t e2 = emm_workspace_words(e, (int)r, (int)r, (int)n, EMM_UPPER);
-  const size_t ew = e1 > e2 ? e1 : e2;
+  const size_t ew = round_work(l, r, n, kappa);
   uint32_t* work = ew ? cv.take<uint32_t>(ew) : nullptr;
   uint32_t* t = cv.take<uint32_t>(r * kappa * d);
   void* jl_ws = cv.take<char>(jl_scratch_bytes(jl_rows ? jl_rows : 1));
@@ -981,14 +1029,11 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
       gj[j] = cv.take<uint32_t>(gw);
     }
   if (!cv.ok) return GRID_ERR_INVALID_PARAMETERS;
-  auto round_pm = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq) {
-    return Aq->d_evals_pm && pm_fits(q, r, kappa, n, EMM_DENSE) && pm_fits(q, r, r, n, EMM_UPPER);
-  };
   // inner commitments and the Gram over the witness's evaluations (one
   // transform shared by both) on plan q into tt / gg, or their limbs (tt unwritten then)
   auto contract = [&](const grid_gpu_plan* q, const grid_gpu_matrix* Aq, uint32_t* tt,
                       uint32_t* gg, const LimbSpec& tl, const LimbSpec& gl, cudaStream_t cs) {
-    if (round_pm(q, Aq)) {
+    if (pm && Aq->d_evals_pm) {
       // point-major evaluations: both products load their operands with TMA
       int rc = launch_ntt_tc_pm(q, S, r, n, s_hat, cs);
       if (!rc)
@@ -1037,7 +1082,7 @@ int grid_gpu_prover_round_dev(const grid_gpu_matrix* A, const uint32_t* S, size_
     };
     LimbSpec tl = spec(t_limbs, b1, t1), gl = spec(g_limbs, b2, t2);
     if (!is_crt(p)) {
-      if (!round_pm(p, A)) tl = gl = LimbSpec();  // the poly-major products leave them to a pass
+      if (!pm || !A->d_evals_pm) tl = gl = LimbSpec();  // gathering products: a pass of its own
       rc_chain = contract(p, A, t, g, tl, gl, hi);
     } else {
       for (int j = 0; j < 3 && !rc_chain; ++j)

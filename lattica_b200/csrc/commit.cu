@@ -282,18 +282,22 @@ int launch_emm_tile(dim3 grid, const uint32_t* X, const uint32_t* Y, uint32_t* d
 
 }  // namespace
 
-size_t emm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode) {
+size_t emm_gather_words(const grid_gpu_plan* p, int M, int N, int K, int mode) {
   if (M <= 0 || N <= 0 || K <= 0 || p->d % EG) return 0;
   const EmmGeometry g = emm_geometry(M, N, K, (int)p->d, mode, p->num_sms);
   EmmTcGeometry tg;
   const int splits = !g.mv && emm_tc_geometry(p, M, N, K, mode, &tg) ? tg.splits : g.splits;
   const size_t outputs = mode == OUT_UPPER ? (size_t)M * (M + 1) / 2 : (size_t)M * N;
-  const size_t words = splits > 1 ? (size_t)splits * outputs * p->d : 0;
+  return splits > 1 ? (size_t)splits * outputs * p->d : 0;
+}
+
+size_t emm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode) {
+  const size_t words = emm_gather_words(p, M, N, K, mode);
   const size_t pm = emm_pm_workspace_words(p, M, N, K, mode);  // point-major operands
   return words > pm ? words : pm;
 }
 
-// out_evals: dense [M][N][d] or packed-upper [M(M+1)/2][d]. work: >= emm_workspace_words.
+// out_evals: dense [M][N][d] or packed-upper [M(M+1)/2][d]. work: >= emm_gather_words.
 int launch_emm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N, int K,
                int ldy, int mode, uint32_t* out_evals, uint32_t* work, cudaStream_t s) {
   if (is_crt(p)) return p->ntt_status;  // evaluation-domain products need an NTT for q

@@ -162,7 +162,8 @@ void build_tc256_tables(uint32_t q, uint64_t psi, std::vector<unsigned char>& ou
 
 // commit.cu: out_e[m][n] = sum_k X[m][k][e] * Y[n][k][e] for every evaluation point.
 enum EmmOut : int { EMM_DENSE = 0, EMM_UPPER = 1 };
-size_t emm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode);
+size_t emm_gather_words(const grid_gpu_plan* p, int M, int N, int K, int mode);  // launch_emm
+size_t emm_workspace_words(const grid_gpu_plan* p, int M, int N, int K, int mode);  // any engine
 int launch_emm(const grid_gpu_plan* p, const uint32_t* X, const uint32_t* Y, int M, int N, int K,
                int ldy, int mode, uint32_t* out_evals, uint32_t* work, cudaStream_t s);
 int launch_pointwise(const grid_gpu_plan* p, uint32_t* dst, const uint32_t* rhs, size_t words,
@@ -207,8 +208,8 @@ int launch_to_point_major(const uint32_t* in, uint32_t* out, size_t rows, size_t
 int launch_sum_inverse(const grid_gpu_plan* p, const uint32_t* part, int outputs, int splits,
                        int sym_r, uint32_t* out, const LimbSpec& limbs, cudaStream_t s,
                        bool in_round = false);
-// The least workspace grid_gpu_gram_dev runs in (grid_gpu_gram_workspace: what it runs
-// best in).
+// The least workspace grid_gpu_gram_dev runs in, by the gathering products
+// (grid_gpu_gram_workspace: what it runs best in).
 int gram_min_workspace(const grid_gpu_plan* p, size_t r, size_t n, size_t* bytes);
 // garbage.cu: (C_ij + C_ji) * 2^-1 on the upper triangle; z_hat = sum_i c_hat_i (.) s_hat_i.
 int launch_symmetrize_half(const grid_gpu_plan* p, const uint32_t* C, int r, uint32_t* H,

@@ -965,12 +965,12 @@ VecProduct vec_product(const grid_gpu_plan* p, const VecOperand& o, size_t all_c
 
 }  // namespace
 
+// For the most CTAs that products of up to these lengths take: a shorter one may have more
+// of them (longer vectors take whole blocks of 64 columns), and a workspace may serve both.
 size_t commit_vec_words(const grid_gpu_plan* p, size_t rows, size_t cols0, size_t cols1,
                         size_t batch) {
-  const VecOperand a{nullptr, nullptr, cols0, 0}, b{nullptr, nullptr, cols1, 0};
-  const size_t all = cols0 + cols1;
-  return (size_t)(vec_product(p, a, all).ctas + (cols1 ? vec_product(p, b, all).ctas : 0)) * rows *
-         64 * batch;
+  const size_t ctas = (cols0 + 15) / 16 + (cols1 + 15) / 16;
+  return std::min(ctas, 2 * (size_t)p->num_sms + 2) * rows * 64 * batch;
 }
 
 int launch_commit_vec(const grid_gpu_plan* p, const VecOperand& o0, const VecOperand* o1,
