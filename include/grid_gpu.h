@@ -346,9 +346,9 @@ typedef struct grid_gpu_batch_item {
   uint32_t matrix;
 } grid_gpu_batch_item;
 /* Engines of the grouped product: POINT_MAJOR runs the tensor cores over
- * point-major evaluations (the witnesses' transform stores [point][poly], each
- * instance at its own 128-aligned columns; every matrix needs its point-major
- * copy: d = 64, rows <= 32, cols a multiple of 4; k_split a multiple of 32;
+ * point-major evaluations (the witnesses' transform stores [point][poly], the
+ * instances of a tile in blocks of 128 columns; every matrix needs its point-major
+ * copy and cols a multiple of 4: d = 64, rows <= 32; k_split a multiple of 32;
  * else GRID_ERR_UNSUPPORTED_DEGREE / GRID_ERR_INVALID_PARAMETERS); TENSOR runs
  * them over gathered poly-major evaluations (d % 4 == 0, tensor-core plan,
  * else GRID_ERR_UNSUPPORTED_DEGREE); CUDA_CORE never uses them; AUTO =

@@ -340,8 +340,9 @@ int build_tables(const grid_gpu_plan* plan, grid_gpu_matrix* const* mats, size_t
   }
   // The point-major engine needs the point-major forward transform (d = 64,
   // tensor cores), every matrix's point-major evaluations over a multiple of four
-  // columns, K ranges of whole chunks, and transform tiles whose source rows and
-  // destination columns stay below 2^31; AUTO takes it where those hold.
+  // columns (the engine's contract in grid_gpu.h; its rows are padded and would take any),
+  // K ranges of whole chunks, and transform tiles whose source rows and destination
+  // columns stay below 2^31; AUTO takes it where those hold.
   bool pm_ok = plan->pm_emm && ntt_tc_available(plan) && k_split % 32 == 0 &&
                tb.s_polys <= (uint64_t)INT32_MAX - 128 && tb.pm_polys <= (uint64_t)INT32_MAX - 128;
   for (size_t i = 0; pm_ok && i < nmats; ++i)

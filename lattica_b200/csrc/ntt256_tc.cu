@@ -36,7 +36,7 @@
 //   MMA (warp 16 + j % 2): fwd(j) after P(j), inv(j) after F(j), into the same columns.
 // A wait that timed out ends a role's waits, not its steps, so the others still meet it at
 // their barriers; every wait is bounded.
-// Bound: instruction issue and the integer pipes (0.62 and 0.5 of their cycles), then the
+// Bound: instruction issue and the integer pipes (0.66 and 0.58 of their cycles), then the
 // waits of two groups that overlap only each other. 2^20 polynomials: 1.20 ms with sixteen
 // warps in step (0.47 of the issue slots), with the 4-point steps outside the products or,
 // a fifth fewer instructions, between them; 1.10 with two groups; 1.08 with the MMA and

@@ -25,8 +25,8 @@
 //     two batches of 8 + 8: combine the planes, multiply by b, write S and D
 //   E0, E1 (warps 8-15): 32 outputs each in two batches, m = 2 i and 2 i + 1 from the two
 //     products; staged per group and stored by TMA
-// Measured at 2^22 polynomials: 0.64 ms alone and 0.72 ms in a loop that reaches the power
-// cap; with both full matrices in shared memory, one epilogue phase after the other in
+// Measured at 2^22 polynomials: 0.64 ms alone and 0.75 to 0.78 ms in a loop that reaches the
+// power cap; with both full matrices in shared memory, one epilogue phase after the other in
 // all 16 warps and the results staged in the input's two buffers 0.78 to 0.84 ms. Without
 // the MMAs 0.56 ms, without the integer arithmetic 0.57 (768 bytes a polynomial at the
 // measured HBM rate: 0.49).
